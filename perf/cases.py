@@ -256,3 +256,78 @@ def tolerance(case):
     if path == "attention":
         return {"rel": 1e-2 if bf16 else 1e-3}
     return {"rel": 6.5e-3 if bf16 else 8.5e-4}
+
+
+def _e4m3(x):
+    """x rounded to the nearest e4m3 value, saturating."""
+    return x.clamp(-448.0, 448.0).to(torch.float8_e4m3fn).float()
+
+
+def _quantized_rows(x):
+    """x (rows, k) in float32 as e4m3 values times a scale per row (the row's largest magnitude / 448), in 64 bits."""
+    scale = x.abs().amax(dim=1, keepdim=True) / 448.0
+    return _e4m3(x * (1.0 / torch.where(scale > 0, scale, torch.ones_like(scale)))).double() * scale.double()
+
+
+def _quantized_blocks(x, scale):
+    """x (rows, k) in float32 as e2m1 values times an e4m3 scale per 16 and `scale`, in 64 bits."""
+    blocks = x.reshape(x.shape[0], -1, 16)
+    factor = _e4m3(blocks.abs().amax(dim=2, keepdim=True) / (6.0 * scale))
+    step = factor * scale
+    y = blocks * torch.where(step > 0, 1.0 / step, torch.zeros_like(step))
+    bounds = torch.tensor([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], device=x.device)  # between the magnitudes, ties to even
+    magnitude = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], device=x.device, dtype=torch.float64)
+    up, down = torch.bucketize(y.abs(), bounds, right=True), torch.bucketize(y.abs(), bounds)
+    code = torch.where(up % 2 == 0, up, down)
+    return (magnitude[code] * y.sign().double() * step.double()).reshape(x.shape)
+
+
+def exact(case, seed):
+    """run()'s result from the same inputs with the operands' own quantisation, the arithmetic in 64
+    bits. The blocks of a denoise step have none: a rounding moves codes in every quantiser after it."""
+    path = case["path"]
+    if path == "denoise":
+        return None
+    new = _Inputs(seed)
+    kind = TORCH_TYPE[case["type"]]
+    gelu = lambda t: torch.nn.functional.gelu(t, approximate="tanh")
+    if path == "attention":
+        b, h, hk, lq, lk, d = (case[x] for x in ("batch", "heads", "kv_heads", "q_len", "kv_len", "head_dim"))
+        q, keys, values = (new.normal(s, 1.0, kind) for s in ((b, lq, h, d), (b, lk, hk, d), (b, lk, hk, d)))
+        out = torch.empty((b, lq, h, d), device="cuda", dtype=torch.float64)
+        hidden = torch.ones((lq, lk), device="cuda", dtype=torch.bool).triu(1 + lk - lq) if case["causal"] else None
+        for i in range(b):
+            for j in range(h):
+                g = j // (h // hk)
+                scores = q[i, :, j].double() @ keys[i, :, g].double().t() / math.sqrt(d)
+                if hidden is not None:
+                    scores.masked_fill_(hidden, -math.inf)
+                out[i, :, j] = scores.softmax(dim=1) @ values[i, :, g].double()
+        return out
+    if path == "fp8_mlp":
+        m, d, h = case["m"], case["hidden"], case["inner"]
+        x = new.normal((m, d), 1.0, kind)
+        up, down = _quantized_rows(new.normal((h, d), 0.02)), _quantized_rows(new.normal((d, h), 0.02))
+        up_bias, down_bias = (new.normal((n,), 0.01, kind).double() for n in (h, d))
+        inner = gelu(_quantized_rows(x.float()) @ up.t() + up_bias).to(kind)
+        return _quantized_rows(inner.float()) @ down.t() + down_bias + x.double()
+    m, n, k = case["m"], case["n"], case["k"]
+    a = new.normal((m, k), 1.0, kind)
+    w = new.normal((n, k), 0.02)
+    if path == "fp8_matmul":
+        scale = w.abs().max() / 448.0
+        y = a.double() @ (w / scale).to(torch.float8_e4m3fn).double().t() * scale.double()
+        if case["addend"] != "none":
+            y += (new.normal((n,), 0.01, kind) if case["addend"] == "bias" else new.normal((m, n), 1.0, kind)).double()
+        return y
+    if path == "fp8_linear":
+        y = _quantized_rows(a.float()) @ _quantized_rows(w).t()
+    else:
+        y = _quantized_blocks(a.float(), 1.0) @ _quantized_blocks(w, w.abs().max() / (448.0 * 6.0)).t()
+    if case["bias"]:
+        y += new.normal((n,), 0.01, kind).double()
+    if case.get("gelu"):
+        y = gelu(y)
+    if case.get("residual"):
+        y += new.normal((m, n), 1.0, kind).double()
+    return y
