@@ -293,7 +293,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       mbar_arrive_expect_tx(&t.q_full_bar, L::kQBytes);
 #pragma unroll
@@ -336,7 +336,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fmt = p.is_bf16 ? 1u : 0u;
       const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
       const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
@@ -755,7 +755,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   // Load n of the ring (K of block n / 2 when n is even, V of it when odd) goes to slot n % S.
   if (warp == kProducerWarp2) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < kTiles; ++i) {
         mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
@@ -802,7 +802,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // The whole warp walks the loop and one lane issues: what an instruction takes (descriptors,
     // addresses) is then the same in every lane, which lets it live in uniform registers instead of
     // being moved there instruction by instruction by a lone thread.
-    const bool issuer = lane == 0;
+    const bool issuer = elect_one();
     {
       const uint32_t fmt = p.is_bf16 ? 1u : 0u;
       const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);

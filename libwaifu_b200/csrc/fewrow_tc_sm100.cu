@@ -160,7 +160,7 @@ fewrow_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   auto stage_w = [&](int s) { return smem + kRawOff + s * kRawWBytes; };
 
   if (warp == kProducer) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int st = 0; st < num_stages && ok; ++st) {
         const int s = st % kRawStages, xs = st % kXStages;
@@ -186,7 +186,7 @@ fewrow_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
     }
   } else if (warp >= kMma && warp < kMma + kMmaWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       // Every tcgen05 issue costs the issuing thread some 90 cycles, sixteen of them per stage more
       // than the stage's bytes take to arrive: the blocks of a stage are dealt to four threads.
       const int mw = static_cast<int>(warp) - kMma;
@@ -432,7 +432,7 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   griddep_launch_dependents();
 
   if (warp == kQProducer) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int st = 0; st < num_stages && ok; ++st) {
         const int s = st % p.stages;
@@ -454,7 +454,7 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
     }
   } else if (warp >= kQMma) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int mw = static_cast<int>(warp) - kQMma;
       constexpr uint32_t kFmt = KIND == kKindBF16 ? 1u : 0u;
       const uint32_t idesc = umma_idesc(kChannels, static_cast<uint32_t>(p.ntok), kFmt, kFmt);

@@ -381,7 +381,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -461,7 +461,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // The whole warp of the leader walks the loop and one lane issues: what an instruction takes is
     // then the same in every lane.
     if (leader) {
-      const bool issuer = lane == 0;
+      const bool issuer = elect_one();
       // e4m3 is format 0 of kind::f8f6f4; fp16 / bf16 are formats 0 / 1 of kind::f16.
       // (The mixed form exists for half only: both operands of a UMMA share one 16-bit format.)
       constexpr uint32_t kFmt = (KIND == kKindBF16) ? 1u : 0u;
@@ -573,7 +573,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // ------------------------------------------------------------------ scale-factor copier (NVFP4)
     // One thread of the leader moves every stage's scale factors shared -> tensor memory, into
     // the set the MMAs are not reading, and hands the set over with a commit.
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint64_t kStageStep = Cfg::kStageBytes >> 4;
       constexpr uint64_t kSfTileStep = kSfTileBytes >> 4;
       const uint64_t sfa_desc0 = umma_desc_sf(smem_u32(stage_sfa(0)));

@@ -21,6 +21,17 @@ __device__ __forceinline__ uint32_t lane_id() {
   return l;
 }
 
+// True in one lane of a converged warp. The compiler knows that code under it runs in one thread, so
+// what a tcgen05 instruction takes (descriptors, addresses) lives in uniform registers; under
+// `lane == 0` every instruction is issued some 60 to 130 cycles after the one before it, which is
+// what paced the kernels whose instructions are shorter than that (2 x 24 x 4352 x 128 attention
+// 454 -> 389 us; C3's four-bit GEMM, whose scale-factor copies are issued one by one, 103 -> 73).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 // ---- programmatic dependent launch ---------------------------------------------------------
 
 // Blocks until the grid this one was launched behind (same stream, programmatic serialization)
