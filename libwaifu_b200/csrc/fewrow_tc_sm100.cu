@@ -369,17 +369,6 @@ struct QParams {
   uint32_t *status;
 };
 
-__device__ __forceinline__ float gelu_tanh_q(float x) {
-  // x / (1 + 2^z), z = x (c0 + c1 x^2): the tile kernel's form of the tanh GELU, bit for bit.
-  constexpr float kC0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
-  constexpr float kC1 = kC0 * 0.044715f;
-  const float z = x * fmaf(x * x, kC1, kC0);
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
-  return x * r;
-}
-
 // KIND: kKindF8 (e4m3 codes on both sides), or kKindF16 / kKindBF16 for a 16-bit weight and 16-bit
 // rows (fl_matmul's linear-layer case): the same bytes per stage, half the K positions, and
 // nothing to scale.
@@ -521,7 +510,7 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
               const float rs = p.row_scale ? __ldg(p.row_scale + row) : 1.0f;
               float y = __uint_as_float(v[t]) * (rs * cs);
               if (bias16) y += bias;
-              if (p.act == 1) y = gelu_tanh_q(y);
+              if (p.act == 1) y = gelu_tanh(y);
               if (res) {
                 const uint16_t r16 = res[static_cast<long long>(row % p.residual_rows) * p.residual_ld + channel];
                 y += p.is_bf16 ? __uint_as_float(static_cast<uint32_t>(r16) << 16) : __half2float(__ushort_as_half(r16));

@@ -1976,10 +1976,8 @@ int32_t fl_nvfp4_linear(fl_tensor_view_t a_h, fl_tensor_view_t codes_h, fl_tenso
 
     Scratch scratch;
     const size_t xcodes_off = scratch.reserve(static_cast<size_t>(m) * k / 2);
-    const size_t sfa_bytes = static_cast<size_t>(sf_tiled_bytes(m, k, 0));
-    const size_t sfb_bytes = static_cast<size_t>(sf_tiled_bytes(rows, k, 1));  // one spare row group: a
-    const size_t sfa_off = scratch.reserve(sfa_bytes);                          // tile may read past the last
-    const size_t sfb_off = scratch.reserve(sfb_bytes);
+    const size_t sfa_off = scratch.reserve(static_cast<size_t>(sfa_tiled_bytes(m, k)));
+    const size_t sfb_off = scratch.reserve(static_cast<size_t>(sfb_tiled_bytes(rows, k)));
     size_t w_off = 0;
     const bool w_misaligned = !aligned16(raw_ptr(wcodes));
     if (w_misaligned) w_off = scratch.reserve(static_cast<size_t>(rows) * k / 2);
@@ -1988,7 +1986,7 @@ int32_t fl_nvfp4_linear(fl_tensor_view_t a_h, fl_tensor_view_t codes_h, fl_tenso
     // One launch: the activation's codes and scale factors, the weight's block scales re-tiled,
     // zeros in the padding of both (four launches with a gap each before: 1 805 -> 2 005 TFLOP/s on C3).
     cuda_check(nvfp4_prepare(raw_ptr(a), is_bf16, m, k, base + xcodes_off, base + sfa_off,
-                             reinterpret_cast<const uint8_t *>(raw_ptr(wsf)), rows, 1, base + sfb_off, 0),
+                             reinterpret_cast<const uint8_t *>(raw_ptr(wsf)), rows, base + sfb_off, 0),
                "quantising the activation and re-tiling the block scales");
     const void *w_ptr = raw_ptr(wcodes);
     if (w_misaligned) {

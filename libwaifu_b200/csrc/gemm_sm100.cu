@@ -62,6 +62,7 @@ constexpr int kRowBytes = 128;          // bytes of K per operand row per stage
 constexpr int kMmaKBytes = 32;          // bytes of K one tcgen05.mma consumes per row
 constexpr int kMmasPerStage = kRowBytes / kMmaKBytes;
 constexpr int kSfTileBytes = 512;       // 128 rows x 4 scale factors
+constexpr int kSfSets = 3;              // of scale factors in tensor memory
 constexpr int kNumWarps = 12;
 constexpr int kNumThreads = kNumWarps * 32;
 constexpr int kMaxEpilogueWarps = 8;
@@ -208,11 +209,13 @@ struct Config : Roles<B8> {
   static constexpr int kABytes = kBlockM * kRowBytes;
   static constexpr int kBRows = BLOCK_N / CTAS;
   static constexpr int kBBytes = kBRows * kRowBytes;
-  // Scale factors: A has one 128-row group; B is loaded as whole 128-row groups that cover the
-  // tile (a 192-wide tile starts mid-group on odd tiles, so it needs two).
-  static constexpr int kSfbGroups = NVF4 ? (BLOCK_N + 127) / 128 : 0;
+  // Scale factors of a stage: 32 rows x 4 factors to a column of tensor memory. A has four columns
+  // per instruction (128 rows), one 512-byte copy each; B has BLOCK_N / 32 = 6, laid out tile by
+  // tile so that a stage's 24 columns are six copies and nothing else is loaded.
+  static_assert(!NVF4 || BLOCK_N == kNvf4BlockN, "the weight's scale factors are laid out for one tile width");
+  static constexpr int kSfbCopies = NVF4 ? kNvf4SfbTiles : 0;
   static constexpr int kSfaBytes = NVF4 ? kMmasPerStage * kSfTileBytes : 0;
-  static constexpr int kSfbBytes = NVF4 ? kSfbGroups * kMmasPerStage * kSfTileBytes : 0;
+  static constexpr int kSfbBytes = kSfbCopies * kSfTileBytes;
   // Mixed form: 64 raw e4m3 bytes per B row per stage (the 64 K positions a 16-bit stage holds).
   static constexpr int kRawRowBytes = 64;
   static constexpr int kRawBytes = B8 ? kBRows * kRawRowBytes : 0;
@@ -234,36 +237,23 @@ struct Config : Roles<B8> {
   static constexpr int kColParamOffset = kOutStageOffset + kOutStageBytes;
   static constexpr int kSmemBytes = kColParamOffset + kColParamBytes + 1024;  // + slack to align to 1024
   static_assert(kStageBytes % 512 == 0, "the output staging behind the stages has to stay 512-byte aligned");
-  // Tensor memory columns: two accumulators, then two sets of one stage's scale factors. The
-  // copies into a set are issued by a thread of their own, a stage ahead of the MMAs that read
-  // the other set: issued by the MMA thread itself they execute in order with its MMAs, and
-  // cost as much as those.
+  // Tensor memory columns: two accumulators, then three sets of one stage's scale factors. The
+  // copies into a set are issued by a thread of their own, ahead of the MMAs that read the
+  // others: issued by the MMA thread itself they execute in order with its MMAs, and cost as
+  // much as those. Two sets left one stage's MMAs to hide the way commit -> wait -> ten copies ->
+  // commit -> wait; three leave two.
   static constexpr int kAccCols = 2 * BLOCK_N;
   static constexpr int kSfaCols = NVF4 ? kMmasPerStage * 4 : 0;
-  static constexpr int kSfbColsPerMma = NVF4 ? kSfbGroups * 4 : 0;
+  static constexpr int kSfbColsPerMma = NVF4 ? BLOCK_N / 32 : 0;
   static constexpr int kSfbCols = kMmasPerStage * kSfbColsPerMma;
+  static_assert(kSfbCols == 4 * kSfbCopies, "a copy fills four columns");
   static constexpr int kSfSetCols = kSfaCols + kSfbCols;
-  static constexpr int kUsedCols = kAccCols + 2 * kSfSetCols;
+  static constexpr int kUsedCols = kAccCols + kSfSets * kSfSetCols;
   static constexpr int kTmemCols = kUsedCols <= 32 ? 32 : kUsedCols <= 64 ? 64 : kUsedCols <= 128 ? 128
                                    : kUsedCols <= 256 ? 256 : 512;
   static_assert(kUsedCols <= 512, "tensor memory holds 512 columns");
   static_assert(kStages >= 2, "need at least two stages");
 };
-
-__device__ __forceinline__ float gelu_tanh(float x) {
-  // 0.5 x (1 + tanh(u)) == x * sigmoid(2u) == x / (1 + 2^z), u = sqrt(2/pi) (x + 0.044715 x^3),
-  // z = -2 u log2(e) = x (c0 + c1 x^2)
-  // (waifu/src/krea2/dit.rs:170-188 spells the same function as seven graph nodes).
-  // Five FP32 operations and two special-function operations; both approximations are good to
-  // about 2^-22, far inside the 16-bit output step. x -> -inf gives 2^z = inf, 1/inf = 0, -0.
-  constexpr float kC0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
-  constexpr float kC1 = kC0 * 0.044715f;
-  const float z = x * fmaf(x * x, kC1, kC0);
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
-  return x * r;
-}
 
 __device__ __forceinline__ float load16(const void *p, long long idx, int is_bf16) {
   if (is_bf16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(p)[idx]);
@@ -318,8 +308,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   __shared__ __align__(8) uint64_t acc_full_bar[2];
   __shared__ __align__(8) uint64_t acc_empty_bar[2];
   __shared__ __align__(8) uint64_t tile_done_bar[2];  // epilogue -> pushers: the tile is in this GPU's matrix
-  __shared__ __align__(8) uint64_t sf_full_bar[2];    // NVFP4: a set of scale factors is in tensor memory
-  __shared__ __align__(8) uint64_t sf_empty_bar[2];   // NVFP4: the MMAs that read the set are done
+  __shared__ __align__(8) uint64_t sf_full_bar[kSfSets];   // NVFP4: a set of scale factors is in tensor memory
+  __shared__ __align__(8) uint64_t sf_empty_bar[kSfSets];  // NVFP4: the MMAs that read the set are done
   __shared__ __align__(8) uint64_t raw_full_bar[B8 ? STAGES : 1];  // mixed form: a stage's e4m3 weight bytes have landed
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile uint32_t abort_flag;
@@ -346,6 +336,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // the accumulator too, which keeps the epilogue from running two tiles ahead of them.
       mbar_init(&acc_empty_bar[s], (kEpilogueWarps + (scatter ? kPusherWarps : 0)) * CTAS);
       mbar_init(&tile_done_bar[s], kEpilogueWarps);
+    }
+    for (int s = 0; s < kSfSets; ++s) {
       mbar_init(&sf_full_bar[s], 1);
       mbar_init(&sf_empty_bar[s], 1);
     }
@@ -397,13 +389,12 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             ok = false;
             break;
           }
-          // Scale-factor tiles of this k block (NVFP4): kMmasPerStage consecutive 512-byte tiles
-          // per 128-row group, addressed as rows of a (groups * sf_k_tiles, 512 byte) matrix. A
-          // CTA loads the group of its own A rows and every group its tile's B columns touch (in
-          // a pair both CTAs need all of B's factors, since each multiplies its rows by all
-          // BLOCK_N columns).
+          // Scale-factor tiles of this k block (NVFP4), addressed as rows of 512-byte matrices: of
+          // A kMmasPerStage consecutive ones of the CTA's 128 rows, of B the six of the tile's
+          // columns and this stage (in a pair both CTAs need all of B's factors, since each
+          // multiplies its rows by all BLOCK_N columns).
           const int sfa_row = (tm * CTAS + static_cast<int>(cta_rank)) * p.sf_k_tiles + kb * kMmasPerStage;
-          const int sfb_row0 = (n0 / 128) * p.sf_k_tiles + kb * kMmasPerStage;
+          const int sfb_row = (tn * (p.sf_k_tiles / kMmasPerStage) + kb) * Cfg::kSfbCopies;
           if constexpr (B8) {
             // The weight's bytes go to the raw part of the stage under a barrier of this CTA's own,
             // which its converter warps wait on; only A counts on the stage's barrier.
@@ -426,11 +417,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                              n0 + static_cast<int>(cta_rank) * Cfg::kBRows);
             if constexpr (NVF4) {
               tma_load_2d_pair(stage_sfa(stage), &tmap_sfa, bar, 0, sfa_row);
-#pragma unroll
-              for (int g = 0; g < Cfg::kSfbGroups; ++g) {
-                tma_load_2d_pair(stage_sfb(stage) + g * kMmasPerStage * kSfTileBytes, &tmap_sfb, bar, 0,
-                                 sfb_row0 + g * p.sf_k_tiles);
-              }
+              tma_load_2d_pair(stage_sfb(stage), &tmap_sfb, bar, 0, sfb_row);
             }
           } else {
             mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
@@ -438,11 +425,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             tma_load_2d(stage_b(stage), &tmap_b, &full_bar[stage], kb * kRowBytes, n0);
             if constexpr (NVF4) {
               tma_load_2d(stage_sfa(stage), &tmap_sfa, &full_bar[stage], 0, sfa_row);
-#pragma unroll
-              for (int g = 0; g < Cfg::kSfbGroups; ++g) {
-                tma_load_2d(stage_sfb(stage) + g * kMmasPerStage * kSfTileBytes, &tmap_sfb, &full_bar[stage], 0,
-                            sfb_row0 + g * p.sf_k_tiles);
-              }
+              tma_load_2d(stage_sfb(stage), &tmap_sfb, &full_bar[stage], 0, sfb_row);
             }
           }
           if (++stage == STAGES) {
@@ -489,7 +472,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       (void)sfa_desc0;
       (void)sfb_desc0;
       (void)kSfTileStep;
-      uint32_t sf_it = 0;  // NVFP4: K stages so far, over all tiles: picks the scale-factor set and its phase
+      uint32_t sf_set = 0, sf_phase = 0;  // NVFP4: the next stage's set of scale factors, over all tiles
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -499,14 +482,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       for (; ok && walk.next(&item); ++local) {
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
-        // A tile that starts 64 rows into a 128-row scale group reads its B scale factors two
-        // tensor-memory columns further on (32 rows per column).
-        uint32_t sfb_skip = 0;
-        if constexpr (NVF4) {
-          int tm, tn;
-          tile_coords(item.tile, p.tiles_m, p.tiles_n, &tm, &tn);
-          sfb_skip = ((tn * BLOCK_N) % 128) / 32;
-        }
         if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, &abort_flag)) {
           ok = false;
           break;
@@ -523,10 +498,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint64_t adesc = adesc0 + stage * kStageStep;
           const uint64_t bdesc = bdesc0 + stage * kStageStep;
           if constexpr (NVF4) {
-            const uint32_t sf_set = sf_it & 1;
             const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols + sf_set * Cfg::kSfSetCols;
             const uint32_t sfb_tmem = sfa_tmem + Cfg::kSfaCols;
-            if (!mbar_wait(&sf_full_bar[sf_set], (sf_it >> 1) & 1, &abort_flag)) {
+            if (!mbar_wait(&sf_full_bar[sf_set], sf_phase, &abort_flag)) {
               ok = false;
               break;
             }
@@ -535,10 +509,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             for (int j = 0; j < kMmasPerStage; ++j) {
               if constexpr (CTAS == 2) {
                 if (issuer) umma_nvf4_ss_pair(d_tmem, adesc + j * kMmaStep, bdesc + j * kMmaStep, idesc, ((kb - kb_first) | j) != 0 ? 1u : 0u,
-                                  sfa_tmem + j * 4, sfb_tmem + j * Cfg::kSfbColsPerMma + sfb_skip);
+                                  sfa_tmem + j * 4, sfb_tmem + j * Cfg::kSfbColsPerMma);
               } else {
                 if (issuer) umma_nvf4_ss(d_tmem, adesc + j * kMmaStep, bdesc + j * kMmaStep, idesc, ((kb - kb_first) | j) != 0 ? 1u : 0u,
-                             sfa_tmem + j * 4, sfb_tmem + j * Cfg::kSfbColsPerMma + sfb_skip);
+                             sfa_tmem + j * 4, sfb_tmem + j * Cfg::kSfbColsPerMma);
               }
             }
           } else {
@@ -553,8 +527,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           }
           commit_to(&empty_bar[stage]);
           if constexpr (NVF4) {
-            commit_to(&sf_empty_bar[sf_it & 1]);
-            ++sf_it;
+            commit_to(&sf_empty_bar[sf_set]);
+            if (++sf_set == kSfSets) {
+              sf_set = 0;
+              sf_phase ^= 1;
+            }
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -580,15 +557,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const uint64_t sfb_desc0 = umma_desc_sf(smem_u32(stage_sfb(0)));
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t it = 0;
+      uint32_t set = 0, set_phase = 0;
       bool ok = true;
       WorkWalk walk(p, unit, num_units);
       WorkItem item;
       while (ok && walk.next(&item)) {
-        for (int kb = item.kb0; kb < item.kb1; ++kb, ++it) {
-          const uint32_t set = it & 1;
+        for (int kb = item.kb0; kb < item.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, &abort_flag) ||
-              !mbar_wait(&sf_empty_bar[set], ((it >> 1) & 1) ^ 1, &abort_flag)) {
+              !mbar_wait(&sf_empty_bar[set], set_phase ^ 1, &abort_flag)) {
             ok = false;
             break;
           }
@@ -597,27 +573,25 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint64_t sfb_desc = sfb_desc0 + stage * kStageStep;
           const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols + set * Cfg::kSfSetCols;
           const uint32_t sfb_tmem = sfa_tmem + Cfg::kSfaCols;
-#pragma unroll
-          for (int j = 0; j < kMmasPerStage; ++j) {
+          auto copy = [&](uint32_t taddr, uint64_t desc) {
             if constexpr (CTAS == 2) {
-              tmem_cp_sf_pair(sfa_tmem + j * 4, sfa_desc + j * kSfTileStep);
+              tmem_cp_sf_pair(taddr, desc);
             } else {
-              tmem_cp_sf(sfa_tmem + j * 4, sfa_desc + j * kSfTileStep);
+              tmem_cp_sf(taddr, desc);
             }
+          };
 #pragma unroll
-            for (int g = 0; g < Cfg::kSfbGroups; ++g) {
-              const uint64_t d = sfb_desc + (g * kMmasPerStage + j) * kSfTileStep;
-              if constexpr (CTAS == 2) {
-                tmem_cp_sf_pair(sfb_tmem + j * Cfg::kSfbColsPerMma + g * 4, d);
-              } else {
-                tmem_cp_sf(sfb_tmem + j * Cfg::kSfbColsPerMma + g * 4, d);
-              }
-            }
-          }
+          for (int j = 0; j < kMmasPerStage; ++j) copy(sfa_tmem + j * 4, sfa_desc + j * kSfTileStep);
+#pragma unroll
+          for (int j = 0; j < Cfg::kSfbCopies; ++j) copy(sfb_tmem + j * 4, sfb_desc + j * kSfTileStep);
           if constexpr (CTAS == 2) {
             umma_commit_pair_both(&sf_full_bar[set]);
           } else {
             umma_commit(&sf_full_bar[set]);
+          }
+          if (++set == kSfSets) {
+            set = 0;
+            set_phase ^= 1;
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -655,10 +629,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint32_t r = static_cast<uint32_t>(piece) >> 2, q = static_cast<uint32_t>(piece) & 3;
           const uint4 v = *reinterpret_cast<const uint4 *>(raw + piece * 16);
           uint4 lo, hi;
-          e4m3x4_to_f16x4(v.x, &lo.x, &lo.y);
-          e4m3x4_to_f16x4(v.y, &lo.z, &lo.w);
-          e4m3x4_to_f16x4(v.z, &hi.x, &hi.y);
-          e4m3x4_to_f16x4(v.w, &hi.z, &hi.w);
+          e4m3x16_to_f16(v, &lo, &hi);
           uint8_t *row_base = b16 + r * kRowBytes;
           *reinterpret_cast<uint4 *>(row_base + (((2 * q) ^ (r & 7)) << 4)) = lo;
           *reinterpret_cast<uint4 *>(row_base + (((2 * q + 1) ^ (r & 7)) << 4)) = hi;
@@ -1186,13 +1157,13 @@ bool make_tmap_raw(CUtensorMap *map, const void *base, uint64_t rows, uint64_t r
 }
 
 // The scale-factor tiles of one operand as a (tiles, 512 byte) matrix of 32-bit words, read in
-// boxes of kMmasPerStage tiles (the factors of one K stage of one 128-row group), unswizzled.
-bool make_tmap_sf(CUtensorMap *map, const void *base, uint64_t tiles) {
+// boxes of the tiles of one K stage, unswizzled.
+bool make_tmap_sf(CUtensorMap *map, const void *base, uint64_t tiles, int tiles_per_stage) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {kSfTileBytes / 4, tiles};
   cuuint64_t strides[1] = {kSfTileBytes};
-  cuuint32_t box[2] = {kSfTileBytes / 4, static_cast<cuuint32_t>(kMmasPerStage)};
+  cuuint32_t box[2] = {kSfTileBytes / 4, static_cast<cuuint32_t>(tiles_per_stage)};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1228,8 +1199,8 @@ cudaError_t launch_one(const GemmArgs &a, KernelParams kp, uint64_t row_bytes, c
   CUtensorMap tsfa = ta, tsfb = tb;  // only dereferenced by the block-scaled kind
   if constexpr (KIND == kKindNvf4) {
     const uint64_t k_tiles = static_cast<uint64_t>(a.sf_k_tiles);
-    if (!make_tmap_sf(&tsfa, a.sfa, static_cast<uint64_t>((a.m + 127) / 128) * k_tiles) ||
-        !make_tmap_sf(&tsfb, a.sfb, static_cast<uint64_t>((a.n + 127) / 128 + 1) * k_tiles)) {
+    if (!make_tmap_sf(&tsfa, a.sfa, static_cast<uint64_t>((a.m + 127) / 128) * k_tiles, kMmasPerStage) ||
+        !make_tmap_sf(&tsfb, a.sfb, static_cast<uint64_t>(kp.tiles_n) * (k_tiles / kMmasPerStage) * Cfg::kSfbCopies, Cfg::kSfbCopies)) {
       *why = "cuTensorMapEncodeTiled refused the scale factors";
       return cudaErrorInvalidValue;
     }

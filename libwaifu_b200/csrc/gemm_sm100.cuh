@@ -20,6 +20,12 @@ enum Activation : int { kActNone = 0, kActGeluTanh = 1 };
 
 constexpr int kMaxGemmOutputs = 8;
 
+// The four-bit kind's tile width, and how the weight's block scales are laid out for it: per tile
+// of kNvf4BlockN rows and per K stage of 16 blocks, 24 columns of tensor memory (four instructions
+// x 6 columns of 32 rows x 4 factors) as six 512-byte tiles of 32 rows x 4 columns x 4 bytes.
+constexpr int kNvf4BlockN = 192;
+constexpr int kNvf4SfbTiles = 4 * (kNvf4BlockN / 32) / 4;
+
 // Status words the kernels write when a bounded wait runs out.
 enum : uint32_t {
   kStatusOk = 0,
@@ -35,8 +41,9 @@ struct GemmArgs {
   const void *a;  // (m, k)
   const void *b;  // (n, k); with b_is_e4m3 (kGemmF16 only), e4m3 bytes that the kernel widens to half, exactly
   int b_is_e4m3;
-  // NVFP4 only: scale factors in the 128-row x 4-factor tile layout the tensor cores read
-  // (see pack_scale_factors()), and how many 4-factor tiles one row group holds along k.
+  // NVFP4 only: the activation's scale factors in the 128-row x 4-factor tile layout the tensor
+  // cores read, the weight's in the layout above (nvfp4_prepare() writes both), and how many
+  // 4-factor tiles one row group of the activation holds along k.
   const uint8_t *sfa;
   const uint8_t *sfb;
   int sf_k_tiles;

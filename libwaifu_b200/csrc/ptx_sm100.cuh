@@ -170,6 +170,29 @@ __device__ __forceinline__ void e4m3x4_to_f16x4(uint32_t codes, uint32_t *lo, ui
       : "r"(codes));
 }
 
+// Sixteen e4m3 codes (lowest byte first) as sixteen halves; exact.
+__device__ __forceinline__ void e4m3x16_to_f16(const uint4 codes, uint4 *lo, uint4 *hi) {
+  e4m3x4_to_f16x4(codes.x, &lo->x, &lo->y);
+  e4m3x4_to_f16x4(codes.y, &lo->z, &lo->w);
+  e4m3x4_to_f16x4(codes.z, &hi->x, &hi->y);
+  e4m3x4_to_f16x4(codes.w, &hi->z, &hi->w);
+}
+
+// 0.5 x (1 + tanh(u)) == x * sigmoid(2u) == x / (1 + 2^z), u = sqrt(2/pi) (x + 0.044715 x^3),
+// z = -2 u log2(e) = x (c0 + c1 x^2)
+// (waifu/src/krea2/dit.rs:170-188 spells the same function as seven graph nodes).
+// Five FP32 operations and two special-function operations; both approximations are good to
+// about 2^-22, far inside the 16-bit output step. x -> -inf gives 2^z = inf, 1/inf = 0, -0.
+__device__ __forceinline__ float gelu_tanh(float x) {
+  constexpr float kC0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
+  constexpr float kC1 = kC0 * 0.044715f;
+  const float z = x * fmaf(x * x, kC1, kC0);
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
+  return x * r;
+}
+
 // ---- TMA ---------------------------------------------------------------------------------
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *desc) {

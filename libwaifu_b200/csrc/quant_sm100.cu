@@ -652,31 +652,17 @@ __device__ __forceinline__ void nvfp4_act_block(const uint16_t *__restrict__ x, 
   sf_tiled[sf_tiled_offset(r, b, sf_k_tiles)] = sc;
 }
 
-// One thread per 16-element block of a 16-bit activation.
-__global__ void __launch_bounds__(256) quantize_nvfp4_act_kernel(const uint16_t *__restrict__ x, int is_bf16, int m,
-                                                               int k, uint8_t *__restrict__ codes,
-                                                               uint8_t *__restrict__ sf_tiled, int sf_k_tiles,
-                                                               int vec_ok) {
-  griddep_wait();
-  griddep_launch_dependents();
-  const int blocks_per_row = k / 16;
-  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<int64_t>(m) * blocks_per_row) return;
-  nvfp4_act_block(x, is_bf16, k, static_cast<int>(idx / blocks_per_row), static_cast<int>(idx % blocks_per_row), codes,
-                  sf_tiled, sf_k_tiles, vec_ok);
-}
-
 // Everything fl_nvfp4_linear does ahead of its GEMM in one launch (two clears, the activation
 // quantiser and the re-tiling of the weight's block scales were four, with a launch gap each).
 // CTAs [0, a_ctas): one thread per 16-element block of the activation over the whole tiled domain
 // (row groups of 128, K tiles of 4 blocks, `sf_k_tiles` per group): a block of the activation is
 // quantised, one of the padding gets the scale factor 0. The other CTAs: one thread per 4 block
-// scales of the weight (a 32-bit word of the tile layout) over its tiled domain and one spare row
-// group, zeros outside the weight. Nothing has to be cleared beforehand.
+// scales of the weight (a 32-bit word) over whole tiles of kNvf4BlockN rows and whole K stages,
+// zeros outside the weight. Nothing has to be cleared beforehand.
 __global__ void __launch_bounds__(256) nvfp4_prepare_kernel(const uint16_t *__restrict__ x, int is_bf16, int m, int k,
                                                           uint8_t *__restrict__ codes, uint8_t *__restrict__ sfa_tiled,
                                                           int sf_k_tiles, int vec_ok, int a_ctas,
-                                                          const uint8_t *__restrict__ wsf_plain, int rows, int w_groups,
+                                                          const uint8_t *__restrict__ wsf_plain, int rows,
                                                           uint8_t *__restrict__ sfb_tiled) {
   griddep_wait();
   griddep_launch_dependents();
@@ -695,9 +681,9 @@ __global__ void __launch_bounds__(256) nvfp4_prepare_kernel(const uint16_t *__re
     return;
   }
   const int64_t idx = static_cast<int64_t>(static_cast<int>(blockIdx.x) - a_ctas) * blockDim.x + threadIdx.x;
-  const int64_t total = static_cast<int64_t>(w_groups) * 128 * sf_k_tiles;
+  const int64_t total = static_cast<int64_t>((rows + kNvf4BlockN - 1) / kNvf4BlockN) * kNvf4BlockN * sf_k_tiles;
   if (idx >= total) return;
-  const int r = static_cast<int>(idx / sf_k_tiles), t4 = static_cast<int>(idx % sf_k_tiles) * 4;
+  const int r = static_cast<int>(idx / sf_k_tiles), kt = static_cast<int>(idx % sf_k_tiles), t4 = kt * 4;
   uint32_t word = 0;
   if (r < rows) {
     const uint8_t *src = wsf_plain + static_cast<int64_t>(r) * kblocks + t4;
@@ -706,7 +692,10 @@ __global__ void __launch_bounds__(256) nvfp4_prepare_kernel(const uint16_t *__re
       if (t4 + j < kblocks) word |= static_cast<uint32_t>(src[j]) << (8 * j);
     }
   }
-  *reinterpret_cast<uint32_t *>(sfb_tiled + sf_tiled_offset(r, t4, sf_k_tiles)) = word;
+  const int tile = r / kNvf4BlockN, in_tile = r % kNvf4BlockN;
+  const int col = (kt % 4) * (kNvf4BlockN / 32) + in_tile / 32;  // of the stage's 24
+  const int64_t sf_tile = (static_cast<int64_t>(tile) * (sf_k_tiles / 4) + kt / 4) * kNvf4SfbTiles + col / 4;
+  *reinterpret_cast<uint32_t *>(sfb_tiled + sf_tile * 512 + (in_tile % 32) * 16 + (col % 4) * 4) = word;
 }
 
 __global__ void __launch_bounds__(256) amax_f32_kernel(const float *__restrict__ w, int64_t numel, uint32_t *amax_word) {
@@ -742,15 +731,6 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_weight_kernel(const float 
 #pragma unroll
   for (int j = 0; j < 8; ++j) dst[j] = static_cast<uint8_t>(packed[j >> 2] >> ((j & 3) * 8));
   sf_plain[idx] = sc;
-}
-
-__global__ void __launch_bounds__(256) pack_sf_kernel(const uint8_t *__restrict__ sf_plain, int rows, int kblocks,
-                                                    uint8_t *__restrict__ sf_tiled, int sf_k_tiles) {
-  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<int64_t>(rows) * kblocks) return;
-  const int r = static_cast<int>(idx / kblocks);
-  const int b = static_cast<int>(idx % kblocks);
-  sf_tiled[sf_tiled_offset(r, b, sf_k_tiles)] = sf_plain[idx];
 }
 
 // ---- widening and gathers --------------------------------------------------------------------
@@ -945,32 +925,11 @@ cudaError_t quantize_fp8_rows_f32(const float *w, int rows, int k, uint8_t *code
   return cudaGetLastError();
 }
 
-cudaError_t quantize_nvfp4_act(const void *x, int is_bf16, int m, int k, uint8_t *codes, uint8_t *sf_tiled,
-                               cudaStream_t stream) {
-  const int64_t blocks = static_cast<int64_t>(m) * (k / 16);
-  const int grid = static_cast<int>((blocks + 255) / 256);
-  const int vec = aligned16(x) && (reinterpret_cast<uintptr_t>(codes) & 7) == 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, quantize_nvfp4_act_kernel, static_cast<const uint16_t *>(x), is_bf16, m, k, codes,
-                                     sf_tiled, sf_k_tiles_for(k), vec);
-  ++g_helper_launches;
-  return e;
-}
-
 cudaError_t nvfp4_prepare(const void *x, int is_bf16, int m, int k, uint8_t *codes, uint8_t *sfa_tiled,
-                          const uint8_t *wsf_plain, int rows, int w_extra_groups, uint8_t *sfb_tiled, cudaStream_t stream) {
+                          const uint8_t *wsf_plain, int rows, uint8_t *sfb_tiled, cudaStream_t stream) {
   const int sf_k_tiles = sf_k_tiles_for(k);
   const int64_t a_threads = static_cast<int64_t>((m + 127) / 128) * 128 * sf_k_tiles * 4;
-  const int w_groups = (rows + 127) / 128 + w_extra_groups;
-  const int64_t b_threads = static_cast<int64_t>(w_groups) * 128 * sf_k_tiles;
+  const int64_t b_threads = static_cast<int64_t>((rows + kNvf4BlockN - 1) / kNvf4BlockN) * kNvf4BlockN * sf_k_tiles;
   const int a_ctas = static_cast<int>((a_threads + 255) / 256), b_ctas = static_cast<int>((b_threads + 255) / 256);
   const int vec = aligned16(x) && (reinterpret_cast<uintptr_t>(codes) & 7) == 0;
   cudaLaunchConfig_t cfg = {};
@@ -983,7 +942,7 @@ cudaError_t nvfp4_prepare(const void *x, int is_bf16, int m, int k, uint8_t *cod
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, nvfp4_prepare_kernel, static_cast<const uint16_t *>(x), is_bf16, m, k, codes,
-                                     sfa_tiled, sf_k_tiles, vec, a_ctas, wsf_plain, rows, w_groups, sfb_tiled);
+                                     sfa_tiled, sf_k_tiles, vec, a_ctas, wsf_plain, rows, sfb_tiled);
   ++g_helper_launches;
   return e;
 }
@@ -999,15 +958,6 @@ cudaError_t quantize_nvfp4_weight_f32(const float *w, int rows, int k, uint8_t *
   quantize_nvfp4_weight_kernel<<<static_cast<int>((blocks + 255) / 256), 256, 0, stream>>>(w, rows, k, global_scale,
                                                                                           codes, sf_plain);
   g_helper_launches += 3;
-  return cudaGetLastError();
-}
-
-cudaError_t pack_scale_factors(const uint8_t *sf_plain, int rows, int k, uint8_t *sf_tiled, cudaStream_t stream) {
-  const int kblocks = k / 16;
-  const int64_t n = static_cast<int64_t>(rows) * kblocks;
-  pack_sf_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, stream>>>(sf_plain, rows, kblocks, sf_tiled,
-                                                                       sf_k_tiles_for(k));
-  ++g_helper_launches;
   return cudaGetLastError();
 }
 

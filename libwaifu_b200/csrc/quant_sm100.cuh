@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gemm_sm100.cuh"
+
 namespace flsm100 {
 
 // Per-row (token) e4m3: scales[r] = amax_r / 448, codes = e4m3_rn_sat(x * (1 / scales[r])) with
@@ -37,30 +39,26 @@ cudaError_t ln_modulate_quantize_fp8(const void *x, int is_bf16, int m, int k, c
                                      const void *shift, int64_t shift_pitch, int rows_per_group, float eps,
                                      uint8_t *codes, float *row_scales, cudaStream_t stream);
 
-// Scale factors of a (rows, k/16) operand in the tile layout the block-scaled MMA reads: tiles
+// Scale factors of the (m, k/16) activation in the tile layout the block-scaled MMA reads: tiles
 // of 128 rows x 4 factors (512 bytes), byte (r % 32) * 16 + ((r % 128) / 32) * 4 + (b % 4) of
 // tile (r / 128, b / 4); tiles of one row group are consecutive, `sf_k_tiles` per group.
 inline int sf_k_tiles_for(int k) { return ((k / 16 + 3) / 4 + 3) / 4 * 4; }
-inline int64_t sf_tiled_bytes(int rows, int k, int extra_groups) {
-  return static_cast<int64_t>((rows + 127) / 128 + extra_groups) * sf_k_tiles_for(k) * 512;
+inline int64_t sfa_tiled_bytes(int m, int k) { return static_cast<int64_t>((m + 127) / 128) * sf_k_tiles_for(k) * 512; }
+// The weight's, in the layout of kNvf4BlockN-row tiles (gemm_sm100.cuh).
+inline int64_t sfb_tiled_bytes(int rows, int k) {
+  return static_cast<int64_t>((rows + kNvf4BlockN - 1) / kNvf4BlockN) * (sf_k_tiles_for(k) / 4) * kNvf4SfbTiles * 512;
 }
 
-// Per-16-block e2m1 with unsigned-e4m3 block scales, global scale 1; codes (m, k/2) row-major,
-// scale factors written straight into the tile layout (`sf_tiled` zeroed by the caller).
-cudaError_t quantize_nvfp4_act(const void *x, int is_bf16, int m, int k, uint8_t *codes, uint8_t *sf_tiled,
-                               cudaStream_t stream);
-// What fl_nvfp4_linear needs ahead of its GEMM, in one launch: the activation's codes and tiled
-// scale factors (quantize_nvfp4_act) and the weight's plain (rows, k/16) block scales in the tile
-// layout with `w_extra_groups` spare row groups (pack_scale_factors), padding written as zeros, so
-// neither destination has to be cleared first.
+// What fl_nvfp4_linear needs ahead of its GEMM, in one launch: the activation as e2m1 codes (m, k/2)
+// with unsigned-e4m3 scales per 16 (global scale 1) in the tile layout, and the weight's plain
+// (rows, k/16) block scales in theirs; padding is written as zeros, so neither destination has to
+// be cleared first.
 cudaError_t nvfp4_prepare(const void *x, int is_bf16, int m, int k, uint8_t *codes, uint8_t *sfa_tiled,
-                          const uint8_t *wsf_plain, int rows, int w_extra_groups, uint8_t *sfb_tiled, cudaStream_t stream);
+                          const uint8_t *wsf_plain, int rows, uint8_t *sfb_tiled, cudaStream_t stream);
 // NVFP4 weight from fp32: global = amax / (448 * 6); plain (rows, k/16) block scales.
 // `amax_word` is a device word used for the reduction.
 cudaError_t quantize_nvfp4_weight_f32(const float *w, int rows, int k, uint8_t *codes, uint8_t *sf_plain,
                                       float *global_scale, uint32_t *amax_word, cudaStream_t stream);
-// Plain (rows, k/16) scale factors -> tile layout (`sf_tiled` zeroed by the caller).
-cudaError_t pack_scale_factors(const uint8_t *sf_plain, int rows, int k, uint8_t *sf_tiled, cudaStream_t stream);
 
 // flint's swiglu (first half of the last dimension the gate, second the value; silu(g) * v in fp32,
 // narrowed to 16 bits: flint/cpu/glu.cc:36-67) on x (m, 2 h), then per-row e4m3 of the (m, h)
