@@ -655,14 +655,25 @@ constexpr int kTileWarps = 4;
 constexpr int kSoftmaxWarps2 = kTiles * kTileWarps;
 constexpr int kProducerWarp2 = kSoftmaxWarps2;
 constexpr int kMmaWarp2 = kSoftmaxWarps2 + 1;
-constexpr int kThreads2 = (kSoftmaxWarps2 + 2) * 32;
+// Twelve warps, three warpgroups, launched with 168 registers a thread; the one that loads and issues
+// (two of its warps have nothing to do) gives its own up to the two of the softmax, which hold a
+// row of 128 scores: 128 x 88 + 256 x 208 = 384 x 168.
+constexpr int kThreads2 = (kSoftmaxWarps2 + 4) * 32;
+constexpr int kIssueRegs = 88, kSoftmaxRegs = 208;
+static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2 * 168, "no more than the block was launched with");
+// A block's probabilities are handed over in so many parts of its keys. At head_dim 128 the product of
+// the first half runs under the exponentials of the second (2 x 24 x 4352: 396 -> 386 us); at 64,
+// where the products are half as long, one hand-over less is worth more (2 x 8 x 1000 x 2000: 34.6 us
+// in halves, 32.1 whole).
+template <int D>
+constexpr int kPartsOf = D == 128 ? 2 : 1;
 constexpr int kMaxSlots = 6;
 
 struct Tail2 {
   uint64_t q_full_bar[kTiles];
   uint64_t slot_full_bar[kMaxSlots], slot_empty_bar[kMaxSlots];
   uint64_t s_full_bar[kTiles];   // MMA -> softmax: the tile's scores are in tensor memory
-  uint64_t p_full_bar[kTiles];   // softmax -> MMA: the tile's probabilities are in tensor memory
+  uint64_t p_full_bar[kTiles][2];  // softmax -> MMA: that part of the tile's probabilities is in tensor memory
   uint64_t pv_done_bar[kTiles];  // MMA -> softmax: the block is in the tile's output
   uint32_t tmem_base_slot;
   uint32_t abort_flag;
@@ -696,6 +707,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                   const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
   using L = Layout2<D>;
   constexpr int S = L::kSlots;
+  constexpr int kPParts = kPartsOf<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   Tail2 &t = *reinterpret_cast<Tail2 *>(smem + L::kTailOff);
   volatile uint32_t &abort_flag = *reinterpret_cast<volatile uint32_t *>(&t.abort_flag);
@@ -706,11 +718,18 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (threadIdx.x == 0) atomicCAS(p.status, 0u, kStatusAttentionLayout);
     return;
   }
-  // Under a causal mask the later queries have more keys to walk: those CTAs go first, so that the
-  // grid's last round is made of short ones.
-  const int q0 = static_cast<int>(p.mask_type != 0 ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * (kTiles * kBlockQ);
-  const int head = blockIdx.y;
-  const int batch = blockIdx.z;
+  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its keys and values in L2. Under
+  // the causal masks the later queries have more keys to walk: the last unit of every head goes
+  // first, then the one before it, so that the grid ends on the short ones whatever the head.
+  int unit = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
+  if (p.mask_type != 0) {
+    const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
+    const int order = unit + units * (head + heads * batch);
+    unit = units - 1 - order / all;
+    head = order % all % heads;
+    batch = order % all / heads;
+  }
+  const int q0 = unit * (kTiles * kBlockQ);
   const int kv_head = head / p.group;
   const int offset = p.kv_len - p.q_len;
   // Both tiles walk the blocks of keys that some query of the CTA sees; a block none of a tile's
@@ -720,6 +739,13 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int kv_end = last_key_of(p, last_row + offset) + 1;
   const int block0 = kv_begin / kBlockKv;
   const int num_blocks = (kv_end + kBlockKv - 1) / kBlockKv - block0;
+  // Under the causal masks the first tile's queries see nothing of the last blocks the second walks;
+  // a tile past the last query has none.
+  auto blocks_of = [&](int i) -> int {
+    if (q0 + i * kBlockQ >= p.q_len) return 0;
+    const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
+    return min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv - block0);
+  };
 
   if (threadIdx.x == 0) {
     t.abort_flag = 0;
@@ -730,7 +756,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     for (int i = 0; i < kTiles; ++i) {
       mbar_init(&t.q_full_bar[i], 1);
       mbar_init(&t.s_full_bar[i], 1);
-      mbar_init(&t.p_full_bar[i], kTileWarps);
+      for (int h = 0; h < kPParts; ++h) mbar_init(&t.p_full_bar[i][h], kTileWarps);
       mbar_init(&t.pv_done_bar[i], 1);
     }
     fence_barrier_init();
@@ -753,143 +779,8 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   auto slot = [&](int i) { return smem + L::kSlotOff + i * L::kSlotBytes; };
 
   // Load n of the ring (K of block n / 2 when n is even, V of it when odd) goes to slot n % S.
-  if (warp == kProducerWarp2) {
-    // ------------------------------------------------------------------ producer
-    if (elect_one()) {
-      bool ok = true;
-      for (int i = 0; i < kTiles; ++i) {
-        mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
-#pragma unroll
-        for (int a = 0; a < L::kQAtoms; ++a) {
-          tma_load_4d(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, q0 + i * kBlockQ, head,
-                      batch);
-        }
-      }
-      for (int n = 0; n < 2 * num_blocks && ok; ++n) {
-        const int st = n % S, j = n >> 1;
-        if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
-          ok = false;
-          break;
-        }
-        mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
-        if ((n & 1) == 0) {
-#pragma unroll
-          for (int a = 0; a < L::kQAtoms; ++a) {
-            tma_load_4d(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes,
-                        (block0 + j) * kBlockKv, kv_head, batch);
-          }
-        } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
-#pragma unroll
-          for (int a = 0; a < L::kQAtoms; ++a) {
-            tma_load_4d(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes,
-                        (block0 + j) * kBlockKv, kv_head, batch);
-          }
-        } else {
-#pragma unroll
-          for (int a = 0; a < L::kVAtoms; ++a) {
-            tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st],
-                        ((block0 + j) * kBlockKv + a * kAtomElems) * 2, 0, batch * p.kv_heads + kv_head);
-          }
-        }
-      }
-      if (!ok) {
-        abort_flag = 1;
-        atomicCAS(p.status, 0u, kStatusAttentionTimeout);
-      }
-    }
-  } else if (warp == kMmaWarp2) {
-    // ------------------------------------------------------------------ MMA issuer
-    // The whole warp walks the loop and one lane issues: what an instruction takes (descriptors,
-    // addresses) is then the same in every lane, which lets it live in uniform registers instead of
-    // being moved there instruction by instruction by a lone thread.
-    const bool issuer = elect_one();
-    {
-      const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-      const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
-      const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
-      constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
-      constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
-      constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
-      constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
-      const uint64_t qdesc0 = umma_desc_sw128(smem_u32(q_tile(0)));
-      const uint64_t sdesc0 = umma_desc_sw128(smem_u32(slot(0)));
-      bool ok = true;
-      auto scores = [&](int i, uint64_t kd) {  // S_i = Q_i K^T
-        const uint32_t s_tmem = tmem_base + i * L::kSCols;
-        const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
-#pragma unroll
-        for (int m = 0; m < kScoreMmas; ++m) {
-          const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-          if (issuer) umma_ss<kKindF16>(s_tmem, qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep),
-                            kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep), idesc_s, m != 0 ? 1u : 0u);
-        }
-      };
-      // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes
-      // on, the operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64
-      // head_dim positions lie a 128-key atom apart.
-      const uint32_t idesc_o_mn = idesc_o | (1u << 16);
-      const uint64_t mn_fields = umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0);
-      auto product = [&](int i, uint64_t vd, uint32_t first_block) {  // O_i += P_i V
-        const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
-        const uint32_t p_tmem = tmem_base + i * L::kSCols;
-        if (p.v_direct) {
-#pragma unroll
-          for (int m = 0; m < kOutMmas; ++m) {
-            if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4)), idesc_o_mn,
-                        m != 0 ? 1u : (first_block ^ 1u));
-          }
-        } else {
-#pragma unroll
-          for (int m = 0; m < kOutMmas; ++m) {
-            const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-            if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
-                        m != 0 ? 1u : (first_block ^ 1u));
-          }
-        }
-      };
-      auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
-      auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
-      for (int i = 0; i < kTiles && ok; ++i) ok = mbar_wait(&t.q_full_bar[i], 0, &abort_flag);
-      if (ok && num_blocks > 0) ok = wait_full(0);
-      if (ok && num_blocks > 0) {
-        tc_fence_after_sync();
-        for (int i = 0; i < kTiles; ++i) {
-          scores(i, desc_of(0));
-          if (issuer) umma_commit(&t.s_full_bar[i]);
-        }
-        if (issuer) umma_commit(&t.slot_empty_bar[0]);
-      }
-      for (int j = 0; j < num_blocks && ok; ++j) {
-        const bool more = j + 1 < num_blocks;
-        const int nv = 2 * j + 1, nk = 2 * j + 2;
-        const uint32_t first_block = j == 0 ? 1u : 0u;
-        for (int i = 0; i < kTiles && ok; ++i) {
-          // (The second tile reads the slots the first one has just been seen to wait for.)
-          if (!mbar_wait(&t.p_full_bar[i], j & 1, &abort_flag) || (i == 0 && (!wait_full(nv) || (more && !wait_full(nk))))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          // The product reads P from the columns the next scores overwrite: the instructions of one
-          // thread run in the order they were issued.
-          product(i, desc_of(nv), first_block);
-          if (!more && issuer) umma_commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
-          if (more) {
-            scores(i, desc_of(nk));
-            if (issuer) umma_commit(&t.s_full_bar[i]);
-          }
-          if (i == kTiles - 1) {  // both tiles have read the two slots
-            if (issuer) umma_commit(&t.slot_empty_bar[nv % S]);
-            if (more && issuer) umma_commit(&t.slot_empty_bar[nk % S]);
-          }
-        }
-      }
-      if (!ok && issuer) {
-        abort_flag = 1;
-        atomicCAS(p.status, 0u, kStatusAttentionTimeout);
-      }
-    }
-  } else {
+  if (warp < kSoftmaxWarps2) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
     // ------------------------------------------------------------------ softmax and output
     const int tile = static_cast<int>(warp >> 2);
     const uint32_t quarter = warp & 3;
@@ -912,7 +803,8 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     bool ok = true;
     uint32_t sc[kChunks][32];
 
-    for (int j = 0; j < num_blocks && ok; ++j) {
+    const int my_blocks = blocks_of(tile);
+    for (int j = 0; j < my_blocks && ok; ++j) {
       // The row's scores of the block into registers in one round trip. (Scores of block j are
       // issued behind the product of block j - 1: once they are here the tile's output is complete
       // up to that block.)
@@ -962,14 +854,15 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         m_used = m_new;
       }
       const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
       // (a slot whose scores have been used by then).
       const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
-      auto emit = [&](auto bf16_tag) {
+      uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
+      auto emit = [&](auto bf16_tag, int part) {
         constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
+        for (int h = 0; h < kChunks / kPParts; ++h) {
+          const int c = part * (kChunks / kPParts) + h;
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
@@ -982,26 +875,34 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             } else {
               exp2_pair_poly(x, &e0, &e1);
             }
-            sum4[(i >> 1) & 3] += e0 + e1;
+            sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
             sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
           }
         }
       };
-      if (p.is_bf16) {
-        emit(std::true_type{});
-      } else {
-        emit(std::false_type{});
+      // Each half of the block's keys is handed over as soon as it is there: its product runs under
+      // the exponentials of the other half.
+#pragma unroll
+      for (int part = 0; part < kPParts; ++part) {
+        if (p.is_bf16) {
+          emit(std::true_type{}, part);
+        } else {
+          emit(std::false_type{}, part);
+        }
+        tmem_st_32x32(t_scores + part * 32, sc[part]);
+        if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
+        tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
+        tc_fence_before_sync();  // before the MMAs that the hand-over starts
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
       }
-      l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      tmem_st_32x32(t_scores, sc[0]);
-      tmem_st_32x32(t_scores + 32, sc[1]);
-      tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
-      tc_fence_before_sync();  // before the MMAs that the hand-over starts
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&t.p_full_bar[tile]);
+      float s0, s1, s2, s3;
+      f2_unpack(sums[0], &s0, &s1);
+      f2_unpack(sums[1], &s2, &s3);
+      l_run += (s0 + s1) + (s2 + s3);
     }
     // The last product.
-    if (ok && num_blocks > 0) {
+    if (ok && my_blocks > 0) {
       ok = __all_sync(0xffffffffu, mbar_wait(&t.pv_done_bar[tile], 0, &abort_flag));
       tc_fence_after_sync();
     }
@@ -1031,6 +932,164 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (!ok && lane == 0) {
       abort_flag = 1;
       atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+    }
+    } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == kProducerWarp2) {
+      // ------------------------------------------------------------------ producer
+      if (elect_one()) {
+        bool ok = true;
+        auto load = [&](void *dst, const CUtensorMap *map, uint64_t *bar, int32_t c0, int32_t c1, int32_t c2) {
+          tma_load_4d(dst, map, bar, c0, c1, c2, batch);
+        };
+        for (int i = 0; i < kTiles; ++i) {
+          mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
+#pragma unroll
+          for (int a = 0; a < L::kQAtoms; ++a) {
+            load(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, q0 + i * kBlockQ, head);
+          }
+        }
+        for (int n = 0; n < 2 * num_blocks && ok; ++n) {
+          const int st = n % S, j = n >> 1;
+          if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
+          const int key0 = (block0 + j) * kBlockKv;
+          if ((n & 1) == 0) {
+#pragma unroll
+            for (int a = 0; a < L::kQAtoms; ++a) {
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+            }
+          } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
+#pragma unroll
+            for (int a = 0; a < L::kQAtoms; ++a) {
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+            }
+          } else {
+#pragma unroll
+            for (int a = 0; a < L::kVAtoms; ++a) {
+              tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st], (key0 + a * kAtomElems) * 2, 0,
+                          batch * p.kv_heads + kv_head);
+            }
+          }
+        }
+        if (!ok) {
+          abort_flag = 1;
+          atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+        }
+      }
+    } else if (warp == kMmaWarp2) {
+      // ------------------------------------------------------------------ MMA issuer
+      // The whole warp walks the loop and one lane issues: what an instruction takes (descriptors,
+      // addresses) is then the same in every lane, which lets it live in uniform registers instead of
+      // being moved there instruction by instruction by a lone thread.
+      const bool issuer = elect_one();
+      {
+        const uint32_t fmt = p.is_bf16 ? 1u : 0u;
+        const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
+        const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
+        constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
+        constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
+        constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
+        constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
+        const uint64_t qdesc0 = umma_desc_sw128(smem_u32(q_tile(0)));
+        const uint64_t sdesc0 = umma_desc_sw128(smem_u32(slot(0)));
+        bool ok = true;
+        auto commit = [&](uint64_t *bar) {
+          if (issuer) umma_commit(bar);
+        };
+        auto scores = [&](int i, uint64_t kd) {  // S_i = Q_i K^T
+          const uint32_t s_tmem = tmem_base + i * L::kSCols;
+          const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
+#pragma unroll
+          for (int m = 0; m < kScoreMmas; ++m) {
+            const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+            const uint64_t qa = qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep);
+            const uint64_t ka = kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep);
+            if (issuer) umma_ss<kKindF16>(s_tmem, qa, ka, idesc_s, m != 0 ? 1u : 0u);
+          }
+        };
+        // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes
+        // on, the operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64
+        // head_dim positions lie a 128-key atom apart.
+        const uint32_t idesc_o_mn = idesc_o | (1u << 16);
+        const uint64_t mn_fields = umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0);
+        auto product = [&](int i, int part, uint64_t vd, uint32_t first_block) {  // O_i += P_i V over one part of the block's keys
+          const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
+          const uint32_t p_tmem = tmem_base + i * L::kSCols;
+          constexpr int kPartMmas = kOutMmas / kPParts;
+          if (p.v_direct) {
+#pragma unroll
+            for (int k = 0; k < kPartMmas; ++k) {
+              const int m = part * kPartMmas + k;
+              const uint64_t va = (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4));
+              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, va, idesc_o_mn, m != 0 ? 1u : (first_block ^ 1u));
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < kPartMmas; ++k) {
+              const int m = part * kPartMmas + k;
+              const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
+                          m != 0 ? 1u : (first_block ^ 1u));
+            }
+          }
+        };
+        auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
+        auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
+        const int blocks[kTiles] = {blocks_of(0), blocks_of(1)};
+        for (int i = 0; i < kTiles && ok; ++i) ok = mbar_wait(&t.q_full_bar[i], 0, &abort_flag);
+        if (ok && num_blocks > 0) ok = wait_full(0);
+        if (ok && num_blocks > 0) {
+          tc_fence_after_sync();
+#pragma unroll
+          for (int i = 0; i < kTiles; ++i) {
+            if (blocks[i] == 0) continue;
+            scores(i, desc_of(0));
+            commit(&t.s_full_bar[i]);
+          }
+          commit(&t.slot_empty_bar[0]);
+        }
+        for (int j = 0; j < num_blocks && ok; ++j) {
+          const bool more = j + 1 < num_blocks;
+          const int nv = 2 * j + 1, nk = 2 * j + 2;
+          if (!wait_full(nv)) ok = false;
+#pragma unroll
+          for (int i = 0; i < kTiles; ++i) {
+            if (!ok || j >= blocks[i]) continue;
+            // The product reads P from the columns the next scores overwrite: the instructions of one
+            // thread run in the order they were issued.
+#pragma unroll
+            for (int part = 0; part < kPParts; ++part) {
+              if (ok) ok = mbar_wait(&t.p_full_bar[i][part], j & 1, &abort_flag);
+              if (!ok) break;
+              tc_fence_after_sync();
+              product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
+            }
+            if (!ok) continue;
+            if (j + 1 == blocks[i]) {
+              commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
+            } else {
+              if (!wait_full(nk)) {  // (seen by the first tile's turn, for the second's too)
+                ok = false;
+                continue;
+              }
+              tc_fence_after_sync();
+              scores(i, desc_of(nk));
+              commit(&t.s_full_bar[i]);
+            }
+          }
+          if (!ok) break;
+          commit(&t.slot_empty_bar[nv % S]);  // both tiles have read the two slots
+          if (more) commit(&t.slot_empty_bar[nk % S]);
+        }
+        if (!ok && issuer) {
+          abort_flag = 1;
+          atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+        }
+      }
     }
   }
 
