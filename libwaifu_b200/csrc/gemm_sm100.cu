@@ -67,6 +67,11 @@ constexpr int kNumWarps = 12;
 constexpr int kNumThreads = kNumWarps * 32;
 constexpr int kMaxEpilogueWarps = 8;
 constexpr int kPusherWarps = 2;
+// Mixed form: the converter warps share out the stages of the ring, two warps to a stage (slot s
+// belongs to group s % 3, so a group sees every phase of the barriers it waits on). A stage's way
+// through a warp (wait, read, widen, write, proxy fence, arrive) is some 0.4 us however few bytes
+// it has; with all six warps on every stage that was what paced the kernel.
+constexpr int kConverterGroups = 3;
 // Who does what among the twelve warps. Tensor memory lets a warp read the 32 lanes of its index
 // modulo 4 only, so epilogue warps come in fours, each four covering a tile's 128 rows and one
 // share of its columns. The mixed form gives up one of the two fours to have six converter warps:
@@ -325,8 +330,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     abort_flag = 0;
     for (int s = 0; s < STAGES; ++s) {
       // Mixed form: a stage is full when the A bytes have landed (the producer's arrival with
-      // its byte count) and every converter warp of the unit has written its share of B.
-      mbar_init(&full_bar[s], B8 ? 1 + kConverterWarps * CTAS : 1);
+      // its byte count) and every converter warp that has the stage has written its share of B.
+      mbar_init(&full_bar[s], B8 ? 1 + kConverterWarps / kConverterGroups * CTAS : 1);
       mbar_init(&empty_bar[s], 1);
       if constexpr (B8) mbar_init(&raw_full_bar[s], 1);
     }
@@ -610,7 +615,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // 128-byte swizzle (piece index xor row % 8). A warp's 32 lanes take 8 rows x 4 pieces: the
     // reads are 512 contiguous bytes, the writes touch every bank four times, which is the least
     // 512 bytes can.
-    const int cw = static_cast<int>(warp) - kPusherWarp0;
+    constexpr int kGroupWarps = B8 ? kConverterWarps / kConverterGroups : 1;
+    const int cw = (static_cast<int>(warp) - kPusherWarp0) % kGroupWarps;
+    const int group = (static_cast<int>(warp) - kPusherWarp0) / kGroupWarps;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -618,6 +625,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     WorkItem item;
     while (ok && walk.next(&item)) {
       for (int kb = item.kb0; kb < item.kb1; ++kb) {
+        if (stage % kConverterGroups != group) {
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+          continue;
+        }
         if (!mbar_wait(&raw_full_bar[stage], phase, &abort_flag)) {
           ok = false;
           break;
@@ -625,7 +639,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const uint8_t *raw = stage_raw(stage);
         uint8_t *b16 = stage_b(stage);
 #pragma unroll 4
-        for (int piece = cw * 32 + static_cast<int>(lane); piece < Cfg::kBRows * 4; piece += kConverterWarps * 32) {
+        for (int piece = cw * 32 + static_cast<int>(lane); piece < Cfg::kBRows * 4; piece += kGroupWarps * 32) {
           const uint32_t r = static_cast<uint32_t>(piece) >> 2, q = static_cast<uint32_t>(piece) & 3;
           const uint4 v = *reinterpret_cast<const uint4 *>(raw + piece * 16);
           uint4 lo, hi;
