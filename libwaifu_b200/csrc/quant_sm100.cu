@@ -148,6 +148,49 @@ __global__ void __launch_bounds__(256) quantize_fp8_act_reg_kernel(const uint16_
   }
 }
 
+// The same with a warp to a row (k <= 256 * VPT), eight rows to a CTA: nothing waits for another warp,
+// a lane has up to sixteen 16-byte loads on their way, and the maximum is taken on pairs as they
+// lie (max of abs in the 16-bit type, exact; NaNs are passed over as fmaxf passes over them).
+template <int VPT>
+__global__ void __launch_bounds__(256) quantize_fp8_act_warp_kernel(const uint16_t *__restrict__ x, int is_bf16, int m, int k,
+                                                                  uint8_t *__restrict__ codes,
+                                                                  float *__restrict__ scales) {
+  griddep_wait();
+  const int row = static_cast<int>(blockIdx.x) * 8 + static_cast<int>(threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= m) return;
+  const uint4 *xv = reinterpret_cast<const uint4 *>(x + static_cast<int64_t>(row) * k);
+  uint2 *cv = reinterpret_cast<uint2 *>(codes + static_cast<int64_t>(row) * k);
+  const int nvec = k / 8;
+  uint4 q[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) q[i] = lane + i * 32 < nvec ? xv[lane + i * 32] : make_uint4(0, 0, 0, 0);
+  griddep_launch_dependents();
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const uint32_t w[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (is_bf16) {
+        asm("{\n\t.reg .b32 a;\n\tabs.bf16x2 a, %1;\n\tmax.bf16x2 %0, %0, a;\n\t}" : "+r"(top) : "r"(w[j]));
+      } else {
+        asm("{\n\t.reg .b32 a;\n\tabs.f16x2 a, %1;\n\tmax.f16x2 %0, %0, a;\n\t}" : "+r"(top) : "r"(w[j]));
+      }
+    }
+  }
+  float amax = fmaxf(fmaxf(0.0f, widen(static_cast<uint16_t>(top & 0xffff), is_bf16)), widen(static_cast<uint16_t>(top >> 16), is_bf16));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = __fdiv_rn(amax, 448.0f);
+  const float inv = __frcp_rn(scale > 0.0f ? scale : 1.0f);
+  if (lane == 0) scales[row] = scale;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    if (lane + i * 32 < nvec) cv[lane + i * 32] = e4m3x8_of(q[i], is_bf16, inv);
+  }
+}
+
 // Per-row e4m3 of x (m, k) with the rows' maxima given (taken over a wider row than x: x is one
 // rank's column block of a matrix split by output channel, `amax` the maximum over all ranks'
 // blocks), written into columns [col0, col0 + k) of up to eight (m, ld) matrices of codes: this
@@ -799,6 +842,9 @@ inline int capped_grid(int64_t work_items, int per_block) {
 
 int64_t helper_launch_count() { return g_helper_launches.load(); }
 
+// From how many rows on a warp to a row is enough to fill the GPU.
+constexpr int kWarpRows = 592;
+
 cudaError_t quantize_fp8_act(const void *x, int is_bf16, int m, int k, uint8_t *codes, float *scales,
                              cudaStream_t stream) {
   const bool vec = aligned16(x) && aligned16(codes) && (k % 16 == 0);
@@ -814,7 +860,14 @@ cudaError_t quantize_fp8_act(const void *x, int is_bf16, int m, int k, uint8_t *
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e;
-  if (vec && k <= 2048 * 8) {
+  if (vec && k <= 4096 && m >= kWarpRows) {
+    cfg.gridDim = dim3(static_cast<unsigned>((m + 7) / 8), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    if (k <= 1024) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<4>, xs, is_bf16, m, k, codes, scales);
+    else if (k <= 2048) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<8>, xs, is_bf16, m, k, codes, scales);
+    else if (k <= 3072) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<12>, xs, is_bf16, m, k, codes, scales);
+    else e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<16>, xs, is_bf16, m, k, codes, scales);
+  } else if (vec && k <= 2048 * 8) {
     cfg.blockDim = dim3(256, 1, 1);
     if (k <= 2048 * 2) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_reg_kernel<2>, xs, is_bf16, k, codes, scales);
     else if (k <= 2048 * 4) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_reg_kernel<4>, xs, is_bf16, k, codes, scales);
