@@ -476,11 +476,13 @@ def ref() -> _Ref:
 
 
 def gemm_f32_nt(a: np.ndarray, b: np.ndarray, engine: str = "auto") -> np.ndarray:
-    """C = A Bt in float32. engine: "auto" (reference build if present), "reference", "port"."""
+    """C = A Bt in float32. engine: "auto" (the reference build if present, else 64-bit sums), "reference", "port"."""
     a = np.ascontiguousarray(a, dtype=np.float32)
     b = np.ascontiguousarray(b, dtype=np.float32)
     if engine == "reference" or (engine == "auto" and have_ref()):
         return ref().matmul_nt(a, b)
+    if engine == "auto":
+        return gemm_f64_nt(a, b).astype(np.float32)
     m, k = a.shape
     n = b.shape[0]
     out = np.empty((m, n), dtype=np.float32)
