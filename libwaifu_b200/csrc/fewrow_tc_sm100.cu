@@ -17,9 +17,9 @@
 //              exact), writes them with tcgen05.st into one of three units of 128 columns, and hands
 //              the raw stage back;
 //   warps 9-12 four threads issue the sixteen tcgen05.mma kind::f16 (M = 128 channels, N = 16 rows,
-//              K = 16) of a stage, four each, into an accumulator each. Every tcgen05
-//              issue costs the issuing thread some 60 cycles: with one thread issuing all sixteen
-//              the kernel took 16.9 us, with two 14.0 us, with four 12.7 us;
+//              K = 16) of a stage, four each, into an accumulator each (issued by
+//              lane 0 of one, two or four warps the kernel took 16.9, 14.0 and 12.7 us; by an
+//              elected lane of four 12.1);
 //   warps 0-3  then the epilogue: a lane owns a channel, reads its 4 x 16 partial sums and adds them;
 //              scale, bias, residual, one rounding; for every row the warp stores 32 consecutive
 //              channels.
@@ -187,8 +187,7 @@ fewrow_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   } else if (warp >= kMma && warp < kMma + kMmaWarps) {
     if (elect_one()) {
-      // Every tcgen05 issue costs the issuing thread some 90 cycles, sixteen of them per stage more
-      // than the stage's bytes take to arrive: the blocks of a stage are dealt to four threads.
+      // (the blocks of a stage are dealt to four threads: see the head of this file)
       const int mw = static_cast<int>(warp) - kMma;
       const uint32_t idesc = umma_idesc(kChannels, NTOK, 0u, 0u);
       const uint64_t xdesc0 = umma_desc_sw128(smem_u32(stage_x(0)));

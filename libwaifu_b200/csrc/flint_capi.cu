@@ -1152,7 +1152,11 @@ int32_t fl_fp8_matmul_add(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tens
         ++g_gemm_launches;
         return clear_error();
       }
-      if (!no_skinny && !quick.needs_expand &&
+      // (Twelve to sixteen bfloat16 rows against many channels: mma.sync's time grows with the rows, and
+      // the one-round GEMM's does not: 16 x 12288 x 3072 32.0 us here, 20.0 there, 12 x 16384 x 3072 34.8
+      // and 25.2; at 5120 channels 15.9 and 15.1, and 9 x 8192 x 2048 12.8 and 15.7.)
+      const bool one_round = is_bf16 && m >= 12 && rows >= 12288 && k >= 2048 && gemm_widens_bf16(m, rows, k);
+      if (!no_skinny && !quick.needs_expand && !one_round &&
           skinny_upcast_supported(m, rows, k, raw_ptr(a), raw_ptr(weight), raw_ptr(out), quick.residual != nullptr)) {
         cuda_check(skinny_upcast_matmul(raw_ptr(a), is_bf16, m, rows, k, raw_ptr(weight),
                                         reinterpret_cast<const float *>(raw_ptr(scale)), quick.bias, quick.residual,
@@ -1169,15 +1173,17 @@ int32_t fl_fp8_matmul_add(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tens
     // addend go into the epilogue; no widened copy of the weight exists anywhere. Scratch is only
     // needed for operands whose view starts off a 16-byte boundary and for an addend no epilogue
     // can index.
-    // bfloat16 activations (additive; the reference has none): one UMMA takes both operands in one
-    // 16-bit format, and e4m3 -> bfloat16 has no conversion instruction, so the weight is widened
-    // to bfloat16 by a pass of its own into scratch (rows * k * 2 bytes) and the plain kernel runs.
+    // bfloat16 activations (additive; the reference has none): e4m3 -> bfloat16 takes three
+    // conversions where e4m3 -> half takes one, which the one-round kernel has the time for; ahead
+    // of the persistent one the weight is widened to bfloat16 by a pass of its own into scratch
+    // (rows * k * 2 bytes): 4096 x 12288 x 3072 240 us so, 253 widened in its main loop.
     Scratch scratch;
     size_t a_off = 0, w_off = 0;
     const bool a_misaligned = !aligned16(raw_ptr(a));
     const bool w_misaligned = !aligned16(raw_ptr(weight));
     if (a_misaligned) a_off = scratch.reserve(static_cast<size_t>(m) * k * 2);
-    if (is_bf16) {
+    const bool widen_first = is_bf16 && !gemm_widens_bf16(m, rows, k);
+    if (widen_first) {
       w_off = scratch.reserve(static_cast<size_t>(rows) * k * 2);
     } else if (w_misaligned) {
       w_off = scratch.reserve(static_cast<size_t>(rows) * k);
@@ -1193,7 +1199,7 @@ int32_t fl_fp8_matmul_add(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tens
                  "staging the left operand");
       a_ptr = base + a_off;
     }
-    if (is_bf16) {
+    if (widen_first) {
       cuda_check(widen_e4m3(raw_ptr(weight), static_cast<int64_t>(rows) * k, base + w_off, 1, 0), "widening");
       w_ptr = base + w_off;
     } else if (w_misaligned) {
@@ -1206,7 +1212,7 @@ int32_t fl_fp8_matmul_add(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tens
     ep.col_scale_scalar = 1;
     res.resolve(base, m, rows, &ep);
     run_gemm(is_bf16 ? kGemmBF16 : kGemmF16, m, rows, k, a_ptr, w_ptr, nullptr, nullptr, ep, is_bf16, raw_ptr(out),
-             /*b_is_e4m3=*/!is_bf16);
+             /*b_is_e4m3=*/!widen_first);
     return clear_error();
   });
 }

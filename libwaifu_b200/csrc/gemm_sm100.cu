@@ -51,6 +51,7 @@
 
 #include <mutex>
 
+#include "gemm_split_sm100.cuh"
 #include "ptx_sm100.cuh"
 
 namespace flsm100 {
@@ -1292,6 +1293,8 @@ int sm_count() {
   return cached;
 }
 
+bool gemm_widens_bf16(int m, int n, int k) { return gemm_split_plan(kGemmBF16, 1, m, n, k, sm_count()).split > 0; }
+
 // The schedule (see the head of this file). What the stream-K part can save is the idle share of
 // the last round, (units - remainder) / units of a tile's main loop; what it costs, measured, is
 // about ten microseconds of a launch (two more epilogue-side passes per unit, the second of them
@@ -1401,6 +1404,13 @@ cudaError_t launch_gemm(const GemmArgs &a, const char **why) {
     return cudaErrorInvalidValue;
   }
   kp.status = a.status;
+  // Few tiles: all of them at once, their K divided over clusters. (Forcing single CTAs compares
+  // forms of the kernel below; bfloat16 rows against e4m3 bytes exist only here.)
+  const bool bf16_widening = a.b_is_e4m3 && a.kind == kGemmBF16;
+  if ((!a.force_single_cta || bf16_widening) && gemm_split_supported(a)) {
+    const SplitPlan split = gemm_split_plan(a.kind, a.b_is_e4m3, a.m, a.n, a.k, sm_count());
+    if (split.split > 0) return launch_gemm_split(a, split, why);
+  }
   if (a.b_is_e4m3 && (a.kind != kGemmF16 || kp.num_out > 1)) {
     *why = "an e4m3 right operand widened in the kernel goes with half operands and one destination";
     return cudaErrorInvalidValue;

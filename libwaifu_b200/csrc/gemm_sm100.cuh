@@ -39,7 +39,8 @@ struct GemmArgs {
   int m, n, k;  // k counts elements
   // Operands in device memory, rows 16-byte aligned (pitch = k * element size, a multiple of 16).
   const void *a;  // (m, k)
-  const void *b;  // (n, k); with b_is_e4m3 (kGemmF16 only), e4m3 bytes that the kernel widens to half, exactly
+  const void *b;  // (n, k); with b_is_e4m3, e4m3 bytes that the kernel widens exactly (kGemmF16; kGemmBF16 where
+                  // gemm_widens_bf16() says so)
   int b_is_e4m3;
   // NVFP4 only: the activation's scale factors in the 128-row x 4-factor tile layout the tensor
   // cores read, the weight's in the layout above (nvfp4_prepare() writes both), and how many
@@ -94,6 +95,10 @@ struct GemmArgs {
 // Launches the GEMM. Returns cudaSuccess or the launch/encode error; `why` then points at a
 // static description. Never allocates.
 cudaError_t launch_gemm(const GemmArgs &args, const char **why);
+
+// Whether a product of bfloat16 rows and an e4m3 weight is taken as it is (few tiles), or wants the
+// weight widened to bfloat16 beforehand.
+bool gemm_widens_bf16(int m, int n, int k);
 
 // Number of SMs the persistent grid is sized for on the current device.
 int sm_count();

@@ -1,0 +1,596 @@
+// One-round GEMM: products of so few tiles that the persistent kernel (gemm_sm100.cu) would leave
+// most SMs idle or walk a long K with the few that have a tile.
+//
+// A CTA computes one 128 x block_n tile and leaves, so block_n is whatever multiple of 16 spreads
+// the columns over the SMs, and where even that leaves SMs over, a cluster of 2, 4 or 8 CTAs
+// divides the tile's K stages: each accumulates its share in its own tensor memory, writes the
+// columns it does not own into their owners' shared memory (distributed shared memory), and
+// finishes its own block_n / split columns: sum over the cluster in rank order, scale, bias, GELU,
+// residual, one rounding. Nothing passes through global memory and no CTA waits for one that is
+// not resident.
+//   warps 0-7  an e4m3 weight against 16-bit rows: widen a stage's weight tile to the rows' type
+//              (exact) into a two-slot ring of swizzled tiles; then, all kinds, the epilogue
+//   warp  8    producer: TMA loads of the 128 rows and the weight tile of each K stage into a ring
+//   warp  9    MMA: four tcgen05.mma per stage (128 x block_n, 32 bytes of K per row each)
+// Every operand row of a stage is 128 bytes in the 128-byte swizzle, except the raw e4m3 tile of
+// the widening form (64 bytes of K, as it lies).
+#include "gemm_split_sm100.cuh"
+
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "ptx_sm100.cuh"
+
+namespace flsm100 {
+
+namespace {
+
+constexpr int kTileM = 128;
+constexpr int kStageRowBytes = 128;
+constexpr int kStepsPerStage = 4;  // 32 bytes of K per tcgen05.mma
+constexpr int kWorkWarps = 8;
+constexpr int kLoadWarp = kWorkWarps;
+constexpr int kIssueWarp = kWorkWarps + 1;
+constexpr int kSplitThreads = (kWorkWarps + 2) * 32;
+constexpr int kMaxLoadStages = 8;
+constexpr int kMaxWideSlots = 4;
+constexpr int kATileBytes = kTileM * kStageRowBytes;
+constexpr int kSmemPerCta = 227 * 1024 - 1024;  // (static shared memory beside it)
+
+struct SplitParams {
+  int m, n, num_kb;
+  int tiles_m;
+  int split, block_n, cols;  // cols = block_n / split: what a CTA of the cluster finishes
+  int load_stages, load_bytes, wide_off, wide_slots;
+  const float *row_scale;
+  const float *col_scale;
+  int col_scale_scalar;
+  const void *bias;
+  const void *residual;
+  int residual_rows;
+  long long residual_ld;
+  int act, is_bf16;
+  void *out;
+  int vector_io;  // out and the residual are 16-byte aligned with pitches of whole 16-byte pieces
+  uint32_t tmem_cols;
+  uint32_t *status;
+};
+
+// The exchange buffer holds groups of four columns, a group's 128 rows one after the other (so a
+// warp's 32 rows leave as 512 contiguous bytes: sent row by row, 16 bytes each, 128 x 256 sums took
+// their owners 14 us), groups 16 bytes more than that apart (so that readers of one row in
+// neighbouring groups meet different banks).
+constexpr int kGroupBytes = kTileM * 16 + 16;
+
+__device__ __forceinline__ void store_v4(uint32_t addr, const uint32_t *v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+
+__device__ __forceinline__ void store_cluster_v4(uint32_t cluster_addr, const uint32_t *v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+
+// Eight 16-bit values of one 16-byte piece added to x.
+__device__ __forceinline__ void add8(float (&x)[8], const uint4 q, int is_bf16) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (is_bf16) {
+      x[2 * h] += __uint_as_float(w[h] << 16);
+      x[2 * h + 1] += __uint_as_float(w[h] & 0xffff0000u);
+    } else {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[h]));
+      x[2 * h] += f.x;
+      x[2 * h + 1] += f.y;
+    }
+  }
+}
+
+__device__ __forceinline__ const uint16_t *residual_at(const SplitParams &p, int row, int col) {
+  const int r = p.residual_rows == p.m ? row : row % p.residual_rows;
+  return reinterpret_cast<const uint16_t *>(p.residual) + r * p.residual_ld + col;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *at) { asm volatile("prefetch.global.L2 [%0];" ::"l"(at)); }
+
+// KIND: kKindF8, or kKindF16 / kKindBF16 with WIDEN: the weight is e4m3 and the rows are 16-bit.
+template <int KIND, bool WIDEN>
+__global__ void __launch_bounds__(kSplitThreads, 2)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const SplitParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t full_bar[kMaxLoadStages], empty_bar[kMaxLoadStages];
+  __shared__ __align__(8) uint64_t wide_full_bar[kMaxWideSlots], wide_empty_bar[kMaxWideSlots];
+  __shared__ __align__(8) uint64_t acc_full_bar;
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ volatile uint32_t abort_flag;
+
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  const int rank = p.split > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int tile = blockIdx.x / p.split;
+  const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;  // neighbours share a weight tile
+  const int m0 = tm * kTileM, n0 = tn * p.block_n;
+  const int kb0 = p.num_kb * rank / p.split, kb1 = p.num_kb * (rank + 1) / p.split;
+  const int b_row_bytes = WIDEN ? kStageRowBytes / 2 : kStageRowBytes;
+
+  if (warp == 0) {
+    if (static_cast<int>(lane) < p.load_stages) {
+      mbar_init(&full_bar[lane], 1);
+      mbar_init(&empty_bar[lane], 1);
+    }
+    if (lane < kMaxWideSlots) {
+      mbar_init(&wide_full_bar[lane], WIDEN ? kWorkWarps / p.wide_slots : 1);
+      mbar_init(&wide_empty_bar[lane], 1);
+    }
+    if (lane == 0) {
+      abort_flag = 0;
+      mbar_init(&acc_full_bar, 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == kLoadWarp && lane == 0) {
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+    // The first stages of the weight into L2 while the kernel ahead in the stream may still run: a
+    // prefetch writes nothing and the loads below read what they would have read anyway.
+    for (int kb = kb0; kb < kb1 && kb < kb0 + p.load_stages; ++kb) tma_prefetch_l2_2d(&tmap_b, kb * b_row_bytes, n0);
+  }
+  if (warp == kIssueWarp) {
+    tmem_alloc<1>(&tmem_base_slot, p.tmem_cols);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+  griddep_wait();
+  griddep_launch_dependents();
+
+  // The residual of the rows this CTA will finish, into L2 under the main loop.
+  if (p.residual && warp < kWorkWarps) {
+    const int lines = (p.cols * 2 + 127) / 128, first_col = n0 + rank * p.cols;
+    for (int i = static_cast<int>(threadIdx.x); i < kTileM * lines; i += kWorkWarps * 32) {
+      const int row = m0 + i / lines, col = first_col + i % lines * 64;
+      if (row < p.m && col < p.n) prefetch_l2(residual_at(p, row, col));
+    }
+  }
+
+  if (warp == kLoadWarp) {
+    if (elect_one()) {
+      bool ok = true;
+      int s = 0;
+      uint32_t phase = 0;
+      const uint32_t bytes = static_cast<uint32_t>(kATileBytes + p.block_n * b_row_bytes);  // (rows outside arrive as zeros)
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty_bar[s], phase ^ 1, &abort_flag)) {
+          ok = false;
+          break;
+        }
+        uint8_t *base = smem + s * p.load_bytes;
+        mbar_arrive_expect_tx(&full_bar[s], bytes);
+        tma_load_2d(base + kATileBytes, &tmap_b, &full_bar[s], kb * b_row_bytes, n0);
+        tma_load_2d(base, &tmap_a, &full_bar[s], kb * kStageRowBytes, m0);
+        if (++s == p.load_stages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      if (!ok) {
+        abort_flag = 1;
+        atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusProducerTimeout));
+      }
+    }
+  } else if (warp == kIssueWarp) {
+    // (the whole warp walks the loop and one lane issues, as in the persistent kernel)
+    const bool issuer = elect_one();
+    constexpr uint32_t kFmt = KIND == kKindBF16 ? 1u : 0u;
+    const uint32_t idesc = umma_idesc(kTileM, static_cast<uint32_t>(p.block_n), kFmt, kFmt);
+    const uint32_t smem0 = smem_u32(smem);
+    bool ok = true;
+    int s = 0, w = 0;
+    uint32_t phase = 0, wide_phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!mbar_wait(&full_bar[s], phase, &abort_flag) || (WIDEN && !mbar_wait(&wide_full_bar[w], wide_phase, &abort_flag))) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint64_t ad = umma_desc_sw128(smem0 + s * p.load_bytes);
+      const uint64_t bd = umma_desc_sw128(WIDEN ? smem0 + p.wide_off + w * p.block_n * kStageRowBytes
+                                                : smem0 + s * p.load_bytes + kATileBytes);
+#pragma unroll
+      for (int i = 0; i < kStepsPerStage; ++i) {
+        if (issuer) umma_ss<KIND>(tmem_base, ad + i * 2, bd + i * 2, idesc, (kb > kb0 || i > 0) ? 1u : 0u);
+      }
+      if (issuer) {
+        umma_commit(&empty_bar[s]);
+        if (WIDEN) umma_commit(&wide_empty_bar[w]);
+      }
+      if (WIDEN && ++w == p.wide_slots) {
+        w = 0;
+        wide_phase ^= 1;
+      }
+      if (++s == p.load_stages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+    if (ok && issuer) umma_commit(&acc_full_bar);
+    if (!ok && issuer) {
+      abort_flag = 1;
+      atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusMmaTimeout));
+    }
+  } else if constexpr (WIDEN) {
+    // Sixteen e4m3 bytes of a row -> two 16-byte pieces of its 128 bytes, in the 128-byte swizzle.
+    // The warps share out the wide slots (several stages are widened at once), and the load stages are
+    // a multiple of those, so that a warp sees every phase of the barriers it waits on.
+    const int group_warps = kWorkWarps / p.wide_slots;
+    const int w = static_cast<int>(warp) / group_warps;
+    const int first = static_cast<int>(threadIdx.x) % (group_warps * 32);
+    bool ok = true;
+    for (int it = w; it < kb1 - kb0; it += p.wide_slots) {
+      const int s = it % p.load_stages;
+      if (!mbar_wait(&full_bar[s], (it / p.load_stages) & 1, &abort_flag) ||
+          !mbar_wait(&wide_empty_bar[w], ((it / p.wide_slots) & 1) ^ 1, &abort_flag)) {
+        ok = false;
+        break;
+      }
+      const uint8_t *raw = smem + s * p.load_bytes + kATileBytes;
+      uint8_t *wide = smem + p.wide_off + w * p.block_n * kStageRowBytes;
+#pragma unroll 4
+      for (int piece = first; piece < p.block_n * 4; piece += group_warps * 32) {
+        const uint32_t r = static_cast<uint32_t>(piece) >> 2, q = static_cast<uint32_t>(piece) & 3;
+        const uint4 v = *reinterpret_cast<const uint4 *>(raw + piece * 16);
+        uint4 lo, hi;
+        if constexpr (KIND == kKindBF16) {
+          e4m3x16_to_bf16(v, &lo, &hi);
+        } else {
+          e4m3x16_to_f16(v, &lo, &hi);
+        }
+        uint8_t *row_base = wide + r * kStageRowBytes;
+        *reinterpret_cast<uint4 *>(row_base + (((2 * q) ^ (r & 7)) << 4)) = lo;
+        *reinterpret_cast<uint4 *>(row_base + (((2 * q + 1) ^ (r & 7)) << 4)) = hi;
+      }
+      fence_proxy_async_smem();  // the UMMA reads these bytes through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&wide_full_bar[w]);
+    }
+    if (!ok && lane == 0) {
+      abort_flag = 1;
+      atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusProducerTimeout));
+    }
+  }
+
+  // ------------------------------------------------------------------ epilogue
+  // The accumulator is complete: so are all loads and all reads of the ring, which becomes the
+  // exchange buffer: split x 128 rows of `cols` floats, the part of every CTA of the cluster.
+  bool have = false;
+  if (warp < kWorkWarps) {
+    have = __all_sync(0xffffffffu, mbar_wait(&acc_full_bar, 0, &abort_flag));
+    if (!have && lane == 0) {
+      abort_flag = 1;
+      atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusEpilogueTimeout));
+    }
+  }
+  // (The cluster barriers are reached on every path: all waits above are bounded.)
+  if (p.split > 1) {
+    __syncwarp();
+    cluster_sync_all();
+  }
+  if (have) {
+    tc_fence_after_sync();
+    const uint32_t quarter = warp & 3;
+    const int row = static_cast<int>(quarter) * 32 + static_cast<int>(lane);
+    const uint32_t t_row = tmem_base + ((quarter * 32u) << 16);
+    const uint32_t mine = smem_u32(smem) + static_cast<uint32_t>(rank * (p.cols / 4) * kGroupBytes + row * 16);
+    for (int c = static_cast<int>(warp >> 2); c < p.block_n / 16; c += 2) {
+      uint32_t v[16];
+      tmem_ld_32x16(t_row + c * 16, v);
+      tmem_ld_wait(v);
+      const int owner = c * 16 / p.cols;
+      const uint32_t local = mine + static_cast<uint32_t>((c * 16 - owner * p.cols) / 4) * kGroupBytes;
+      if (owner == rank) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_v4(local + j * kGroupBytes, v + 4 * j);
+      } else {
+        const uint32_t dst = map_to_cta(local, static_cast<uint32_t>(owner));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_cluster_v4(dst + j * kGroupBytes, v + 4 * j);
+      }
+    }
+  }
+  __syncwarp();
+  if (p.split > 1) {
+    cluster_sync_all();
+  } else {
+    __syncthreads();
+  }
+  if (have) {
+    // A thread keeps its eight columns and walks the rows, so scales and bias are fetched once, and
+    // the residual of four rows is on its way before the first is needed.
+    const int groups = p.cols / 8, rows_at_once = kWorkWarps * 32 / groups;
+    const int g = static_cast<int>(threadIdx.x) % groups, r0 = static_cast<int>(threadIdx.x) / groups;
+    const int col = n0 + rank * p.cols + g * 8;
+    const int live_rows = (r0 < rows_at_once && col < p.n) ? min(kTileM, p.m - m0) : 0;  // (n is a multiple of 8)
+    float cs[8], bias[8];
+    if (live_rows > 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        cs[i] = p.col_scale ? __ldg(p.col_scale + (p.col_scale_scalar ? 0 : col + i)) : 1.0f;
+        bias[i] = 0.0f;
+      }
+      if (p.bias) {
+        uint4 q;
+        uint16_t *e = reinterpret_cast<uint16_t *>(&q);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = __ldg(reinterpret_cast<const uint16_t *>(p.bias) + col + i);
+        add8(bias, q, p.is_bf16);
+      }
+    }
+    constexpr int kAhead = 4;
+    for (int r = r0; r < live_rows; r += kAhead * rows_at_once) {
+      uint4 res[kAhead];
+      float rs[kAhead];
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        const int row = m0 + r + a * rows_at_once;
+        res[a] = make_uint4(0, 0, 0, 0);
+        rs[a] = 1.0f;
+        if (r + a * rows_at_once >= live_rows) continue;
+        if (p.row_scale) rs[a] = __ldg(p.row_scale + row);
+        if (p.residual) {
+          const uint16_t *at = residual_at(p, row, col);
+          if (p.vector_io) {
+            res[a] = *reinterpret_cast<const uint4 *>(at);
+          } else {
+            uint16_t *e = reinterpret_cast<uint16_t *>(&res[a]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) e[i] = at[i];
+          }
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        const int in_tile = r + a * rows_at_once;
+        if (in_tile >= live_rows) break;
+        const uint8_t *part = smem + g * 2 * kGroupBytes + in_tile * 16;
+        float x[8] = {};
+        for (int s = 0; s < p.split; ++s, part += p.cols / 4 * kGroupBytes) {
+          const float4 lo = *reinterpret_cast<const float4 *>(part), hi = *reinterpret_cast<const float4 *>(part + kGroupBytes);
+          x[0] += lo.x, x[1] += lo.y, x[2] += lo.z, x[3] += lo.w, x[4] += hi.x, x[5] += hi.y, x[6] += hi.z, x[7] += hi.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= rs[a] * cs[i];
+        if (p.bias) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] += bias[i];
+        }
+        if (p.act == kActGeluTanh) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = gelu_tanh(x[i]);
+        }
+        if (p.residual) add8(x, res[a], p.is_bf16);
+        uint32_t w[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (p.is_bf16) {
+            const __nv_bfloat162 q = __floats2bfloat162_rn(x[2 * h], x[2 * h + 1]);
+            w[h] = *reinterpret_cast<const uint32_t *>(&q);
+          } else {
+            const __half2 q = __floats2half2_rn(x[2 * h], x[2 * h + 1]);
+            w[h] = *reinterpret_cast<const uint32_t *>(&q);
+          }
+        }
+        uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + static_cast<long long>(m0 + in_tile) * p.n + col;
+        if (p.vector_io) {
+          *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) dst[i] = static_cast<uint16_t>(i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu);
+        }
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (abort_flag != 0) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies that may still be in flight
+    __syncthreads();
+  }
+  if (warp == kIssueWarp) {
+    tc_fence_after_sync();
+    tmem_dealloc<1>(tmem_base, p.tmem_cols);
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = [] {
+    void *ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess) {
+      return reinterpret_cast<EncodeTiledFn>(ptr);
+    }
+    return static_cast<EncodeTiledFn>(nullptr);
+  }();
+  return fn;
+}
+
+// A (rows, row_bytes) byte matrix read in boxes of box_bytes x box_rows, zeros outside.
+bool make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t row_bytes, uint32_t box_bytes, uint32_t box_rows,
+              CUtensorMapSwizzle swizzle) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {row_bytes, rows};
+  cuuint64_t strides[1] = {row_bytes};
+  cuuint32_t box[2] = {box_bytes, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int KIND, bool WIDEN>
+cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {
+  const uint64_t row_bytes = static_cast<uint64_t>(a.k) * (KIND == kKindF8 ? 1 : 2);
+  CUtensorMap ta, tb;
+  const uint32_t bn = static_cast<uint32_t>(plan.block_n);
+  if (!make_map(&ta, a.a, a.m, row_bytes, kStageRowBytes, kTileM, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !(WIDEN ? make_map(&tb, a.b, a.n, row_bytes / 2, kStageRowBytes / 2, bn, CU_TENSOR_MAP_SWIZZLE_NONE)
+              : make_map(&tb, a.b, a.n, row_bytes, kStageRowBytes, bn, CU_TENSOR_MAP_SWIZZLE_128B))) {
+    *why = "cuTensorMapEncodeTiled refused an operand";
+    return cudaErrorInvalidValue;
+  }
+  auto kernel = gemm_split_kernel<KIND, WIDEN>;
+  static bool attr_set = false;  // per instantiation
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+    if (e != cudaSuccess) {
+      *why = "cudaFuncSetAttribute(max dynamic shared memory) failed";
+      return e;
+    }
+    attr_set = true;
+  }
+  SplitParams p = {};
+  p.m = a.m;
+  p.n = a.n;
+  p.num_kb = static_cast<int>((row_bytes + kStageRowBytes - 1) / kStageRowBytes);
+  p.tiles_m = (a.m + kTileM - 1) / kTileM;
+  const int tiles_n = (a.n + plan.block_n - 1) / plan.block_n;
+  p.split = plan.split;
+  p.block_n = plan.block_n;
+  p.cols = plan.block_n / plan.split;
+  p.load_bytes = kATileBytes + plan.block_n * (WIDEN ? kStageRowBytes / 2 : kStageRowBytes);
+  p.wide_slots = plan.block_n <= 128 ? kMaxWideSlots : 2;
+  const int wide_bytes = WIDEN ? p.wide_slots * plan.block_n * kStageRowBytes : 0;
+  const int most = (kSmemPerCta - 1024 - wide_bytes) / p.load_bytes;
+  const int longest = (p.num_kb + plan.split - 1) / plan.split;
+  p.load_stages = most < kMaxLoadStages ? most : kMaxLoadStages;
+  if (WIDEN) {
+    p.load_stages -= p.load_stages % p.wide_slots;
+  } else if (p.load_stages > longest) {
+    p.load_stages = longest;
+  }
+  p.wide_off = p.load_stages * p.load_bytes;
+  const int ring = p.wide_off + wide_bytes;
+  const int exchange = plan.block_n / 4 * kGroupBytes;
+  p.row_scale = a.row_scale;
+  p.col_scale = a.col_scale;
+  p.col_scale_scalar = a.col_scale_scalar;
+  p.bias = a.bias;
+  p.residual = a.residual;
+  p.residual_rows = a.residual_rows > 0 ? a.residual_rows : a.m;
+  p.residual_ld = a.residual_ld;
+  p.act = a.act;
+  p.is_bf16 = a.out_bf16;
+  p.out = a.out;
+  p.vector_io = (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
+                (!a.residual || ((reinterpret_cast<uintptr_t>(a.residual) & 15) == 0 && a.residual_ld % 8 == 0));
+  p.tmem_cols = 32;
+  while (p.tmem_cols < bn) p.tmem_cols *= 2;
+  p.status = a.status;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.tiles_m * tiles_n * plan.split), 1, 1);
+  cfg.blockDim = dim3(kSplitThreads, 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>((ring > exchange ? ring : exchange) + 1024);
+  cfg.stream = a.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(plan.split);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = plan.split > 1 ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
+  if (e != cudaSuccess) *why = "kernel launch failed";
+  return e;
+}
+
+}  // namespace
+
+bool gemm_split_supported(const GemmArgs &a) {
+  if (a.num_extra_out > 0 || a.row_amax || a.rows_per_group || a.global_scale) return false;
+  if (a.out_ld > 0 && (a.out_ld != a.n || a.out_col0 != 0)) return false;
+  return encode_fn() != nullptr;
+}
+
+// Estimated times in microseconds, fitted to a sweep of every block_n and split over 1280 to 16384
+// channels, k = 640 to 12288 and 16 to 2048 rows (the choice they make is within 1.5 % of the best
+// measured one on average, 13 % at worst). A stage takes its latency, or its bytes through L2 with
+// every CTA pulling at once, or (widening) what the converters need for block_n rows; then come the
+// exchange and the epilogue, which grow with block_n, and the launch.
+//   77 x 2560 x 2048, half: 17.7 us on the persistent kernel, 11.2 here; 300 x 1280 x 640 15.4 and
+//   7.8; 512 x 5120 x 3072 in bfloat16 39 (with a widening pass) and 30.7; e4m3 rows with
+//   the quantiser, 300 x 1280 x 1280 15.3 and 10.0, 1024 x 3072 x 3072 21.8 and 20.1.
+SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms) {
+  SplitPlan best = {0, 0};
+  if (kind != kGemmE4M3 && !b_is_e4m3) return best;
+  const bool widen = kind != kGemmE4M3;
+  const int num_kb = (k * (widen ? 2 : 1) + kStageRowBytes - 1) / kStageRowBytes;
+  const int tiles_m = (m + kTileM - 1) / kTileM;
+  // The persistent kernel: rounds of whole tiles (pairs of CTAs above one row block), a long K cut in
+  // halves where that leaves no unit without one (gemm_schedule), and for bfloat16 rows the pass
+  // that widens the weight ahead of it. 16-bit rows are taken over up to a tenth above that estimate,
+  // where the measured times cross (200 x 12288 x 3072 in half 32.2 and 30.9 us). e4m3 rows, whose K
+  // is never divided here, leave a K that the other kernel halves to it (512 x 3072 x 12288: 36.6 us
+  // there, 39.8 here).
+  const int units = tiles_m == 1 ? sms : sms / 2;
+  const long long tiles = tiles_m == 1 ? (n + 127) / 128 : static_cast<long long>((m + 255) / 256) * ((n + 255) / 256);
+  float persistent = static_cast<float>((tiles + units - 1) / units * num_kb) *
+                     (tiles_m == 1 ? (widen ? 0.23f : 0.19f) : (widen ? 0.31f : 0.35f));
+  if (2 * tiles <= units && num_kb >= 80) {
+    if (!widen) return best;
+    persistent *= 0.75f;
+  }
+  persistent += tiles_m == 1 ? 10.0f : 12.8f;
+  if (kind == kGemmBF16) persistent += static_cast<float>(n) * k * 0.65e-6f;
+  float best_time = persistent * (widen ? 1.1f : 1.0f);
+  // The linears on quantised rows promise that one product of all row groups and a product per group,
+  // and the fused and the separate quantiser, agree to the last bit: their K stays in one piece,
+  // where every sum is the persistent kernel's (10.9 -> 12.4 us at 128 x 3072 x 3072, still below 13.8).
+  const int max_split = widen ? 8 : 1;
+  for (int split = 1; split <= max_split; split *= 2) {
+    // clusters of four and eight do not fill every SM of a GPC
+    const int room = split <= 2 ? sms : split == 4 ? sms * 9 / 10 : sms * 3 / 4;
+    if (num_kb < 2 * split) break;
+    const int step = 16 * split;
+    for (int bn = std::max(32, step); bn <= 256; bn += step) {
+      const long long ctas = static_cast<long long>(tiles_m) * ((n + bn - 1) / bn) * split;
+      if (ctas > room) continue;
+      const float bytes = kATileBytes + bn * (widen ? kStageRowBytes / 2 : kStageRowBytes);
+      const float through_l2 = ctas * bytes / (widen ? 8.0e6f : 12.5e6f);
+      const float stage = std::max(std::max(widen ? 0.39f : 0.215f, through_l2), bn * (widen ? 0.0023f : 0.0016f));
+      const float exchange = split == 1 ? 0.0f : split == 2 ? 1.1f : split == 4 ? 2.3f : 4.7f;
+      const float scale = split == 1 ? 1.0f : split == 2 ? 0.707f : split == 4 ? 0.5f : 0.354f;
+      const float time = (num_kb + split - 1) / split * stage + bn * scale * (widen ? 0.044f : 0.03f) + exchange + (widen ? 2.6f : 6.3f);
+      if (time < best_time) {
+        best_time = time;
+        best = {bn, split};
+      }
+    }
+  }
+  return best;
+}
+
+cudaError_t launch_gemm_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {
+  *why = "";
+  switch (a.kind) {
+    case kGemmE4M3: return launch_split<kKindF8, false>(a, plan, why);
+    case kGemmBF16: return launch_split<kKindBF16, true>(a, plan, why);
+    default: return launch_split<kKindF16, true>(a, plan, why);
+  }
+}
+
+}  // namespace flsm100

@@ -1,0 +1,28 @@
+// Host-side interface of the one-round GEMM (gemm_split_sm100.cu): the products whose tiles all fit
+// the GPU at once, of launch_gemm's operands and epilogue.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "gemm_sm100.cuh"
+
+namespace flsm100 {
+
+// How a product is cut: tiles of 128 rows x `block_n` columns, each computed by a cluster of
+// `split` CTAs that divide its K stages. split == 0: the product stays with the persistent kernel.
+struct SplitPlan {
+  int block_n;
+  int split;
+};
+
+// Host arithmetic only; for e4m3 against e4m3, and (`b_is_e4m3`) 16-bit rows against an e4m3 weight
+// that is widened in the kernel.
+SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms);
+
+// Whether the kernel has all that `args` asks for (one destination of pitch n, no row groups, no
+// row maxima).
+bool gemm_split_supported(const GemmArgs &args);
+
+cudaError_t launch_gemm_split(const GemmArgs &args, const SplitPlan &plan, const char **why);
+
+}  // namespace flsm100

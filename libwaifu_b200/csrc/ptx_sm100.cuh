@@ -7,6 +7,8 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 namespace flsm100 {
@@ -176,6 +178,26 @@ __device__ __forceinline__ void e4m3x16_to_f16(const uint4 codes, uint4 *lo, uin
   e4m3x4_to_f16x4(codes.y, &lo->z, &lo->w);
   e4m3x4_to_f16x4(codes.z, &hi->x, &hi->y);
   e4m3x4_to_f16x4(codes.w, &hi->z, &hi->w);
+}
+
+// The same as bfloat16 values, exact: no conversion instruction goes there in one step, so code ->
+// half -> float -> bfloat16, each step exact (a NaN stays one).
+__device__ __forceinline__ void e4m3x16_to_bf16(const uint4 codes, uint4 *lo, uint4 *hi) {
+  const uint32_t in[4] = {codes.x, codes.y, codes.z, codes.w};
+  uint32_t out[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t h[2];
+    e4m3x4_to_f16x4(in[i], &h[0], &h[1]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&h[j]));
+      const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+      out[2 * i + j] = *reinterpret_cast<const uint32_t *>(&b);
+    }
+  }
+  *lo = make_uint4(out[0], out[1], out[2], out[3]);
+  *hi = make_uint4(out[4], out[5], out[6], out[7]);
 }
 
 // 0.5 x (1 + tanh(u)) == x * sigmoid(2u) == x / (1 + 2^z), u = sqrt(2/pi) (x + 0.044715 x^3),
