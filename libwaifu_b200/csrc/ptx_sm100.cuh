@@ -27,7 +27,8 @@ __device__ __forceinline__ uint32_t lane_id() {
 // what a tcgen05 instruction takes (descriptors, addresses) lives in uniform registers; under
 // `lane == 0` every instruction is issued some 60 to 130 cycles after the one before it, which is
 // what paced the kernels whose instructions are shorter than that (2 x 24 x 4352 x 128 attention
-// 454 -> 389 us; C3's four-bit GEMM, whose scale-factor copies are issued one by one, 103 -> 73).
+// 454 -> 389 us; the four-bit GEMM of 4352 x 9216 x 3072, whose scale-factor copies are issued one by
+// one, 103 -> 73).
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
