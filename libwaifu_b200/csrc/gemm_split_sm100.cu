@@ -534,12 +534,21 @@ bool gemm_split_supported(const GemmArgs &a) {
 //   77 x 2560 x 2048, half: 17.7 us on the persistent kernel, 11.2 here; 300 x 1280 x 640 15.4 and
 //   7.8; 512 x 5120 x 3072 in bfloat16 39 (with a widening pass) and 30.7; e4m3 rows with
 //   the quantiser, 300 x 1280 x 1280 15.3 and 10.0, 1024 x 3072 x 3072 21.8 and 20.1.
-SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms) {
+SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k) {
   SplitPlan best = {0, 0};
   if (kind != kGemmE4M3 && !b_is_e4m3) return best;
   const bool widen = kind != kGemmE4M3;
   const int num_kb = (k * (widen ? 2 : 1) + kStageRowBytes - 1) / kStageRowBytes;
   const int tiles_m = (m + kTileM - 1) / kTileM;
+  // The linears on quantised rows give the same bits with and without the rows' maxima, to one destination
+  // and to several, in row groups and without; some of those forms run on the persistent kernel alone.
+  // So e4m3 rows stay there wherever that kernel cuts a tile's K in two (260 x 9488 x 5376), and keep K in
+  // one piece here (10.9 -> 12.4 us at 128 x 3072 x 3072, still below 13.8).
+  if (!widen && stream_k) {
+    int tile_plan[8];
+    gemm_plan(kind, m, n, k, sms, 1, tile_plan);
+    if (tile_plan[6] > 0) return best;
+  }
   // The persistent kernel: rounds of whole tiles (pairs of CTAs above one row block), a long K cut in
   // halves where that leaves no unit without one (gemm_schedule), and for bfloat16 rows the pass
   // that widens the weight ahead of it. 16-bit rows are taken over up to a tenth above that estimate,
@@ -557,9 +566,6 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
   persistent += tiles_m == 1 ? 10.0f : 12.8f;
   if (kind == kGemmBF16) persistent += static_cast<float>(n) * k * 0.65e-6f;
   float best_time = persistent * (widen ? 1.1f : 1.0f);
-  // The linears on quantised rows promise that one product of all row groups and a product per group,
-  // and the fused and the separate quantiser, agree to the last bit: their K stays in one piece,
-  // where every sum is the persistent kernel's (10.9 -> 12.4 us at 128 x 3072 x 3072, still below 13.8).
   const int max_split = widen ? 8 : 1;
   for (int split = 1; split <= max_split; split *= 2) {
     // clusters of four and eight do not fill every SM of a GPC

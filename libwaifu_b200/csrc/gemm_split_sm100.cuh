@@ -16,8 +16,9 @@ struct SplitPlan {
 };
 
 // Host arithmetic only; for e4m3 against e4m3, and (`b_is_e4m3`) 16-bit rows against an e4m3 weight
-// that is widened in the kernel.
-SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms);
+// that is widened in the kernel. `stream_k`: whether the persistent kernel may cut tiles in two (it has
+// the workspace for it).
+SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k);
 
 // Whether the kernel has all that `args` asks for (one destination of pitch n, no row groups, no
 // row maxima).

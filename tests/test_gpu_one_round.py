@@ -116,3 +116,35 @@ def test_causal_units_of_several_heads(flint, oracle, n, h, hk, L, S, d):
     want = oracle.attention(q, k, v, True, True)
     assert oracle.rel_l2(got, want) <= 5e-3
     assert np.abs(got - want).max() <= 2 * oracle.ulp16_at(float(np.abs(want).max()), True)
+
+
+@pytest.mark.parametrize("m,n,k", [(260, 9488, 5376), (814, 4816, 11120), (1024, 384, 12288), (300, 1280, 1280), (200, 2584, 880),
+                                   (128, 3072, 3072)])
+def test_linears_on_quantised_rows_give_the_same_bits(flint, m, n, k):
+    """fl_fp8_linear, which takes the one-round kernel where that is faster, against the forms that run on
+    the persistent kernel alone (row maxima, several destinations): where that kernel cuts a tile's
+    K in two, as in the first three shapes, and where it does not, the sums are the same."""
+    import torch
+    F = flint
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    bf = F.DType.BFLOAT16
+
+    def new(shape, std, kind=torch.bfloat16, dtype=bf):
+        t = (torch.randn(shape, device="cuda", generator=gen) * std).to(kind)
+        return F.Tensor.from_device_ptr(t.data_ptr(), shape, dtype, keepalive=t)
+
+    x, bias, res = new((m, k), 1.0), new((n,), 0.1), new((m, n), 1.0)
+    codes, scales = F.quantize_fp8_rows(new((n, k), 0.02, torch.float32, F.DType.FLOAT))
+    want = F.fp8_linear(x, codes, scales, bias, res, F.ACT_GELU_TANH).numpy()
+    row_amax = F.Tensor.empty((m,), F.DType.FLOAT)
+    got = F.fp8_linear_amax(x, codes, scales, row_amax, bias, res, F.ACT_GELU_TANH).numpy()
+    assert np.array_equal(got, want), "with the rows' maxima"
+    wide = F.Tensor.empty((m, n + 8), bf)
+    F.fp8_linear_scatter(x, codes, scales, [wide], 8, bias, res, F.ACT_GELU_TANH)
+    assert np.array_equal(wide.numpy()[:, 8:], want), "into a column block"
+    xc, xs = F.Tensor.empty((m, k), F.DType.FP8E4M3), F.Tensor.empty((m,), F.DType.FLOAT)
+    F.check(F.lib().fl_quantize_fp8_activation(x.raw(), xc.raw(), xs.raw()))
+    out = F.Tensor.empty((m, n), bf)
+    F.fp8_linear_quantized(xc, xs, codes, scales, bias, res, F.ACT_GELU_TANH, out)
+    assert np.array_equal(out.numpy(), want), "on rows quantised beforehand"
+    F.synchronize()
