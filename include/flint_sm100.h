@@ -404,13 +404,17 @@ FLAPI int32_t fl_sm100_few_rows_plan(int32_t m, int32_t n, int32_t k, int32_t we
 
 /* Which kernel a product of few rows takes by its shape alone (operands aligned, the environment's
  * switches unset); host arithmetic only, no GPU needed. entry 0: fl_fp8_matmul[_add] with half
- * rows, 1: fl_fp8_linear (and _static, _quantized), 2: fl_matmul[_add] on 16-bit operands; n the
- * weight's rows (output channels). Returns 2: a tensor-core few-row kernel (the weight on the M side
- * of the instruction), 1: the mma.sync few-row kernel, 0: the tile kernel; -1 for a bad argument. */
+ * rows, 1: fl_fp8_linear (and _static, _quantized), 2: fl_matmul[_add] on 16-bit operands,
+ * 4: fl_fp8_matmul[_add] with bfloat16 rows; n the weight's rows (output channels). Returns 2: a
+ * tensor-core few-row kernel (the weight on the M side of the instruction), 1: the mma.sync few-row
+ * kernel, 0: none of them, but the one-round kernel (fl_sm100_one_round_plan) or the tile kernel; -1
+ * for a bad argument. */
 FLAPI int32_t fl_sm100_few_rows_route(int32_t entry, int32_t m, int32_t n, int32_t k);
 
-/* Which tile kernel a product of `kind` (0 half, 1 bfloat16, 2 e4m3, 3 nvfp4) and shape would run on
- * and how its tiles are dealt out over a device of `sms` SMs; host arithmetic only, no GPU needed, so
+/* Which form of the persistent tile kernel a product of `kind` (0 half, 1 bfloat16, 2 e4m3, 3 nvfp4)
+ * and shape runs on and how its tiles are dealt out over a device of `sms` SMs, where it runs there: a
+ * product of few rows (fl_sm100_few_rows_route) or few tiles (fl_sm100_one_round_plan) may not.
+ * Host arithmetic only, no GPU needed, so
  * that the schedule can be checked anywhere. plan[8]: [0] CTAs per unit (2: a cluster pair sharing a
  * 256-row tile), [1] tile width, [2] tiles, [3] K stages (128 bytes of K each) per tile, [4] units,
  * [5] rounds of whole tiles (tile = round * units + unit), [6] tiles of the stream-K part that
@@ -419,6 +423,18 @@ FLAPI int32_t fl_sm100_few_rows_route(int32_t entry, int32_t m, int32_t n, int32
  * round is simply partly filled) or at least [4]. */
 FLAPI int32_t fl_sm100_gemm_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t allow_stream_k,
                                  int32_t *plan);
+
+/* How the one-round kernel cuts a product against an e4m3 weight, of half (kind 0), bfloat16 (1) or
+ * quantised rows (2), that no few-row kernel takes and that has one destination, no row groups and
+ * no row maxima; host arithmetic only, no GPU needed. `allow_stream_k`: whether the persistent kernel
+ * has its workspace (0: fl_fp8_linear_static, or FLINT_SM100_NO_STREAM_K=1). plan[8]: [0] tile width
+ * (tiles have 128 rows; 0: the product stays with the persistent kernel and the rest is 0), [1] CTAs
+ * of a cluster, which divide a tile's K stages (rank r has [3] * r / [1] up to [3] * (r + 1) / [1]) and
+ * finish [0] / [1] columns each, [2] CTAs, [3] K stages of a tile, [4] slots of the load ring,
+ * [5] of the ring of widened weight tiles (0 for quantised rows), [6] bytes of a load slot,
+ * [7] dynamic shared memory of a CTA. */
+FLAPI int32_t fl_sm100_one_round_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t allow_stream_k,
+                                      int32_t *plan);
 
 /* Storage over device memory the caller already owns (for instance a torch tensor's): nothing
  * is copied and nothing is freed on destroy. The device counterpart of fl_tensor_data_borrow(). */

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "gemm_sm100.cuh"
+#include "gemm_split_sm100.cuh"
 #include "quant_sm100.cuh"
 #include "block_sm100.cuh"
 #include "skinny_sm100.cuh"
@@ -579,6 +580,18 @@ bool fewrow_tc_route(int m, int rows, int k) {
   return k >= 2048 ? rows >= 8192 || (rows >= 6144 && m >= 2) || (rows >= 3072 && m >= 8)
                    : rows >= 16384 || (rows >= 12288 && m >= 4) || (rows >= 8192 && m >= 8);
 }
+// fl_fp8_matmul[_add], twelve to sixteen bfloat16 rows against many channels (gemm_split_kernel):
+// mma.sync's time grows with the rows and the channels, the one-round GEMM's with neither until its
+// tiles widen. Microseconds at twelve and sixteen rows, mma.sync / one-round:
+//   k       8192 channels         10240                 12288                 16384
+//   1024    7.7 8.2 / 10.8 10.6   9.5 9.9 / 10.8 10.7   9.8 10.3 / 12.6 12.4  12.0 12.4 / 14.9 14.6
+//   2048    13.6 14.6 / 16.2 15.9 15.6 16.6 / 14.0 14.7 17.7 18.9 / 16.1 16.0 22.7 24.3 / 18.5 18.7
+//   3072    19.2 20.5 / 19.1 19.6 24.5 26.9 / 19.6 18.2 27.9 31.3 / 19.9 20.8 34.6 37.1 / 27.7 24.7
+// From 12288 channels and 2048-deep rows on it is ahead at every shape measured; at 10240 too, by less at
+// 2048, and those have stayed with mma.sync.
+bool bf16_one_round_route(int m, int rows, int k) {
+  return m >= 12 && rows >= 12288 && k >= 2048 && gemm_widens_bf16(m, rows, k);
+}
 // fl_matmul[_add], 16-bit rows against a 16-bit weight (fewrow_q8_kernel, kind::f16):
 bool fewrow_w16_route(int m, int n, int k) {
   if (m > 64 || k < 2048) return false;
@@ -647,7 +660,9 @@ void run_gemm(GemmKind kind, int m, int n, int k, const void *a, const void *b, 
   g.out_col0 = ep.out_col0;
   g.status = status_word();
   g.stream = 0;
-  // FLINT_SM100_SINGLE_CTA=1 keeps every GEMM on the single-CTA kernel (for A/B measurements).
+  // FLINT_SM100_SINGLE_CTA=1 keeps every GEMM on the persistent kernel, without CTA pairs (for A/B
+  // measurements); bfloat16 rows against an e4m3 weight, where few tiles go to the one-round kernel
+  // without a widened copy of the weight, still go there.
   static const bool single_cta = []() {
     const char *v = std::getenv("FLINT_SM100_SINGLE_CTA");
     return v && v[0] == '1';
@@ -1152,10 +1167,7 @@ int32_t fl_fp8_matmul_add(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tens
         ++g_gemm_launches;
         return clear_error();
       }
-      // (Twelve to sixteen bfloat16 rows against many channels: mma.sync's time grows with the rows, and
-      // the one-round GEMM's does not: 16 x 12288 x 3072 32.0 us here, 20.0 there, 12 x 16384 x 3072 34.8
-      // and 25.2; at 5120 channels 15.9 and 15.1, and 9 x 8192 x 2048 12.8 and 15.7.)
-      const bool one_round = is_bf16 && m >= 12 && rows >= 12288 && k >= 2048 && gemm_widens_bf16(m, rows, k);
+      const bool one_round = is_bf16 && bf16_one_round_route(m, rows, k);
       if (!no_skinny && !quick.needs_expand && !one_round &&
           skinny_upcast_supported(m, rows, k, raw_ptr(a), raw_ptr(weight), raw_ptr(out), quick.residual != nullptr)) {
         cuda_check(skinny_upcast_matmul(raw_ptr(a), is_bf16, m, rows, k, raw_ptr(weight),
@@ -2568,6 +2580,7 @@ int32_t fl_sm100_few_rows_route(int32_t entry, int32_t m, int32_t n, int32_t k) 
     case 0: return fewrow_tc_route(m, n, k) ? 2 : m <= 16 ? 1 : 0;
     case 1: return fewrow_q8_route(m, n, k) ? 2 : m <= 4 ? 1 : 0;
     case 2: return fewrow_w16_route(m, n, k) ? 2 : m <= 16 ? 1 : 0;
+    case 4: return m <= 16 && !bf16_one_round_route(m, n, k) ? 1 : 0;
     default: return -1;
   }
 }
@@ -2579,6 +2592,18 @@ int32_t fl_sm100_gemm_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_
     if (m < 1 || n < 1 || k < 1 || sms < 2) invalid("m, n, k are positive and the device has at least two SMs");
     int out[8];
     gemm_plan(static_cast<GemmKind>(kind), m, n, k, sms, allow_stream_k, out);
+    for (int i = 0; i < 8; ++i) plan[i] = out[i];
+    return clear_error();
+  });
+}
+
+int32_t fl_sm100_one_round_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t allow_stream_k, int32_t *plan) {
+  return guard([&]() -> int32_t {
+    if (!plan) invalid("plan is null");
+    if (kind < kGemmF16 || kind > kGemmE4M3) invalid("kind is 0 (half rows), 1 (bfloat16 rows) or 2 (quantised rows)");
+    if (m < 1 || n < 1 || k < 1 || sms < 2) invalid("m, n, k are positive and the device has at least two SMs");
+    int out[8];
+    gemm_split_describe(static_cast<GemmKind>(kind), m, n, k, sms, allow_stream_k != 0, out);
     for (int i = 0; i < 8; ++i) plan[i] = out[i];
     return clear_error();
   });

@@ -1327,7 +1327,7 @@ GemmSchedule gemm_schedule(int tiles, int max_units, int num_kb, bool allow_stre
   return s;
 }
 
-// Which kernel a product runs on, and its schedule; host arithmetic only.
+// Which form of this kernel a product runs on where it runs here, and its schedule; host arithmetic only.
 void gemm_plan(GemmKind kind, int m, int n, int k, int sms, int allow_stream_k, int *plan) {
   const int row_bytes = kind == kGemmE4M3 ? k : kind == kGemmNvf4 ? k / 2 : k * 2;
   const int num_kb = (row_bytes + kRowBytes - 1) / kRowBytes;

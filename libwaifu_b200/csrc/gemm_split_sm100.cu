@@ -440,6 +440,34 @@ bool make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t row_by
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// What a launch makes of a plan; host arithmetic only.
+struct SplitGeometry {
+  int num_kb, tiles_m, ctas;
+  int load_bytes, load_stages, wide_slots, wide_off;
+  int smem_bytes;
+};
+
+SplitGeometry split_geometry(bool widen, int m, int n, int k, const SplitPlan &plan) {
+  SplitGeometry g = {};
+  g.num_kb = (k * (widen ? 2 : 1) + kStageRowBytes - 1) / kStageRowBytes;
+  g.tiles_m = (m + kTileM - 1) / kTileM;
+  g.ctas = g.tiles_m * ((n + plan.block_n - 1) / plan.block_n) * plan.split;
+  g.load_bytes = kATileBytes + plan.block_n * (widen ? kStageRowBytes / 2 : kStageRowBytes);
+  g.wide_slots = plan.block_n <= 128 ? kMaxWideSlots : 2;
+  const int wide_bytes = widen ? g.wide_slots * plan.block_n * kStageRowBytes : 0;
+  const int longest = (g.num_kb + plan.split - 1) / plan.split;
+  g.load_stages = std::min((kSmemPerCta - 1024 - wide_bytes) / g.load_bytes, kMaxLoadStages);
+  if (widen) {
+    g.load_stages -= g.load_stages % g.wide_slots;
+  } else {
+    g.load_stages = std::min(g.load_stages, longest);
+  }
+  g.wide_off = g.load_stages * g.load_bytes;
+  const int exchange = plan.block_n / 4 * kGroupBytes;
+  g.smem_bytes = std::max(g.wide_off + wide_bytes, exchange) + 1024;
+  return g;
+}
+
 template <int KIND, bool WIDEN>
 cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {
   const uint64_t row_bytes = static_cast<uint64_t>(a.k) * (KIND == kKindF8 ? 1 : 2);
@@ -464,26 +492,16 @@ cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **
   SplitParams p = {};
   p.m = a.m;
   p.n = a.n;
-  p.num_kb = static_cast<int>((row_bytes + kStageRowBytes - 1) / kStageRowBytes);
-  p.tiles_m = (a.m + kTileM - 1) / kTileM;
-  const int tiles_n = (a.n + plan.block_n - 1) / plan.block_n;
+  const SplitGeometry g = split_geometry(WIDEN, a.m, a.n, a.k, plan);
+  p.num_kb = g.num_kb;
+  p.tiles_m = g.tiles_m;
   p.split = plan.split;
   p.block_n = plan.block_n;
   p.cols = plan.block_n / plan.split;
-  p.load_bytes = kATileBytes + plan.block_n * (WIDEN ? kStageRowBytes / 2 : kStageRowBytes);
-  p.wide_slots = plan.block_n <= 128 ? kMaxWideSlots : 2;
-  const int wide_bytes = WIDEN ? p.wide_slots * plan.block_n * kStageRowBytes : 0;
-  const int most = (kSmemPerCta - 1024 - wide_bytes) / p.load_bytes;
-  const int longest = (p.num_kb + plan.split - 1) / plan.split;
-  p.load_stages = most < kMaxLoadStages ? most : kMaxLoadStages;
-  if (WIDEN) {
-    p.load_stages -= p.load_stages % p.wide_slots;
-  } else if (p.load_stages > longest) {
-    p.load_stages = longest;
-  }
-  p.wide_off = p.load_stages * p.load_bytes;
-  const int ring = p.wide_off + wide_bytes;
-  const int exchange = plan.block_n / 4 * kGroupBytes;
+  p.load_bytes = g.load_bytes;
+  p.wide_slots = g.wide_slots;
+  p.load_stages = g.load_stages;
+  p.wide_off = g.wide_off;
   p.row_scale = a.row_scale;
   p.col_scale = a.col_scale;
   p.col_scale_scalar = a.col_scale_scalar;
@@ -500,9 +518,9 @@ cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **
   while (p.tmem_cols < bn) p.tmem_cols *= 2;
   p.status = a.status;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(p.tiles_m * tiles_n * plan.split), 1, 1);
+  cfg.gridDim = dim3(static_cast<unsigned>(g.ctas), 1, 1);
   cfg.blockDim = dim3(kSplitThreads, 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>((ring > exchange ? ring : exchange) + 1024);
+  cfg.dynamicSmemBytes = static_cast<size_t>(g.smem_bytes);
   cfg.stream = a.stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -588,6 +606,15 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
     }
   }
   return best;
+}
+
+void gemm_split_describe(GemmKind kind, int m, int n, int k, int sms, bool stream_k, int *plan) {
+  for (int i = 0; i < 8; ++i) plan[i] = 0;
+  const SplitPlan cut = gemm_split_plan(kind, kind != kGemmE4M3, m, n, k, sms, stream_k);
+  if (cut.split == 0) return;
+  const SplitGeometry g = split_geometry(kind != kGemmE4M3, m, n, k, cut);
+  plan[0] = cut.block_n, plan[1] = cut.split, plan[2] = g.ctas, plan[3] = g.num_kb;
+  plan[4] = g.load_stages, plan[5] = kind != kGemmE4M3 ? g.wide_slots : 0, plan[6] = g.load_bytes, plan[7] = g.smem_bytes;
 }
 
 cudaError_t launch_gemm_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {

@@ -20,6 +20,10 @@ struct SplitPlan {
 // the workspace for it).
 SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k);
 
+// The same with what a launch makes of it, all 0 without a plan: plan[8] is block_n, split, CTAs, K stages,
+// ring slots, widened slots (16-bit rows), bytes of a ring slot, dynamic shared memory of a CTA.
+void gemm_split_describe(GemmKind kind, int m, int n, int k, int sms, bool stream_k, int *plan);
+
 // Whether the kernel has all that `args` asks for (one destination of pitch n, no row groups, no
 // row maxima).
 bool gemm_split_supported(const GemmArgs &args);

@@ -1,5 +1,6 @@
 """The tile kernel's schedule, checked without a GPU: fl_sm100_gemm_plan() gives the numbers a
-launch would use, and the walk every role of a CTA makes over them (mirrored here from
+launch of that kernel uses (whether a product is launched there is the few-row kernels' and the
+one-round kernel's rules' business), and the walk every role of a CTA makes over them (mirrored here from
 gemm_sm100.cu's WorkWalk) must cover every K stage of every tile exactly once; a tile cut by the
 stream-K part must have exactly two holders, neighbouring units, the head held by the earlier unit
 (the first thing it does in that part) and the tail by the later one (the last thing it does), which
