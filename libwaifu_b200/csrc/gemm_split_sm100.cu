@@ -545,8 +545,7 @@ bool gemm_split_supported(const GemmArgs &a) {
 }
 
 // Estimated times in microseconds, fitted to a sweep of every block_n and split over 1280 to 16384
-// channels, k = 640 to 12288 and 16 to 2048 rows (the choice they make is within 1.5 % of the best
-// measured one on average, 13 % at worst). A stage takes its latency, or its bytes through L2 with
+// channels, k = 640 to 12288 and 16 to 2048 rows. A stage takes its latency, or its bytes through L2 with
 // every CTA pulling at once, or (widening) what the converters need for block_n rows; then come the
 // exchange and the epilogue, which grow with block_n, and the launch.
 //   77 x 2560 x 2048, half: 17.7 us on the persistent kernel, 11.2 here; 300 x 1280 x 640 15.4 and
@@ -568,11 +567,11 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
     if (tile_plan[6] > 0) return best;
   }
   // The persistent kernel: rounds of whole tiles (pairs of CTAs above one row block), a long K cut in
-  // halves where that leaves no unit without one (gemm_schedule), and for bfloat16 rows the pass
-  // that widens the weight ahead of it. 16-bit rows are taken over up to a tenth above that estimate,
-  // where the measured times cross (200 x 12288 x 3072 in half 32.2 and 30.9 us). e4m3 rows, whose K
-  // is never divided here, leave a K that the other kernel halves to it (512 x 3072 x 12288: 36.6 us
-  // there, 39.8 here).
+  // halves where that leaves no unit without one (gemm_schedule; its other cut, of the tail of more
+  // tiles, is not priced: 16-bit rows measured 0.63 to 0.98 of it here), and for bfloat16 rows the pass
+  // that widens the weight ahead of it. e4m3 rows, whose K is never divided here, leave a K that the
+  // other kernel halves to it, whether or not it may (512 x 3072 x 12288: 36.6 us there, 39.8 here; whole
+  // on both sides, 38.2 and 35.7, but 212 x 6736 x 11440 44.1 and 49.9).
   const int units = tiles_m == 1 ? sms : sms / 2;
   const long long tiles = tiles_m == 1 ? (n + 127) / 128 : static_cast<long long>((m + 255) / 256) * ((n + 255) / 256);
   float persistent = static_cast<float>((tiles + units - 1) / units * num_kb) *
@@ -583,7 +582,24 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
   }
   persistent += tiles_m == 1 ? 10.0f : 12.8f;
   if (kind == kGemmBF16) persistent += static_cast<float>(n) * k * 0.65e-6f;
-  float best_time = persistent * (widen ? 1.1f : 1.0f);
+  // Where the two kernels' measured times cross, over some 300 shapes of each kind with estimates from 0.75
+  // to 1.2 of each other and weights that come from HBM. Half: the persistent kernel takes 1.12 of its
+  // estimate, this one 0.98, so products up to a tenth above it come here (216 x 11544 x 1280: estimates
+  // 19.4 and 19.0, measured 17.6 here, 21.9 there). bfloat16: 1.06 and 1.00 up to k = 2048, 1.01 and 1.02
+  // to 4096, 0.96 and 1.05 beyond (1547 x 2024 x 2912, estimates 33.9 and 30.9, measured 35.5 and 33.3),
+  // but not where the widened copy it reads is 100 MB and no longer in L2 (367 x 8792 x 11296 132 us there,
+  // 108 here).
+  // e4m3 rows whose pitch is no multiple of a 32-byte sector cost a fifth sector per 128 bytes, and tiles
+  // of 128 rows read a long K more often than the persistent kernel's of 256 (1342 x 1672: 37.2 us here and
+  // 33.8 there at k = 7120, 26.9 and 29.3 at 7104), unless that one needs a second round.
+  // Taken and more than 2 % slower are 2, 4 and 8 of those shapes.
+  float margin = 1.0f;
+  if (kind == kGemmF16) margin = 1.1f;
+  if (kind == kGemmBF16) {
+    margin = static_cast<int64_t>(n) * k < 50'000'000 ? std::max(0.7f, 1.1f - 3.5e-5f * static_cast<float>(k)) : 1.0f;
+  }
+  if (!widen && k % 32 != 0 && num_kb > 32 && tiles_m > 1 && tiles <= units) margin = 0.85f;
+  float best_time = persistent * margin;
   const int max_split = widen ? 8 : 1;
   for (int split = 1; split <= max_split; split *= 2) {
     // clusters of four and eight do not fill every SM of a GPC

@@ -73,6 +73,19 @@ def test_widths_and_clusters_of_the_measured_shapes():
     assert cut(QUANTISED, 260, 9488, 5376) == (0, 0) and plan(QUANTISED, 260, 9488, 5376, 148, 0)["split"] == 1
 
 
+def test_products_that_measured_slower_stay_with_the_persistent_kernel():
+    """The line between the two kernels at shapes measured on both sides of it."""
+    for m, n, k in [(1547, 2024, 2912), (1578, 2080, 1936), (1211, 2144, 9488), (1190, 2256, 11008), (1687, 1536, 9600),
+                    (1024, 3072, 12288)]:
+        assert plan(BF16, m, n, k)["split"] == 0, (m, n, k)
+    for m, n, k in [(938, 2256, 6512), (1342, 1672, 7120), (271, 6888, 7728), (244, 9968, 8272)]:
+        assert plan(QUANTISED, m, n, k)["split"] == 0, (m, n, k)
+    for kind, m, n, k in [(HALF, 216, 11544, 1280), (HALF, 286, 12000, 1008), (BF16, 868, 5208, 2256), (BF16, 100, 1280, 32768),
+                          (BF16, 367, 8792, 11296),
+                          (QUANTISED, 1342, 1672, 7104), (QUANTISED, 297, 11472, 2704), (QUANTISED, 36, 880, 9552)]:
+        assert plan(kind, m, n, k)["split"] > 0, (m, n, k)
+
+
 def test_refusals():
     out = (ctypes.c_int32 * 8)()
     for bad in [(3, 1, 8, 16, 148), (-1, 1, 8, 16, 148), (0, 0, 8, 16, 148), (0, 1, 8, 16, 1)]:
