@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) quantize_fp8_act_reg_kernel(const uint16_
 }
 
 // The same with a warp to a row (k <= 256 * VPT), eight rows to a CTA: nothing waits for another warp,
-// a lane has up to sixteen 16-byte loads on their way, and the maximum is taken on pairs as they
+// a lane has up to eight 16-byte loads on their way, and the maximum is taken on pairs as they
 // lie (max of abs in the 16-bit type, exact; NaNs are passed over as fmaxf passes over them).
 template <int VPT>
 __global__ void __launch_bounds__(256) quantize_fp8_act_warp_kernel(const uint16_t *__restrict__ x, int is_bf16, int m, int k,
@@ -842,8 +842,17 @@ inline int capped_grid(int64_t work_items, int per_block) {
 
 int64_t helper_launch_count() { return g_helper_launches.load(); }
 
-// From how many rows on a warp to a row is enough to fill the GPU.
-constexpr int kWarpRows = 592;
+// Where a warp to a row measured faster than a CTA to a row, by the time of quantiser and product together
+// (e4m3 GEMM of 3072, 6144 and 12288 channels, weights from HBM), microseconds, CTA / warp:
+//   k      n       592 rows      1184          1480          2368          4352
+//   640    6144    25.9 / 25.6   26.1 / 25.6   26.5 / 25.2   42.4 / 40.3   59.4 / 56.0
+//   1024   6144    17.9 / 18.3   26.8 / 26.9   27.4 / 26.7   43.2 / 41.8   60.8 / 58.1
+//   2048   6144    20.5 / 21.5   30.3 / 31.0   31.2 / 31.2   47.7 / 47.0   65.8 / 64.6
+//   3072   6144    24.3 / 26.9   33.5 / 36.0   34.4 / 36.3   51.8 / 53.1   75.5 / 75.8
+//   3072   3072    17.7 / 18.1   23.0 / 25.5   24.5 / 26.1   34.0 / 35.1   46.8 / 46.0
+//   4096   12288   47.0 / 50.8   57.2 / 59.8   63.2 / 64.3   98.8 / 99.9   165 / 171
+// A deep row is long work for one warp, and eight of them to a CTA leave SMs without one below 1184 rows.
+inline bool warp_to_a_row(int m, int k) { return k <= 768 ? m >= 592 : k <= 2048 && m >= 1480; }
 
 cudaError_t quantize_fp8_act(const void *x, int is_bf16, int m, int k, uint8_t *codes, float *scales,
                              cudaStream_t stream) {
@@ -860,13 +869,11 @@ cudaError_t quantize_fp8_act(const void *x, int is_bf16, int m, int k, uint8_t *
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e;
-  if (vec && k <= 4096 && m >= kWarpRows) {
+  if (vec && warp_to_a_row(m, k)) {
     cfg.gridDim = dim3(static_cast<unsigned>((m + 7) / 8), 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
     if (k <= 1024) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<4>, xs, is_bf16, m, k, codes, scales);
-    else if (k <= 2048) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<8>, xs, is_bf16, m, k, codes, scales);
-    else if (k <= 3072) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<12>, xs, is_bf16, m, k, codes, scales);
-    else e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<16>, xs, is_bf16, m, k, codes, scales);
+    else e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_warp_kernel<8>, xs, is_bf16, m, k, codes, scales);
   } else if (vec && k <= 2048 * 8) {
     cfg.blockDim = dim3(256, 1, 1);
     if (k <= 2048 * 2) e = cudaLaunchKernelEx(&cfg, quantize_fp8_act_reg_kernel<2>, xs, is_bf16, k, codes, scales);

@@ -86,13 +86,35 @@ def test_nan_codes_stay_nan(flint, oracle, is_bf16):
 @pytest.mark.parametrize("m,k", [(592, 16), (593, 1040), (601, 2064), (600, 3072), (700, 3088), (592, 4096)])
 @pytest.mark.parametrize("is_bf16", [True, False])
 def test_a_warp_to_a_row_quantises_bit_exactly(flint, oracle, m, k, is_bf16):
-    """quantize_fp8_act_warp_kernel: from 592 rows, k up to 4096."""
+    """Either side of quantize_fp8_act_warp_kernel's range in k (its rows are below)."""
     F = flint
     rng = np.random.default_rng(m + k)
     x = randn(rng, (m, k))
     x[1] = 0
     x[2, k - 1], x[3, 0] = 90.0, -3e4
     x[4] *= 1e-6
+    x16 = oracle.narrow(x, is_bf16)
+    t = dev(F, x16, F.DType.BFLOAT16 if is_bf16 else F.DType.FLOAT16)
+    codes, scales = F.Tensor.empty((m, k), F.DType.FP8E4M3), F.Tensor.empty((m,), F.DType.FLOAT)
+    F.check(F.lib().fl_quantize_fp8_activation(t.raw(), codes.raw(), scales.raw()))
+    want_codes, want_scales = oracle.quantize_fp8_act(x16, is_bf16)
+    assert np.array_equal(scales.numpy().view(np.uint32), want_scales.view(np.uint32))
+    assert np.array_equal(codes.numpy(), want_codes)
+
+
+@pytest.mark.parametrize("m,k", [(592, 16), (593, 768), (592, 784), (1480, 784), (1481, 1024), (1487, 1040), (1480, 2048), (1480, 2064)])
+@pytest.mark.parametrize("is_bf16", [True, False])
+def test_rows_with_nans_and_infinities_quantise_bit_exactly(flint, oracle, m, k, is_bf16):
+    """quantize_fp8_act_warp_kernel (rows of up to 768 from 592 of them on, of up to 2048 from 1480) and
+    its neighbours: a row's maximum passes over its NaNs, whichever half of a pair they are in, an
+    infinity makes the scale one, and a row of NaNs has scale 0."""
+    F = flint
+    rng = np.random.default_rng(m + 3 * k)
+    x = randn(rng, (m, k))
+    x[0], x[1, :] = 0, np.nan
+    x[2, 0], x[3, k - 1], x[4, 1] = np.nan, np.nan, -np.nan
+    x[5, 3], x[6, k - 2], x[7, 0], x[7, 1] = np.inf, -np.inf, np.nan, np.inf
+    x[m - 1, k - 1], x[m - 2] = 3e4, 1e-7 * x[m - 2]
     x16 = oracle.narrow(x, is_bf16)
     t = dev(F, x16, F.DType.BFLOAT16 if is_bf16 else F.DType.FLOAT16)
     codes, scales = F.Tensor.empty((m, k), F.DType.FP8E4M3), F.Tensor.empty((m,), F.DType.FLOAT)
