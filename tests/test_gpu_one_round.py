@@ -1,8 +1,11 @@
 """GPU parity of the products whose tiles all run at once (gemm_split_sm100.cu), through the C ABI against
 the CPU oracle: one row and one column block and their remainders, K in one piece and divided over
 clusters of two, four and eight, K of an odd number of stages, a result no 16-byte store can write,
-every term of the epilogue, and the weight's NaN codes. Sizes that earlier dispatch rules send
-elsewhere (few rows) are left out."""
+every term of the epilogue, and the weight's NaN codes. Each shape's cut (tile width, CTAs of a cluster)
+stands beside it and is asserted, so that a change of the rule cannot empty the test. Half rows that the
+few-row kernels take are left out; bfloat16 ones are in where a rule sends them here."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -24,6 +27,16 @@ def matmul(F, a, codes, scale, is_bf16, addend=None):
     return y
 
 
+def cut(F, kind, m, n, k):
+    """(tile width, CTAs of a cluster) of a product of half (0), bfloat16 (1) or quantised (2) rows on this card."""
+    import torch
+    out = (ctypes.c_int32 * 8)()
+    F.check(F.lib().fl_sm100_one_round_plan(kind, m, n, k, torch.cuda.get_device_properties(0).multi_processor_count, 1, out))
+    return out[0], out[1]
+
+
+CUTS = {(77, 2560, 2048): (128, 4), (65, 1288, 640): (32, 2), (127, 136, 272): (32, 2), (128, 1280, 656): (32, 2), (129, 1304, 1040): (64, 2),
+        (300, 1280, 640): (64, 2), (512, 5120, 784): (144, 1), (1000, 1280, 1280): (160, 2), (70, 264, 4096): (128, 8), (130, 72, 12288): (128, 8)}
 SHAPES = [(77, 2560, 2048), (65, 1288, 640), (127, 136, 272), (128, 1280, 656), (129, 1304, 1040), (300, 1280, 640),
           (512, 5120, 784), (1000, 1280, 1280), (70, 264, 4096), (130, 72, 12288)]
 
@@ -32,6 +45,7 @@ SHAPES = [(77, 2560, 2048), (65, 1288, 640), (127, 136, 272), (128, 1280, 656), 
 @pytest.mark.parametrize("is_bf16", [False, True])
 @pytest.mark.parametrize("addend", ["none", "bias", "residual"])
 def test_matmul(flint, oracle, m, n, k, is_bf16, addend):
+    assert cut(flint, int(is_bf16), m, n, k) == CUTS[m, n, k]
     rng = np.random.default_rng(m * 7 + n + k)
     a = oracle.narrow(randn(rng, (m, k)), is_bf16)
     codes = random_codes(rng, n, k)
@@ -40,11 +54,71 @@ def test_matmul(flint, oracle, m, n, k, is_bf16, addend):
     check_parity(oracle, got, oracle.fp8_matmul(a, codes, [np.float32(0.0137)], add, is_bf16), is_bf16, what=f"{m}x{n}x{k}")
 
 
+@pytest.mark.parametrize("m,n,k,width,split", [(129, 11880, 272, 176, 1), (257, 8712, 272, 192, 1), (65, 11880, 1616, 192, 2),
+                                               (129, 2376, 2064, 192, 4), (257, 10296, 272, 224, 1), (129, 7128, 1616, 224, 2),
+                                               (257, 11880, 272, 256, 1), (129, 9064, 1616, 256, 2)])
+@pytest.mark.parametrize("is_bf16", [False, True])
+def test_matmul_in_wide_tiles(flint, oracle, m, n, k, width, split, is_bf16):
+    assert cut(flint, int(is_bf16), m, n, k) == (width, split)
+    rng = np.random.default_rng(m * 7 + n + k)
+    a, codes, add = oracle.narrow(randn(rng, (m, k)), is_bf16), random_codes(rng, n, k), oracle.narrow(randn(rng, (m, n)), is_bf16)
+    got = matmul(flint, a, codes, 0.0137, is_bf16, add)
+    check_parity(oracle, got, oracle.fp8_matmul(a, codes, [np.float32(0.0137)], add, is_bf16), is_bf16, what=f"{m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("m,n,k,width,split", [(12, 12288, 2048, 192, 2), (16, 16384, 3072, 224, 2), (17, 1288, 1040, 32, 2), (32, 3072, 3072, 128, 4),
+                                               (64, 2560, 656, 64, 2)])
+@pytest.mark.parametrize("addend", ["none", "bias", "residual"])
+def test_few_bfloat16_rows(flint, oracle, m, n, k, width, split, addend):
+    """Twelve to sixteen rows against many channels, and up to 64, which only half rows have a kernel for."""
+    assert cut(flint, 1, m, n, k) == (width, split)
+    rng = np.random.default_rng(m * 7 + n + k)
+    a, codes = oracle.narrow(randn(rng, (m, k)), True), random_codes(rng, n, k)
+    add = None if addend == "none" else oracle.narrow(randn(rng, (n,) if addend == "bias" else (m, n)), True)
+    before = flint.launch_count()
+    got = matmul(flint, a, codes, 0.0137, True, add)
+    assert flint.launch_count() == before + 1  # no pass that widens the weight
+    check_parity(oracle, got, oracle.fp8_matmul(a, codes, [np.float32(0.0137)], add, True), True, what=f"{m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("is_bf16", [False, True])
+def test_a_residual_that_repeats(flint, oracle, is_bf16):
+    """An addend of 67 rows under three blocks of 67: it repeats with a period that is no tile's."""
+    F = flint
+    dt = F.DType.BFLOAT16 if is_bf16 else F.DType.FLOAT16
+    rng = np.random.default_rng(8)
+    n, k = 1288, 1040
+    assert cut(F, int(is_bf16), 3 * 67, n, k) == (64, 2)
+    a, codes, add = oracle.narrow(randn(rng, (3, 67, k)), is_bf16), random_codes(rng, n, k), oracle.narrow(randn(rng, (67, n)), is_bf16)
+    out = F.Tensor.empty((3, 67, n), dt)
+    args = dev(F, a, dt), dev(F, codes, F.DType.FP8E4M3), dev(F, np.array([0.0137], np.float32), F.DType.FLOAT), dev(F, add, dt), out
+    before = F.launch_count()
+    F.check(F.lib().fl_fp8_matmul_add(*(t.raw() for t in args)))
+    assert F.launch_count() == before + 1  # nothing was expanded
+    got = out.numpy().reshape(3 * 67, n)
+    F.synchronize()
+    want = oracle.fp8_matmul(a.reshape(3 * 67, k), codes, [np.float32(0.0137)], np.tile(add, (3, 1)), is_bf16)
+    check_parity(oracle, got, want, is_bf16, what="periodic residual")
+
+
+LINEAR_CUTS = {(65, 1288, 656): (32, 1), (128, 3072, 3072): (32, 1), (200, 640, 2064): (32, 1), (257, 1280, 256): (32, 1), (700, 640, 272): (32, 1),
+               (1024, 1280, 1280): (80, 1), (90, 72, 12288): (0, 0),  # (the persistent kernel, K in halves)
+               (33, 4840, 256): (48, 1), (33, 7128, 272): (64, 1), (33, 11880, 256): (96, 1), (129, 7128, 256): (112, 1), (129, 10824, 272): (160, 1),
+               (129, 13112, 256): (192, 1), (257, 10296, 256): (224, 1), (257, 11880, 1040): (256, 1)}
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 4840, 256), (33, 7128, 272), (33, 11880, 256), (129, 7128, 256), (129, 10824, 272), (129, 13112, 256),
+                                   (257, 10296, 256), (257, 11880, 1040)])
+def test_linear_in_tiles_of_every_width(flint, oracle, m, n, k):
+    test_linear_with_every_term(flint, oracle, m, n, k, True)
+
+
 @pytest.mark.parametrize("m,n,k", [(65, 1288, 656), (128, 3072, 3072), (200, 640, 2064), (257, 1280, 256), (700, 640, 272),
                                    (1024, 1280, 1280), (90, 72, 12288)])
 @pytest.mark.parametrize("is_bf16", [True, False])
 def test_linear_with_every_term(flint, oracle, m, n, k, is_bf16):
     F = flint
+    assert cut(F, 2, m, n, k) == LINEAR_CUTS[m, n, k]
     rng = np.random.default_rng(m + n + k)
     dt = F.DType.BFLOAT16 if is_bf16 else F.DType.FLOAT16
     x = oracle.narrow(randn(rng, (m, k)), is_bf16)
@@ -61,6 +135,7 @@ def test_results_off_a_16_byte_boundary(flint, oracle):
     F = flint
     rng = np.random.default_rng(5)
     m, n, k = 100, 264, 512
+    assert cut(F, 0, m, n, k)[1] > 0
     a, codes = oracle.narrow(randn(rng, (m, k)), False), random_codes(rng, n, k)
     store = F.Tensor.from_numpy(np.zeros(m * n + 8, np.uint16), F.DType.FLOAT16, F.Device.CUDA)
     out = store.view_as((m, n), (n, 1), 1)
@@ -76,6 +151,7 @@ def test_results_off_a_16_byte_boundary(flint, oracle):
 def test_nan_codes_stay_nan(flint, oracle, is_bf16):
     rng = np.random.default_rng(6)
     m, n, k = 80, 1280, 640
+    assert cut(flint, int(is_bf16), m, n, k)[1] > 0
     a, codes = oracle.narrow(randn(rng, (m, k)), is_bf16), random_codes(rng, n, k)
     codes[3, 17], codes[700, 639] = 0x7F, 0xFF
     y = oracle.widen(matmul(flint, a, codes, 0.0137, is_bf16), is_bf16)
@@ -140,6 +216,22 @@ def test_causal_units_of_several_heads(flint, oracle, n, h, hk, L, S, d):
     assert np.abs(got - want).max() <= 2 * oracle.ulp16_at(float(np.abs(want).max()), True)
 
 
+@pytest.mark.parametrize("block_size", [64, 100, 128, 257, 400])
+@pytest.mark.parametrize("n,h,hk,L,S,d", [(2, 3, 3, 600, 600, 64), (1, 4, 2, 260, 900, 128), (3, 2, 1, 385, 385, 128)])
+def test_block_causal_units_of_several_heads(flint, oracle, n, h, hk, L, S, d, block_size):
+    """The same under the block-causal mask: blocks below a tile of keys, across its boundary, of a tile and
+    wider than two, so that both tiles of a unit may end on the same block of keys or on different ones."""
+    F = flint
+    rng = np.random.default_rng(L + S + d + block_size)
+    q, k, v = (oracle.narrow(randn(rng, s), True) for s in ((n, h, L, d), (n, hk, S, d), (n, hk, S, d)))
+    out = F.attention(*(dev(F, t, F.DType.BFLOAT16) for t in (q, k, v)), 2, block_size)
+    got = oracle.widen(out.numpy(), True).astype(np.float64)
+    F.synchronize()
+    want = oracle.attention(q, k, v, 2, True, block_size)
+    assert oracle.rel_l2(got, want) <= 5e-3
+    assert np.abs(got - want).max() <= 2 * oracle.ulp16_at(float(np.abs(want).max()), True)
+
+
 @pytest.mark.parametrize("m,n,k", [(260, 9488, 5376), (814, 4816, 11120), (1024, 384, 12288), (300, 1280, 1280), (200, 2584, 880),
                                    (128, 3072, 3072)])
 def test_linears_on_quantised_rows_give_the_same_bits(flint, m, n, k):
@@ -169,4 +261,7 @@ def test_linears_on_quantised_rows_give_the_same_bits(flint, m, n, k):
     out = F.Tensor.empty((m, n), bf)
     F.fp8_linear_quantized(xc, xs, codes, scales, bias, res, F.ACT_GELU_TANH, out)
     assert np.array_equal(out.numpy(), want), "on rows quantised beforehand"
+    if cut(F, 2, m, n, k)[1] > 0:  # (without its workspace the persistent kernel cuts nothing)
+        F.fp8_linear_static(x, codes, scales, bias, res, F.ACT_GELU_TANH, out)
+        assert np.array_equal(out.numpy(), want), "without an allocation"
     F.synchronize()
