@@ -178,10 +178,12 @@ def test_a_warp_to_a_row_quantises_bit_exactly(flint, oracle, m, k, is_bf16):
     assert np.array_equal(codes.numpy(), want_codes)
 
 
-@pytest.mark.parametrize("m,k", [(592, 16), (593, 768), (592, 784), (1480, 784), (1481, 1024), (1487, 1040), (1480, 2048), (1480, 2064)])
+@pytest.mark.parametrize("m,k", [(592, 16), (593, 768), (592, 784), (1480, 784), (1481, 1024), (1487, 1040), (1480, 2048), (1480, 2064),
+                                 (3551, 2064), (3552, 2064), (3555, 3072), (3552, 3088)])
 @pytest.mark.parametrize("is_bf16", [True, False])
 def test_rows_with_nans_and_infinities_quantise_bit_exactly(flint, oracle, m, k, is_bf16):
-    """quantize_fp8_act_warp_kernel (rows of up to 768 from 592 of them on, of up to 2048 from 1480) and
+    """quantize_fp8_act_warp_kernel (rows of up to 768 from 592 of them on, of up to 2048 from 1480, of
+    up to 3072 from 3552) and
     its neighbours: a row's maximum passes over its NaNs, whichever half of a pair they are in, an
     infinity makes the scale one, and a row of NaNs has scale 0."""
     F = flint
