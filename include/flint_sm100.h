@@ -219,12 +219,13 @@ FLAPI int32_t fl_fp8_linear(fl_tensor_view_t a, fl_tensor_view_t data, fl_tensor
  * in one fixed device array compiled into the library, about 16.3 MiB, which every GPU that loads
  * the library holds until the process ends. The call makes no cudaMalloc, cudaFree, cudaHostAlloc
  * or other allocating call. Arguments and checks are fl_fp8_linear()'s; the arithmetic is the
- * quantiser kernel followed by the product kernel fl_fp8_linear() takes from five rows on (the
+ * quantiser kernel followed by the product kernel fl_fp8_linear() takes from five rows on (a
  * tcgen05 tile GEMM, or for at most 32 rows against a wide weight the few-row tensor-core kernel)
- * for every row count, so from five rows on the results are bit-identical to fl_fp8_linear()'s, and
- * for one to four rows, where fl_fp8_linear() may take a one-launch few-row kernel with another
- * summation order, they agree within the path's tolerance. FLINT_SM100_SINGLE_CTA and
- * fl_sm100_gemm_timing() do not apply here.
+ * for every row count, so from five rows on the results are bit-identical to fl_fp8_linear()'s,
+ * except where that cuts a product's tiles in two along k (fl_sm100_gemm_plan's [6]; its workspace is
+ * an allocation). There, and for one to four rows, where fl_fp8_linear() may take a one-launch
+ * few-row kernel with another summation order, they agree within the path's tolerance.
+ * FLINT_SM100_SINGLE_CTA and fl_sm100_gemm_timing() do not apply here.
  *
  * Limits, refused with FL_ERROR_INVALID_ARG before anything is launched: at most 65536 activation
  * rows (the product of a's leading dimensions), at most 16 Mi elements in m * k (4352 x 3072 fits),
@@ -273,7 +274,9 @@ FLAPI int32_t fl_fp8_linear_scatter(fl_tensor_view_t a, fl_tensor_view_t data, f
  *     this GPU's and, through fl_sm100_ipc_import(), its peers', with plain 16-byte stores. Leaves the
  *     rows' scales in row_scales <float>(rows) if that is not NULL. k, ld, col0 multiples of 16.
  * The gathered codes and scales then go to fl_fp8_linear_quantized(), and the result equals the
- * unsplit fl_fp8_linear chain bit for bit. The caller orders the ranks (a barrier or any collective
+ * unsplit fl_fp8_linear chain bit for bit, unless the few-row kernels take the unsplit products or
+ * only one of the two has its tiles cut in two along k (fl_sm100_gemm_plan's [6]: products of fewer
+ * columns have fewer tiles). The caller orders the ranks (a barrier or any collective
  * on the stream) between the scatter and the first read. No counterpart in the reference. */
 FLAPI int32_t fl_fp8_linear_amax(fl_tensor_view_t a, fl_tensor_view_t data, fl_tensor_view_t scales, fl_tensor_view_t bias,
                                  fl_tensor_view_t residual, int32_t act, fl_tensor_view_t out, fl_tensor_view_t row_amax);

@@ -397,8 +397,9 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           break;
         }
         tc_fence_after_sync();
-        // Two independent accumulator chains, issued in turn: an instruction into an accumulator
-        // waits for the one before it, so in turn they take the time of one chain.
+        // The two products' instructions are issued in turn. Under an elected lane one after the other
+        // measured the same (1 x 12 x 4352 x 128 in diagonal blocks of 256: 51.8 us both ways, head_dim
+        // 64 34.5 and 35.0; 8 x 32 x 100 x 4000 168.8 and 169.3).
         static_assert(kScoreMmas == kOutMmas || kScoreMmas * 2 == kOutMmas, "interleave below");
         constexpr int kOutPerScore = kOutMmas / kScoreMmas;
         const bool odd = (j & 1) != 0;
@@ -718,9 +719,10 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (threadIdx.x == 0) atomicCAS(p.status, 0u, kStatusAttentionLayout);
     return;
   }
-  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its keys and values in L2. Under
-  // the causal masks the later queries have more keys to walk: the last unit of every head goes
-  // first, then the one before it, so that the grid ends on the short ones whatever the head.
+  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its
+  // keys and values in L2. Under the causal masks the later queries have more keys to walk: the last
+  // unit of every head goes first, then the one before it, so that the grid ends on the short ones
+  // whatever the head.
   int unit = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
   if (p.mask_type != 0) {
     const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
@@ -732,8 +734,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int q0 = unit * (kTiles * kBlockQ);
   const int kv_head = head / p.group;
   const int offset = p.kv_len - p.q_len;
-  // Both tiles walk the blocks of keys that some query of the CTA sees; a block none of a tile's
-  // queries sees costs that tile a block of zero probabilities.
+  // Both tiles start at the first block of keys that some query of the CTA sees.
   const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
   const int kv_begin = first_key_of(p, q0 + offset);
   const int kv_end = last_key_of(p, last_row + offset) + 1;

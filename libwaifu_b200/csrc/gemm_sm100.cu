@@ -68,8 +68,9 @@ constexpr int kNumWarps = 12;
 constexpr int kNumThreads = kNumWarps * 32;
 constexpr int kMaxEpilogueWarps = 8;
 constexpr int kPusherWarps = 2;
-// Mixed form: the converter warps share out the stages of the ring, two warps to a stage (slot s
-// belongs to group s % 3, so a group sees every phase of the barriers it waits on). A stage's way
+// Mixed form: the converter warps share out the slots of the ring, two warps to a slot (slot s
+// belongs to group s % 3, so a group sees every phase of the barriers it waits on; of the pair form's
+// five slots the first two groups have two each and the third one). A stage's way
 // through a warp (wait, read, widen, write, proxy fence, arrive) is some 0.4 us however few bytes
 // it has; with all six warps on every stage that was what paced the kernel.
 constexpr int kConverterGroups = 3;
