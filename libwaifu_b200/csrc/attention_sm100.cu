@@ -934,7 +934,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       abort_flag = 1;
       atomicCAS(p.status, 0u, kStatusAttentionTimeout);
     }
-    } else {
+  } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     if (warp == kProducerWarp2) {
       // ------------------------------------------------------------------ producer
