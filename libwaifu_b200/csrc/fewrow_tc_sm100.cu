@@ -364,6 +364,7 @@ struct QParams {
   int ntok;    // N of the instruction: the rows rounded up to a multiple of 16
   int cpc;     // channels per CTA: at most 128, a multiple of 8
   int stages;
+  int weight_early;  // the kernel ahead is the rows' quantiser, started once all before it was complete
   uint32_t tmem_cols;
   uint32_t *status;
 };
@@ -403,7 +404,7 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
     // (the first stages of the weight into L2 ahead of the wait on the kernel before, as above)
-    for (int st = 0; st < num_stages && st < p.stages; ++st) {
+    for (int st = 0; !p.weight_early && st < num_stages && st < p.stages; ++st) {
 #pragma unroll
       for (int a = 0; a < kAtoms; ++a) tma_prefetch_l2_2d(&tmap_w, st * kStageK + a * 128, n0);
     }
@@ -416,6 +417,26 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t load_bytes = static_cast<uint32_t>(p.cpc * kStageK + kAtoms * x_atom);  // (bytes outside arrive as zeros)
+  auto load_w = [&](int st) {
+#pragma unroll
+    for (int a = 0; a < kAtoms; ++a) {
+      tma_load_2d(smem + (st % p.stages) * stage_bytes + a * kAtomBytes, &tmap_w, &full_bar[st % p.stages], st * kStageK + a * 128, n0);
+    }
+  };
+  // Behind the rows' own quantiser, which lets this kernel start once everything ahead of it in the
+  // stream is complete, only the rows have to be waited for: the ring's weight is on its way under the
+  // quantiser (2 x 18432 x 3072 in bfloat16, both launches, weight from HBM: 14.37 -> 13.93 us).
+  const int early = p.weight_early ? min(num_stages, p.stages) : 0;
+  if (warp == kQProducer && early > 0) {
+    if (elect_one()) {
+      for (int st = 0; st < early; ++st) {
+        mbar_arrive_expect_tx(&full_bar[st], load_bytes);
+        load_w(st);
+      }
+    }
+    __syncwarp();
+  }
   griddep_wait();
   griddep_launch_dependents();
 
@@ -424,16 +445,17 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       bool ok = true;
       for (int st = 0; st < num_stages && ok; ++st) {
         const int s = st % p.stages;
-        if (!mbar_wait(&empty_bar[s], ((st / p.stages) & 1) ^ 1, &abort_flag)) {
-          ok = false;
-          break;
+        if (st >= early) {
+          if (!mbar_wait(&empty_bar[s], ((st / p.stages) & 1) ^ 1, &abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&full_bar[s], load_bytes);
+          load_w(st);
         }
-        uint8_t *base = smem + s * stage_bytes;
-        mbar_arrive_expect_tx(&full_bar[s], static_cast<uint32_t>(p.cpc * kStageK + kAtoms * x_atom));  // (bytes outside arrive as zeros)
 #pragma unroll
         for (int a = 0; a < kAtoms; ++a) {
-          tma_load_2d(base + a * kAtomBytes, &tmap_w, &full_bar[s], st * kStageK + a * 128, n0);
-          tma_load_2d(base + kRawWBytes + a * x_atom, &tmap_x, &full_bar[s], st * kStageK + a * 128, 0);
+          tma_load_2d(smem + s * stage_bytes + kRawWBytes + a * x_atom, &tmap_x, &full_bar[s], st * kStageK + a * 128, 0);
         }
       }
       if (!ok) {
@@ -674,8 +696,8 @@ namespace {
 // elem: bytes per element of both operands (1: e4m3 codes, 2: half or bfloat16 as `is_bf16` says).
 cudaError_t launch_q8(int elem, const void *rows, const float *row_scale, int m, int n, int k, const void *w,
                       const float *col_scale, int col_scale_scalar, const void *bias, const void *residual,
-                      int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, uint32_t *status,
-                      cudaStream_t stream, const char **why) {
+                      int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, bool weight_early,
+                      uint32_t *status, cudaStream_t stream, const char **why) {
   *why = "";
   const int ntok = (m + 15) / 16 * 16;
   const uint64_t kbytes = static_cast<uint64_t>(k) * elem;
@@ -723,6 +745,7 @@ cudaError_t launch_q8(int elem, const void *rows, const float *row_scale, int m,
   p.ntok = ntok;
   p.cpc = cpc;
   p.stages = stages;
+  p.weight_early = weight_early ? 1 : 0;
   const int acc_cols = q8::kIssuers * q8::kQChains * ntok;
   p.tmem_cols = acc_cols <= 64 ? 64u : acc_cols <= 128 ? 128u : acc_cols <= 256 ? 256u : 512u;
   p.status = status;
@@ -747,10 +770,10 @@ cudaError_t launch_q8(int elem, const void *rows, const float *row_scale, int m,
 
 cudaError_t fewrow_q8_linear(const uint8_t *codes, const float *row_scale, int m, int n, int k, const uint8_t *w,
                              const float *col_scale, int col_scale_scalar, const void *bias, const void *residual,
-                             int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, uint32_t *status,
-                             cudaStream_t stream, const char **why) {
+                             int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, bool weight_early,
+                             uint32_t *status, cudaStream_t stream, const char **why) {
   return launch_q8(1, codes, row_scale, m, n, k, w, col_scale, col_scale_scalar, bias, residual, residual_rows, residual_ld,
-                   act, is_bf16, out, status, stream, why);
+                   act, is_bf16, out, weight_early, status, stream, why);
 }
 
 bool fewrow_w16_supported(int m, int n, int k, const void *x, const void *w, const void *out) {
@@ -764,8 +787,8 @@ bool fewrow_w16_supported(int m, int n, int k, const void *x, const void *w, con
 cudaError_t fewrow_w16_matmul(const void *x, int is_bf16, int m, int n, int k, const void *w, const void *bias,
                               const void *residual, int residual_rows, int64_t residual_ld, void *out, uint32_t *status,
                               cudaStream_t stream, const char **why) {
-  return launch_q8(2, x, nullptr, m, n, k, w, nullptr, 0, bias, residual, residual_rows, residual_ld, 0, is_bf16, out, status,
-                   stream, why);
+  return launch_q8(2, x, nullptr, m, n, k, w, nullptr, 0, bias, residual, residual_rows, residual_ld, 0, is_bf16, out, false,
+                   status, stream, why);
 }
 
 }  // namespace flsm100

@@ -27,10 +27,13 @@ bool fewrow_q8_supported(int m, int n, int k, const void *codes, const void *w, 
 
 // out (m, n) = round16( act( (codes . w^T) * (row_scale[row] * col_scale[channel or 0]) + bias ) + residual ),
 // the arithmetic of fl_fp8_linear's epilogue in its order (fp32 accumulation). One launch, no scratch.
+// `weight_early`: the launch ahead of it is quantize_fp8_act's of these rows, which lets the next kernel
+// start only after its own wait, when all earlier work is complete: the weight is then read without
+// waiting for it (not where a copy of the weight was queued between the two).
 cudaError_t fewrow_q8_linear(const uint8_t *codes, const float *row_scale, int m, int n, int k, const uint8_t *w,
                              const float *col_scale, int col_scale_scalar, const void *bias, const void *residual,
-                             int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, uint32_t *status,
-                             cudaStream_t stream, const char **why);
+                             int residual_rows, int64_t residual_ld, int act, int is_bf16, void *out, bool weight_early,
+                             uint32_t *status, cudaStream_t stream, const char **why);
 
 // The same kernel on 16-bit operands (fl_matmul's linear-layer case, kind::f16): x (m, k) and w (n, k)
 // half or bfloat16, out = round16(x . w^T + bias (n) + residual rows). At most 64 rows, k and n

@@ -1533,15 +1533,16 @@ bool fewrow_q8_wins(int m, int rows, int k) {
   return !off && fewrow_q8_route(m, rows, k);
 }
 
-// Runs it if it wins and can take the operands; false when the tile kernel should run.
+// Runs it if it wins and can take the operands; false when the tile kernel should run. `weight_early`: the
+// rows' quantiser is the launch right ahead.
 bool try_fewrow_q8(const uint8_t *codes, const float *row_scales, int m, int rows, int k, const void *w,
-                   const Epilogue &ep, int is_bf16, void *out, uint32_t *status) {
+                   const Epilogue &ep, int is_bf16, void *out, bool weight_early, uint32_t *status) {
   if (ep.row_amax != nullptr || ep.num_extra_out != 0 || ep.out_ld != 0) return false;
   if (!fewrow_q8_wins(m, rows, k) || !fewrow_q8_supported(m, rows, k, codes, w, out)) return false;
   const char *why = "";
   cudaError_t e = fewrow_q8_linear(codes, row_scales, m, rows, k, reinterpret_cast<const uint8_t *>(w), ep.col_scale,
                                    ep.col_scale_scalar, ep.bias, ep.residual, ep.residual_rows, ep.residual_ld, ep.act,
-                                   is_bf16, out, status, 0, &why);
+                                   is_bf16, out, weight_early, status, 0, &why);
   if (e != cudaSuccess) cuda_check(e, (std::string("few-row FP8 linear: ") + why).c_str());
   ++g_gemm_launches;
   return true;
@@ -1644,7 +1645,9 @@ int32_t fp8_linear_impl(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_tensor
     }
     ep.act = act;
     ep.row_amax = row_amax;
-    if (try_fewrow_q8(codes, row_scales, m, rows, k, w_ptr, ep, is_bf16, raw_ptr(out), status_word())) return clear_error();
+    if (try_fewrow_q8(codes, row_scales, m, rows, k, w_ptr, ep, is_bf16, raw_ptr(out), !w_misaligned, status_word())) {
+      return clear_error();
+    }
     run_gemm(kGemmE4M3, m, rows, k, codes, w_ptr, nullptr, nullptr, ep, is_bf16, raw_ptr(out));
     return clear_error();
   });
@@ -2251,7 +2254,7 @@ int32_t fp8_linear_quantized_impl(fl_tensor_view_t codes_h, fl_tensor_view_t row
     }
     if (out_h && rows_per_group == 0 &&
         try_fewrow_q8(reinterpret_cast<const uint8_t *>(a_ptr), ep.row_scale, m, rows, k, w_ptr, ep,
-                               out_dtype == FL_DTYPE_BFLOAT16, sd.first, status_word())) {
+                      out_dtype == FL_DTYPE_BFLOAT16, sd.first, false, status_word())) {
       return clear_error();
     }
     run_gemm(kGemmE4M3, m, rows, k, a_ptr, w_ptr, nullptr, nullptr, ep, out_dtype == FL_DTYPE_BFLOAT16, sd.first);
@@ -2785,7 +2788,7 @@ int32_t fl_fp8_linear_static(fl_tensor_view_t a_h, fl_tensor_view_t data_h, fl_t
         ep.residual_ld = rows;
       }
       ep.act = act;
-      if (try_fewrow_q8(codes, row_scales, m, rows, k, raw_ptr(weight), ep, is_bf16, raw_ptr(out), status)) return clear_error();
+      if (try_fewrow_q8(codes, row_scales, m, rows, k, raw_ptr(weight), ep, is_bf16, raw_ptr(out), true, status)) return clear_error();
     }
 
     GemmArgs g{};

@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(128) quantize_fp8_act_kernel(const uint16_t *_
                                                              uint8_t *__restrict__ codes,
                                                              float *__restrict__ scales) {
   griddep_wait();
+  griddep_launch_dependents();
   __shared__ float red[4];
   const int64_t row = blockIdx.x;
   const uint16_t *xr = x + row * k;
@@ -98,7 +99,6 @@ __global__ void __launch_bounds__(128) quantize_fp8_act_kernel(const uint16_t *_
   const float scale = __fdiv_rn(amax, 448.0f);
   const float inv = __frcp_rn(scale > 0.0f ? scale : 1.0f);
   if (threadIdx.x == 0) scales[row] = scale;
-  griddep_launch_dependents();
   if (VEC) {
     const uint4 *xv = reinterpret_cast<const uint4 *>(xr);
     uint2 *cv = reinterpret_cast<uint2 *>(cr);
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(256) quantize_fp8_act_reg_kernel(const uint16_
                                                                  uint8_t *__restrict__ codes,
                                                                  float *__restrict__ scales) {
   griddep_wait();
+  griddep_launch_dependents();
   __shared__ float red[8];
   const int64_t row = blockIdx.x;
   const uint4 *xv = reinterpret_cast<const uint4 *>(x + row * k);
@@ -140,7 +141,6 @@ __global__ void __launch_bounds__(256) quantize_fp8_act_reg_kernel(const uint16_
   const float scale = __fdiv_rn(amax, 448.0f);
   const float inv = __frcp_rn(scale > 0.0f ? scale : 1.0f);
   if (threadIdx.x == 0) scales[row] = scale;
-  griddep_launch_dependents();
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * 256;

@@ -147,6 +147,33 @@ def test_few_rows_on_the_tensor_cores_match_the_tile_kernel(flint, oracle):
     assert np.array_equal(out2.numpy(), few)
 
 
+@pytest.mark.parametrize("m,n,k", [(2, 18432, 3072), (16, 8200, 2064)])
+def test_a_weight_written_just_ahead_is_the_one_read(flint, m, n, k):
+    """The product reads its weight while its own quantiser still runs: a weight that the launch ahead of
+    that quantiser writes has to be complete by then. The same buffer rewritten ahead of every call gives
+    the bits that weights of their own give."""
+    import torch
+    F = flint
+    gen = torch.Generator(device="cuda").manual_seed(k + n)
+    view = lambda t, dt: F.Tensor.from_device_ptr(t.data_ptr(), tuple(t.shape), dt, keepalive=t)
+    x = view(torch.randn((m, k), device="cuda", generator=gen).bfloat16(), F.DType.BFLOAT16)
+    scales = view(torch.rand((n,), device="cuda", generator=gen), F.DType.FLOAT)
+    weights = [torch.randn((n, k), device="cuda", generator=gen).to(torch.float8_e4m3fn).view(torch.uint8) for _ in range(3)]
+    outs = [torch.zeros((m, n), device="cuda", dtype=torch.bfloat16) for _ in range(12)]
+    own = [torch.zeros((m, n), device="cuda", dtype=torch.bfloat16) for _ in weights]
+    buffer = torch.zeros_like(weights[0])
+    for w, out in zip(weights, own):
+        torch.cuda.synchronize()
+        F.fp8_linear(x, view(w, F.DType.FP8E4M3), scales, None, None, 0, out=view(out, F.DType.BFLOAT16))
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        buffer.copy_(weights[i % 3])
+        F.fp8_linear(x, view(buffer, F.DType.FP8E4M3), scales, None, None, 0, out=view(out, F.DType.BFLOAT16))
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        assert torch.equal(out.view(torch.int16), own[i % 3].view(torch.int16)), i
+
+
 @pytest.mark.parametrize("m,rows_per_group,n,k", [(768, 256, 264, 320), (1152, 512, 520, 3072), (8704, 4352, 3072, 512)])
 def test_row_groups_equal_one_product_per_group(flint, oracle, m, rows_per_group, n, k):
     """fl_fp8_linear_quantized_grouped: rows in groups, each with its own per-channel scales and bias
