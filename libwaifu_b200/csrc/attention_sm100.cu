@@ -103,6 +103,7 @@ struct KernelParams {
   int mask_type;   // 0 none, 1 causal, 2 block causal, 3 block diagonal (flint/capi.h:118-133)
   int block_size;
   float scale_log2;
+  int take_over;  // two-tile kernel: CTAs go on with the units of CTAs that have not started
   int v_direct;  // two-tile kernel: v is read as it lies (an MN-major operand), not through its transposition
   uint32_t *status;
 };
@@ -651,6 +652,12 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 // ...); tensor memory holds 2 x (128 + head_dim) <= 512 columns. Per tile the chain is serial
 // (scores -> softmax -> P -> product -> the next scores, which overwrite P); the other tile's
 // chain runs in its gaps.
+//
+// The grid has a CTA per unit (two tiles of one head's queries), but a running CTA may take over units
+// whose own CTA has not started yet (clusterlaunchcontrol.try_cancel) instead of leaving its SM to
+// it. Keys, values and queries of the next unit then arrive, and its first scores are computed, under
+// the last products and the output of the one before, and barriers and tensor memory are set up once
+// per SM. The hardware hands the units out in the grid's order, as it starts CTAs.
 constexpr int kTiles = 2;
 constexpr int kTileWarps = 4;
 constexpr int kSoftmaxWarps2 = kTiles * kTileWarps;
@@ -658,9 +665,9 @@ constexpr int kProducerWarp2 = kSoftmaxWarps2;
 constexpr int kMmaWarp2 = kSoftmaxWarps2 + 1;
 // Twelve warps, three warpgroups, launched with 168 registers a thread; the one that loads and issues
 // (two of its warps have nothing to do) gives its own up to the two of the softmax, which hold a
-// row of 128 scores: 128 x 88 + 256 x 208 = 384 x 168.
+// row of 128 scores: 128 x 96 + 256 x 200, which is below 384 x 168.
 constexpr int kThreads2 = (kSoftmaxWarps2 + 4) * 32;
-constexpr int kIssueRegs = 88, kSoftmaxRegs = 208;
+constexpr int kIssueRegs = 96, kSoftmaxRegs = 200;
 static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2 * 168, "no more than the block was launched with");
 // A block's probabilities are handed over in so many parts of its keys. At head_dim 128 the product of
 // the first half runs under the exponentials of the second (2 x 24 x 4352: 396 -> 386 us); at 64,
@@ -669,9 +676,14 @@ static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2
 template <int D>
 constexpr int kPartsOf = D == 128 ? 2 : 1;
 constexpr int kMaxSlots = 6;
+constexpr int kTakeOverBlocks = 16;  // the longest walk whose CTA goes on with another unit
 
 struct Tail2 {
-  uint64_t q_full_bar[kTiles];
+  uint4 claim;            // the answer to the last try_cancel
+  uint64_t claim_bar;     // ... which has arrived
+  uint64_t unit_full_bar[2], unit_empty_bar[2];  // producer -> all: the next unit is in next_unit[slot]; all -> producer
+  int4 next_unit[2];      // block indices x, y, z of a unit, w = 0 when there is none left
+  uint64_t q_full_bar[kTiles], q_empty_bar[kTiles];
   uint64_t slot_full_bar[kMaxSlots], slot_empty_bar[kMaxSlots];
   uint64_t s_full_bar[kTiles];   // MMA -> softmax: the tile's scores are in tensor memory
   uint64_t p_full_bar[kTiles][2];  // softmax -> MMA: that part of the tile's probabilities is in tensor memory
@@ -694,6 +706,7 @@ struct Layout2 {
   static constexpr int kQOff = 0;
   static constexpr int kSlotOff = kQOff + kTiles * kQBytes;
   static constexpr int kTailOff = kSlotOff + kSlots * kSlotBytes;
+  static_assert(kTailOff % 16 == 0, "the claim is 16-byte aligned");
   static constexpr int kSmemBytes = kTailOff + static_cast<int>(sizeof(Tail2));
   static constexpr int kSCols = kBlockKv;           // tile t's scores at column t * kSCols, its P over their first half
   static constexpr int kOCol = kTiles * kSCols;     // tile t's output at kOCol + t * D
@@ -701,6 +714,70 @@ struct Layout2 {
   static_assert(kOCol + kTiles * D <= kTmemCols, "tensor memory holds 512 columns");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
+
+// Two tiles of 128 queries of one head and the blocks of keys they walk, from the first on (of the
+// masks only the block diagonal one hides a run's first keys, and it is not served here).
+struct Unit2 {
+  int head, batch, q0;
+  int num_blocks;
+  int blocks[kTiles];  // how many of them each tile walks: 0 for a tile past the last query
+
+  // Without a mask the units of one head run side by side and share its keys and values in L2. Under
+  // the causal masks the later queries have more keys to walk: the last unit of every head goes first,
+  // then the one before it, so that the grid ends on the short ones whatever the head.
+  __device__ __forceinline__ Unit2(const KernelParams &p, int x, int y, int z) : head(y), batch(z) {
+    int unit = x;
+    if (p.mask_type != 0) {
+      const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
+      const int order = x + units * (y + heads * z);
+      unit = units - 1 - order / all;
+      head = order % all % heads;
+      batch = order % all / heads;
+    }
+    q0 = unit * (kTiles * kBlockQ);
+    const int offset = p.kv_len - p.q_len;
+    const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
+    num_blocks = (last_key_of(p, last_row + offset) + kBlockKv) / kBlockKv;
+    // Under the causal masks the first tile's queries see nothing of the last blocks the second walks.
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) {
+      const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
+      blocks[i] = q0 + i * kBlockQ >= p.q_len ? 0 : min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv);
+    }
+  }
+};
+
+// Asks for a CTA of this grid that has not started: sixteen bytes of answer, counted on `bar`.
+__device__ __forceinline__ void claim_next_cta(uint4 *answer, uint64_t *bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// The block indices of the CTA that was taken over, w = 1; w = 0 where none was left.
+__device__ __forceinline__ int4 claimed_cta(const uint4 *answer) {
+  int4 c;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 r;\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b32 x, y, z, u;\n\t"
+      "ld.shared.b128 r, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.b32 %3, 1, 0, p;\n\t"
+      "mov.b32 x, 0;\n\t"
+      "mov.b32 y, 0;\n\t"
+      "mov.b32 z, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {x, y, z, u}, r;\n\t"
+      "mov.b32 %0, x;\n\t"
+      "mov.b32 %1, y;\n\t"
+      "mov.b32 %2, z;\n\t"
+      "}"
+      : "=r"(c.x), "=r"(c.y), "=r"(c.z), "=r"(c.w)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return c;
+}
 
 template <int D>
 __global__ void __launch_bounds__(kThreads2, 1)
@@ -719,34 +796,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (threadIdx.x == 0) atomicCAS(p.status, 0u, kStatusAttentionLayout);
     return;
   }
-  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its
-  // keys and values in L2. Under the causal masks the later queries have more keys to walk: the last
-  // unit of every head goes first, then the one before it, so that the grid ends on the short ones
-  // whatever the head.
-  int unit = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
-  if (p.mask_type != 0) {
-    const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
-    const int order = unit + units * (head + heads * batch);
-    unit = units - 1 - order / all;
-    head = order % all % heads;
-    batch = order % all / heads;
-  }
-  const int q0 = unit * (kTiles * kBlockQ);
-  const int kv_head = head / p.group;
   const int offset = p.kv_len - p.q_len;
-  // Both tiles start at the first block of keys that some query of the CTA sees.
-  const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
-  const int kv_begin = first_key_of(p, q0 + offset);
-  const int kv_end = last_key_of(p, last_row + offset) + 1;
-  const int block0 = kv_begin / kBlockKv;
-  const int num_blocks = (kv_end + kBlockKv - 1) / kBlockKv - block0;
-  // Under the causal masks the first tile's queries see nothing of the last blocks the second walks;
-  // a tile past the last query has none.
-  auto blocks_of = [&](int i) -> int {
-    if (q0 + i * kBlockQ >= p.q_len) return 0;
-    const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
-    return min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv - block0);
-  };
 
   if (threadIdx.x == 0) {
     t.abort_flag = 0;
@@ -754,8 +804,14 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       mbar_init(&t.slot_full_bar[i], 1);
       mbar_init(&t.slot_empty_bar[i], 1);
     }
+    mbar_init(&t.claim_bar, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&t.unit_full_bar[i], 1);
+      mbar_init(&t.unit_empty_bar[i], kSoftmaxWarps2 + 1);
+    }
     for (int i = 0; i < kTiles; ++i) {
       mbar_init(&t.q_full_bar[i], 1);
+      mbar_init(&t.q_empty_bar[i], 1);
       mbar_init(&t.s_full_bar[i], 1);
       for (int h = 0; h < kPParts; ++h) mbar_init(&t.p_full_bar[i][h], kTileWarps);
       mbar_init(&t.pv_done_bar[i], 1);
@@ -775,159 +831,179 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = t.tmem_base_slot;
+  griddep_wait();
+  griddep_launch_dependents();
 
   auto q_tile = [&](int i) { return smem + L::kQOff + i * L::kQBytes; };
   auto slot = [&](int i) { return smem + L::kSlotOff + i * L::kSlotBytes; };
+  // Unit number `count` of this CTA (from 1 on), once the producer has put it there; w = 0: none left.
+  auto read_next_unit = [&](int count, int4 *c) -> bool {
+    if (!mbar_wait(&t.unit_full_bar[count & 1], ((count - 1) >> 1) & 1, &abort_flag)) return false;
+    *c = t.next_unit[count & 1];
+    return true;
+  };
 
-  // Load n of the ring (K of block n / 2 when n is even, V of it when odd) goes to slot n % S.
+  // Load n of the ring, counted over all of the CTA's units (K of a block, V of it, K of the next), goes
+  // to slot n % S.
   if (warp < kSoftmaxWarps2) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
     // ------------------------------------------------------------------ softmax and output
     const int tile = static_cast<int>(warp >> 2);
     const uint32_t quarter = warp & 3;
-    const int tq0 = q0 + tile * kBlockQ;  // the tile's first query
     const int row = static_cast<int>(quarter) * 32 + static_cast<int>(lane);
-    const int q_pos = tq0 + row + offset;
-    const int key_first = first_key_of(p, q_pos), key_last = last_key_of(p, q_pos);
-    const int tile_last_row = min(tq0 + kBlockQ, p.q_len) - 1;
-    // What every query of the tile sees (an empty range for a tile past the last query: every block
-    // is then an edge block, and nothing of it is stored).
-    const int common_first = first_key_of(p, tile_last_row + offset), common_last = last_key_of(p, tq0 + offset);
     const uint32_t t_lane = tmem_base + ((quarter * 32u) << 16);
     const uint32_t t_scores = t_lane + tile * L::kSCols;  // the row's 128 scores, then its 128 probabilities in 64 columns
     const uint32_t t_out = t_lane + L::kOCol + tile * D;
     constexpr int kChunks = kBlockKv / 32;
     static_assert(kChunks == 4, "four chunks of scores pack into the first two");
     constexpr float kRescaleStep = 8.0f;
-    float m_used = -INFINITY;
-    float l_run = 0.0f;
     bool ok = true;
     uint32_t sc[kChunks][32];
+    uint32_t s_phase = 0, pv_phase = 0;  // of the tile's scores and of its finished outputs
+    int4 at = make_int4(blockIdx.x, blockIdx.y, blockIdx.z, 1);
 
-    const int my_blocks = blocks_of(tile);
-    for (int j = 0; j < my_blocks && ok; ++j) {
-      // The row's scores of the block into registers in one round trip. (Scores of block j are
-      // issued behind the product of block j - 1: once they are here the tile's output is complete
-      // up to that block.)
-      ok = __all_sync(0xffffffffu, mbar_wait(&t.s_full_bar[tile], j & 1, &abort_flag));
-      if (!ok) break;
-      tc_fence_after_sync();
+#pragma unroll 1
+    for (int count = 1; ok && at.w != 0; ++count) {
+      const Unit2 u(p, at.x, at.y, at.z);
+      const int tq0 = u.q0 + tile * kBlockQ;  // the tile's first query
+      const int key_last = last_key_of(p, tq0 + row + offset);
+      const int common_last = last_key_of(p, tq0 + offset);  // what every query of the tile sees
+      float m_used = -INFINITY;
+      float l_run = 0.0f;
+      const int my_blocks = tile == 0 ? u.blocks[0] : u.blocks[1];
+      for (int j = 0; j < my_blocks && ok; ++j) {
+        // The row's scores of the block into registers in one round trip. (Scores of block j are
+        // issued behind the product of block j - 1: once they are here the tile's output is complete
+        // up to that block.)
+        ok = __all_sync(0xffffffffu, mbar_wait(&t.s_full_bar[tile], s_phase, &abort_flag));
+        if (!ok) break;
+        s_phase ^= 1;
+        tc_fence_after_sync();
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
+        for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
-      const int block_key0 = (block0 + j) * kBlockKv;
-      const bool edge = block_key0 < common_first || block_key0 + kBlockKv - 1 > common_last;
-      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (edge) {
+        for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
+        const int block_key0 = j * kBlockKv;
+        const bool edge = block_key0 + kBlockKv - 1 > common_last;
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (edge) {
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (block_key0 + c * 32 + i > key_last) sc[c][i] = __float_as_uint(-INFINITY);
+            }
+          }
+        }
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = block_key0 + c * 32 + i;
-            if (key > key_last || key < key_first) sc[c][i] = __float_as_uint(-INFINITY);
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
-        }
-      }
-      const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
-      if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
-        const float m_new = fmaxf(m_used, m_blk);
-        const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
-        l_run *= alpha;
-        if (j > 0) {
-#pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
-            uint32_t v[16];
-            tmem_ld_32x16(t_out + c * 16, v);
-            tmem_ld_wait(v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x16(t_out + c * 16, v);
-          }
-        }
-        m_used = m_new;
-      }
-      const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
-      // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
-      // (a slot whose scores have been used by then).
-      const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
-      uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
-      auto emit = [&](auto bf16_tag, int part) {
-        constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
-#pragma unroll
-        for (int h = 0; h < kChunks / kPParts; ++h) {
-          const int c = part * (kChunks / kPParts) + h;
-#pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
-            float e0, e1;
-            if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
-              float x0, x1;
-              f2_unpack(x, &x0, &x1);
-              e0 = fast_exp2(x0);
-              e1 = fast_exp2(x1);
-            } else {
-              exp2_pair_poly(x, &e0, &e1);
-            }
-            sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
-            sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
+            m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
           }
         }
-      };
-      // Each half of the block's keys is handed over as soon as it is there: its product runs under
-      // the exponentials of the other half.
-#pragma unroll
-      for (int part = 0; part < kPParts; ++part) {
-        if (p.is_bf16) {
-          emit(std::true_type{}, part);
-        } else {
-          emit(std::false_type{}, part);
-        }
-        tmem_st_32x32(t_scores + part * 32, sc[part]);
-        if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
-        tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
-        tc_fence_before_sync();  // before the MMAs that the hand-over starts
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
-      }
-      float s0, s1, s2, s3;
-      f2_unpack(sums[0], &s0, &s1);
-      f2_unpack(sums[1], &s2, &s3);
-      l_run += (s0 + s1) + (s2 + s3);
-    }
-    // The last product.
-    if (ok && my_blocks > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&t.pv_done_bar[tile], 0, &abort_flag));
-      tc_fence_after_sync();
-    }
-    if (ok) {
-      const bool live = tq0 + row < p.q_len;
-      const float inv = 1.0f / l_run;
-      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + batch * p.out_stride[0] + head * p.out_stride[1] +
-                      static_cast<int64_t>(tq0 + row) * p.out_stride[2];
+        const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+        if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
+          const float m_new = fmaxf(m_used, m_blk);
+          const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
+          l_run *= alpha;
+          if (j > 0) {
 #pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32(t_out + c * 32, v);
-        tmem_ld_wait(v);
-        if (live) {
+            for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
+              uint32_t v[16];
+              tmem_ld_32x16(t_out + c * 16, v);
+              tmem_ld_wait(v);
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 w;
-            w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
-            w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
-            w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
-            w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
-            *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
+              for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+              tmem_st_32x16(t_out + c * 16, v);
+            }
+          }
+          m_used = m_new;
+        }
+        const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
+        // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
+        // (a slot whose scores have been used by then).
+        const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
+        uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
+        auto emit = [&](auto bf16_tag, int part) {
+          constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
+#pragma unroll
+          for (int h = 0; h < kChunks / kPParts; ++h) {
+            const int c = part * (kChunks / kPParts) + h;
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
+              float e0, e1;
+              if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
+                float x0, x1;
+                f2_unpack(x, &x0, &x1);
+                e0 = fast_exp2(x0);
+                e1 = fast_exp2(x1);
+              } else {
+                exp2_pair_poly(x, &e0, &e1);
+              }
+              sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
+              sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
+            }
+          }
+        };
+        // Each half of the block's keys is handed over as soon as it is there: its product runs under
+        // the exponentials of the other half.
+#pragma unroll
+        for (int part = 0; part < kPParts; ++part) {
+          if (p.is_bf16) {
+            emit(std::true_type{}, part);
+          } else {
+            emit(std::false_type{}, part);
+          }
+          tmem_st_32x32(t_scores + part * 32, sc[part]);
+          if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
+          tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
+          tc_fence_before_sync();  // before the MMAs that the hand-over starts
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
+        }
+        float s0, s1, s2, s3;
+        f2_unpack(sums[0], &s0, &s1);
+        f2_unpack(sums[1], &s2, &s3);
+        l_run += (s0 + s1) + (s2 + s3);
+      }
+      // The last product.
+      if (ok && my_blocks > 0) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&t.pv_done_bar[tile], pv_phase, &abort_flag));
+        pv_phase ^= 1;
+        tc_fence_after_sync();
+      }
+      if (ok && my_blocks > 0) {
+        const bool live = tq0 + row < p.q_len;
+        const float inv = 1.0f / l_run;
+        uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + u.batch * p.out_stride[0] + u.head * p.out_stride[1] +
+                        static_cast<int64_t>(tq0 + row) * p.out_stride[2];
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32(t_out + c * 32, v);
+          tmem_ld_wait(v);
+          if (live) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              uint4 w;
+              w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
+              w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
+              w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
+              w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
+              *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
+            }
           }
         }
+        // The next unit's first product overwrites this output: it waits for probabilities that the tile's
+        // four warps hand over only after these reads.
+        tc_fence_before_sync();
+      }
+      if (ok) {
+        ok = __all_sync(0xffffffffu, read_next_unit(count, &at));
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(&t.unit_empty_bar[count & 1]);
       }
     }
     if (!ok && lane == 0) {
@@ -940,41 +1016,76 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       // ------------------------------------------------------------------ producer
       if (elect_one()) {
         bool ok = true;
-        auto load = [&](void *dst, const CUtensorMap *map, uint64_t *bar, int32_t c0, int32_t c1, int32_t c2) {
-          tma_load_4d(dst, map, bar, c0, c1, c2, batch);
-        };
-        for (int i = 0; i < kTiles; ++i) {
-          mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
+        int n = 0;  // loads of the ring so far
+        uint32_t q_phase[kTiles] = {0, 0};
+        int4 at = make_int4(blockIdx.x, blockIdx.y, blockIdx.z, 1);
+        for (int count = 1; ok && at.w != 0; ++count) {
+          const Unit2 u(p, at.x, at.y, at.z);
+          const int kv_head = u.head / p.group;
+          auto load = [&](void *dst, const CUtensorMap *map, uint64_t *bar, int32_t c0, int32_t c1, int32_t c2) {
+            tma_load_4d(dst, map, bar, c0, c1, c2, u.batch);
+          };
+          for (int i = 0; i < 2 * u.num_blocks && ok; ++i, ++n) {
+            const int st = n % S, key0 = (i >> 1) * kBlockKv;
+            if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
+            if ((i & 1) == 0) {
 #pragma unroll
-          for (int a = 0; a < L::kQAtoms; ++a) {
-            load(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, q0 + i * kBlockQ, head);
+              for (int a = 0; a < L::kQAtoms; ++a) {
+                load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+              }
+            } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
+#pragma unroll
+              for (int a = 0; a < L::kQAtoms; ++a) {
+                load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+              }
+            } else {
+#pragma unroll
+              for (int a = 0; a < L::kVAtoms; ++a) {
+                tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st], (key0 + a * kAtomElems) * 2, 0,
+                            u.batch * p.kv_heads + kv_head);
+              }
+            }
+            // The queries behind the first block of keys, once the last scores of the unit before have been
+            // computed.
+            for (int q = 0; i == 0 && q < kTiles && ok; ++q) {
+              if (u.blocks[q] == 0) continue;
+              if (!mbar_wait(&t.q_empty_bar[q], q_phase[q] ^ 1, &abort_flag)) {
+                ok = false;
+                break;
+              }
+              q_phase[q] ^= 1;
+              mbar_arrive_expect_tx(&t.q_full_bar[q], L::kQBytes);
+#pragma unroll
+              for (int a = 0; a < L::kQAtoms; ++a) {
+                load(q_tile(q) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[q], a * kAtomBytes, u.q0 + q * kBlockQ, u.head);
+              }
+            }
           }
-        }
-        for (int n = 0; n < 2 * num_blocks && ok; ++n) {
-          const int st = n % S, j = n >> 1;
-          if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
+          if (!ok) break;
+          // The next unit is claimed once the last block of this one is on its way: as late as its own
+          // loads allow, so that the CTA that is ahead takes it.
+          if (p.take_over) {
+            mbar_arrive_expect_tx(&t.claim_bar, sizeof(t.claim));
+            claim_next_cta(&t.claim, &t.claim_bar);
+            if (!mbar_wait(&t.claim_bar, (count - 1) & 1, &abort_flag)) {
+              ok = false;
+              break;
+            }
+            at = claimed_cta(&t.claim);
+            fence_proxy_async_smem();  // the answer has been read before the next one overwrites it
+          } else {
+            at.w = 0;
+          }
+          if (!mbar_wait(&t.unit_empty_bar[count & 1], (((count - 1) >> 1) & 1) ^ 1, &abort_flag)) {
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
-          const int key0 = (block0 + j) * kBlockKv;
-          if ((n & 1) == 0) {
-#pragma unroll
-            for (int a = 0; a < L::kQAtoms; ++a) {
-              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
-            }
-          } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
-#pragma unroll
-            for (int a = 0; a < L::kQAtoms; ++a) {
-              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
-            }
-          } else {
-#pragma unroll
-            for (int a = 0; a < L::kVAtoms; ++a) {
-              tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st], (key0 + a * kAtomElems) * 2, 0,
-                          batch * p.kv_heads + kv_head);
-            }
-          }
+          t.next_unit[count & 1] = at;
+          mbar_arrive(&t.unit_full_bar[count & 1]);
         }
         if (!ok) {
           abort_flag = 1;
@@ -1042,51 +1153,97 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         };
         auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
         auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
-        const int blocks[kTiles] = {blocks_of(0), blocks_of(1)};
-        for (int i = 0; i < kTiles && ok; ++i) ok = mbar_wait(&t.q_full_bar[i], 0, &abort_flag);
-        if (ok && num_blocks > 0) ok = wait_full(0);
-        if (ok && num_blocks > 0) {
-          tc_fence_after_sync();
-#pragma unroll
-          for (int i = 0; i < kTiles; ++i) {
-            if (blocks[i] == 0) continue;
-            scores(i, desc_of(0));
-            commit(&t.s_full_bar[i]);
-          }
-          commit(&t.slot_empty_bar[0]);
+        int n = 0;  // the ring's load that holds K of the current unit's first block
+        uint32_t q_phase[kTiles] = {0, 0}, p_phase[kTiles] = {0, 0};
+        int cur[kTiles], num_blocks;
+        {
+          const Unit2 u(p, blockIdx.x, blockIdx.y, blockIdx.z);
+          cur[0] = u.blocks[0], cur[1] = u.blocks[1], num_blocks = u.num_blocks;
         }
-        for (int j = 0; j < num_blocks && ok; ++j) {
-          const bool more = j + 1 < num_blocks;
-          const int nv = 2 * j + 1, nk = 2 * j + 2;
-          if (!wait_full(nv)) ok = false;
+        // Tile i's scores with the keys in load nk; `last`: of its unit, so that its queries may be replaced.
+        auto issue_scores = [&](int i, int nk, bool last) {
+          tc_fence_after_sync();
+          scores(i, desc_of(nk));
+          commit(&t.s_full_bar[i]);
+          if (last) commit(&t.q_empty_bar[i]);
+        };
+        auto wait_queries = [&](int i) -> bool {
+          const bool there = mbar_wait(&t.q_full_bar[i], q_phase[i], &abort_flag);
+          q_phase[i] ^= 1;
+          return there;
+        };
+        bool started[kTiles] = {false, false};  // the tile's first scores of the unit are under way
+        for (int count = 1; ok && num_blocks > 0; ++count) {
 #pragma unroll
           for (int i = 0; i < kTiles; ++i) {
-            if (!ok || j >= blocks[i]) continue;
-            // The product reads P from the columns the next scores overwrite: the instructions of one
-            // thread run in the order they were issued.
+            if (!ok || started[i] || cur[i] == 0) continue;
+            ok = wait_queries(i) && wait_full(n);
+            if (ok) issue_scores(i, n, cur[i] == 1);
+          }
+          if (!ok) break;
+          commit(&t.slot_empty_bar[n % S]);
+          started[0] = started[1] = false;
+          int nxt[kTiles] = {0, 0}, next_blocks = 0;
+          bool known = false;
+          for (int j = 0; j < num_blocks && ok; ++j) {
+            const bool more = j + 1 < num_blocks;
+            const int nv = n + 2 * j + 1, nk = nv + 1;  // (nk: of this unit's next block or the next unit's first)
+            if (!wait_full(nv)) ok = false;
 #pragma unroll
-            for (int part = 0; part < kPParts; ++part) {
-              if (ok) ok = mbar_wait(&t.p_full_bar[i][part], j & 1, &abort_flag);
-              if (!ok) break;
-              tc_fence_after_sync();
-              product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
-            }
-            if (!ok) continue;
-            if (j + 1 == blocks[i]) {
-              commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
-            } else {
+            for (int i = 0; i < kTiles; ++i) {
+              if (!ok || j >= cur[i]) continue;
+              // The product reads P from the columns the next scores overwrite: the instructions of one
+              // thread run in the order they were issued.
+#pragma unroll
+              for (int part = 0; part < kPParts; ++part) {
+                if (ok) ok = mbar_wait(&t.p_full_bar[i][part], p_phase[i], &abort_flag);
+                if (!ok) break;
+                tc_fence_after_sync();
+                product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
+              }
+              if (!ok) continue;
+              p_phase[i] ^= 1;
+              bool last = j + 2 == cur[i];
+              if (j + 1 == cur[i]) {
+                commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
+                if (more) continue;
+                // Through with the unit: on with the first scores of the next one, which run under the
+                // other tile's last product and this one's output.
+                if (!known) {
+                  known = true;
+                  int4 c;
+                  if (!read_next_unit(count, &c)) {
+                    ok = false;
+                    continue;
+                  }
+                  __syncwarp();
+                  if (issuer) mbar_arrive(&t.unit_empty_bar[count & 1]);
+                  if (c.w != 0) {
+                    const Unit2 u(p, c.x, c.y, c.z);
+                    nxt[0] = u.blocks[0], nxt[1] = u.blocks[1], next_blocks = u.num_blocks;
+                  }
+                }
+                if (nxt[i] == 0) continue;
+                if (!wait_queries(i)) {
+                  ok = false;
+                  continue;
+                }
+                started[i] = true;
+                last = nxt[i] == 1;
+              }
               if (!wait_full(nk)) {  // (seen by the first tile's turn, for the second's too)
                 ok = false;
                 continue;
               }
-              tc_fence_after_sync();
-              scores(i, desc_of(nk));
-              commit(&t.s_full_bar[i]);
+              issue_scores(i, nk, last);
             }
+            if (!ok) break;
+            commit(&t.slot_empty_bar[nv % S]);  // both tiles have read the two slots
+            if (more) commit(&t.slot_empty_bar[nk % S]);
           }
-          if (!ok) break;
-          commit(&t.slot_empty_bar[nv % S]);  // both tiles have read the two slots
-          if (more) commit(&t.slot_empty_bar[nk % S]);
+          n += 2 * num_blocks;
+          num_blocks = next_blocks;
+          cur[0] = nxt[0], cur[1] = nxt[1];
         }
         if (!ok && issuer) {
           abort_flag = 1;
@@ -1183,8 +1340,18 @@ cudaError_t launch2(const AttentionArgs &a, const CUtensorMap &tq, const CUtenso
   const int per_cta = kTiles * kBlockQ;
   const dim3 grid(static_cast<unsigned>((a.q_len + per_cta - 1) / per_cta), static_cast<unsigned>(a.heads),
                   static_cast<unsigned>(a.batch));
-  kernel<<<grid, kThreads2, L::kSmemBytes, a.stream>>>(tq, tk, tvt, kp);
-  return cudaGetLastError();
+  // (barriers, tensor memory and the descriptors' way in may run under the end of the kernel before)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads2, 1, 1);
+  cfg.dynamicSmemBytes = L::kSmemBytes;
+  cfg.stream = a.stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, tq, tk, tvt, kp);
 }
 
 }  // namespace
@@ -1280,6 +1447,10 @@ cudaError_t attention(const AttentionArgs &a, const char **why) {
   kp.status = a.status;
   const AttentionPlan plan = attention_plan(a);
   const bool two_tiles = plan.two_tiles;
+  // Walks of a few blocks are worth going on from one to the next; on long ones, which the power limit
+  // paces, it measured slower (4 x 32 x 1000 causal, eight blocks at most: 63.4 -> 57.4 us; 2 x 24 x 4352
+  // without a mask, 34 blocks: 450 -> 469).
+  kp.take_over = (a.kv_len + kBlockKv - 1) / kBlockKv <= kTakeOverBlocks ? 1 : 0;
   kp.v_direct = plan.v_direct ? 1 : 0;
 
   if (!kp.v_direct) {

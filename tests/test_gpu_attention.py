@@ -201,3 +201,28 @@ def test_block_masks(flint, oracle, mask, block, n, h, hk, L, S, d, is_bf16):
         assert np.array_equal(got, run(flint, q, k, v, 1, is_bf16))      # the causal mask, bit for bit
     if block >= S and mask == 3:
         assert np.array_equal(got, run(flint, q, k, v, 0, is_bf16))      # no mask, bit for bit
+
+
+@pytest.mark.parametrize("n,h,hk,L,S,d", [
+    (4, 40, 10, 300, 300, 128),  # 320 units, of which every other has a tile without a query
+    (2, 90, 90, 130, 131, 64),   # two blocks of keys a unit, the second with three
+    (1, 200, 100, 257, 260, 64),
+    (1, 150, 2, 600, 700, 128),  # three lengths of unit under the causal mask, the longest first
+    (3, 52, 52, 129, 129, 128),  # the causal first tiles see one block of the two
+    (1, 160, 8, 140, 2049, 64),  # a walk too long to be followed by another
+])
+@pytest.mark.parametrize("causal", [False, True])
+def test_more_units_than_the_gpu_holds(flint, oracle, n, h, hk, L, S, d, causal):
+    """A CTA goes on with units whose own CTA never starts: queries, rings, phases and the output's
+    tensor memory pass from one unit to the next, with lengths that change on the way."""
+    rng = np.random.default_rng(L + S + h)
+    q, k, v = make(oracle, rng, n, h, hk, L, S, d, True)
+    got = run(flint, q, k, v, causal, True)
+    check(oracle, got, oracle.attention(q, k, v, causal, True), True, f"{(n, h, hk, L, S, d)} causal={causal}")
+
+
+def test_more_units_than_the_gpu_holds_with_one_block_each(flint, oracle):
+    rng = np.random.default_rng(5)
+    q, k, v = make(oracle, rng, 2, 96, 96, 200, 77, 64, False)
+    got = run(flint, q, k, v, False, False)
+    check(oracle, got, oracle.attention(q, k, v, False, False), False, "one block")
