@@ -8,10 +8,10 @@
 //   warp  8    producer: TMA tile loads of A and B (and the NVFP4 scale-factor tiles) into a
 //              ring of shared-memory stages, signalled through mbarriers
 //   warp  9    MMA: one thread issues tcgen05.mma on the staged tiles, accumulating in tensor
-//              memory; tcgen05.commit hands stages back to the producer and finished
-//              accumulators to the epilogue
-//   warps 10-11 in the NVFP4 kind one thread of them copies scale factors into tensor memory; in
-//              the scatter form (a product gathered on several GPUs) the epilogue's TMA stores go
+//              memory (in the NVFP4 kind it copies a stage's scale factors there first);
+//              tcgen05.commit hands stages back to the producer and finished accumulators to the
+//              epilogue
+//   warps 10-11 in the scatter form (a product gathered on several GPUs) the epilogue's TMA stores go
 //              to every destination matrix, this GPU's and its peers', and these warps are idle;
 //              only where a destination cannot be described by a tensor map do they push: once the
 //              epilogue has written a tile into this GPU's matrix they copy its rows to the peers'
@@ -84,7 +84,7 @@ struct Roles {
   static constexpr int kColumnShares = kEpilogueWarps / 4;
   static constexpr int kProducerWarp = kEpilogueWarps;
   static constexpr int kMmaWarp = kEpilogueWarps + 1;
-  static constexpr int kAuxWarp0 = kEpilogueWarps + 2;       // pushers / scale-factor copier, or converters
+  static constexpr int kAuxWarp0 = kEpilogueWarps + 2;       // pushers, or converters
   static constexpr int kAuxWarps = kNumWarps - kAuxWarp0;    // 2, or 6
 };
 // Tiles are walked in bands of tile columns, columns fastest inside a band, so that the tiles in
@@ -244,11 +244,10 @@ struct Config : Roles<B8> {
   static constexpr int kColParamOffset = kOutStageOffset + kOutStageBytes;
   static constexpr int kSmemBytes = kColParamOffset + kColParamBytes + 1024;  // + slack to align to 1024
   static_assert(kStageBytes % 512 == 0, "the output staging behind the stages has to stay 512-byte aligned");
-  // Tensor memory columns: two accumulators, then three sets of one stage's scale factors. The
-  // copies into a set are issued by a thread of their own, ahead of the MMAs that read the
-  // others: issued by the MMA thread itself they execute in order with its MMAs, and cost as
-  // much as those. Two sets left one stage's MMAs to hide the way commit -> wait -> ten copies ->
-  // commit -> wait; three leave two.
+  // Tensor memory columns: two accumulators, then three sets of one stage's scale factors, which the
+  // MMA thread copies there ahead of the stage's MMAs: both run in the order of their issue, so nothing
+  // is handed over (a copying thread of its own, with a commit and a wait in both directions for every
+  // set, took 82.4 us for the whole of 4352 x 9216 x 3072, this 78.6).
   static constexpr int kAccCols = 2 * BLOCK_N;
   static constexpr int kSfaCols = NVF4 ? kMmasPerStage * 4 : 0;
   static constexpr int kSfbColsPerMma = NVF4 ? BLOCK_N / 32 : 0;
@@ -315,8 +314,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   __shared__ __align__(8) uint64_t acc_full_bar[2];
   __shared__ __align__(8) uint64_t acc_empty_bar[2];
   __shared__ __align__(8) uint64_t tile_done_bar[2];  // epilogue -> pushers: the tile is in this GPU's matrix
-  __shared__ __align__(8) uint64_t sf_full_bar[kSfSets];   // NVFP4: a set of scale factors is in tensor memory
-  __shared__ __align__(8) uint64_t sf_empty_bar[kSfSets];  // NVFP4: the MMAs that read the set are done
   __shared__ __align__(8) uint64_t raw_full_bar[B8 ? STAGES : 1];  // mixed form: a stage's e4m3 weight bytes have landed
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile uint32_t abort_flag;
@@ -343,10 +340,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // the accumulator too, which keeps the epilogue from running two tiles ahead of them.
       mbar_init(&acc_empty_bar[s], (kEpilogueWarps + (scatter ? kPusherWarps : 0)) * CTAS);
       mbar_init(&tile_done_bar[s], kEpilogueWarps);
-    }
-    for (int s = 0; s < kSfSets; ++s) {
-      mbar_init(&sf_full_bar[s], 1);
-      mbar_init(&sf_empty_bar[s], 1);
     }
     fence_barrier_init();
   }
@@ -479,7 +472,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       (void)sfa_desc0;
       (void)sfb_desc0;
       (void)kSfTileStep;
-      uint32_t sf_set = 0, sf_phase = 0;  // NVFP4: the next stage's set of scale factors, over all tiles
+      uint32_t sf_set = 0;  // NVFP4: the next stage's set of scale factors, over all tiles
+      (void)sf_set;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -507,11 +501,21 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           if constexpr (NVF4) {
             const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols + sf_set * Cfg::kSfSetCols;
             const uint32_t sfb_tmem = sfa_tmem + Cfg::kSfaCols;
-            if (!mbar_wait(&sf_full_bar[sf_set], sf_phase, &abort_flag)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
+            // Copies and multiplications issued by one thread run in the order they were issued.
+            const uint64_t sfa_desc = sfa_desc0 + stage * kStageStep;
+            const uint64_t sfb_desc = sfb_desc0 + stage * kStageStep;
+            auto copy = [&](uint32_t taddr, uint64_t desc) {
+              if (!issuer) return;
+              if constexpr (CTAS == 2) {
+                tmem_cp_sf_pair(taddr, desc);
+              } else {
+                tmem_cp_sf(taddr, desc);
+              }
+            };
+#pragma unroll
+            for (int j = 0; j < kMmasPerStage; ++j) copy(sfa_tmem + j * 4, sfa_desc + j * kSfTileStep);
+#pragma unroll
+            for (int j = 0; j < Cfg::kSfbCopies; ++j) copy(sfb_tmem + j * 4, sfb_desc + j * kSfTileStep);
 #pragma unroll
             for (int j = 0; j < kMmasPerStage; ++j) {
               if constexpr (CTAS == 2) {
@@ -533,13 +537,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
           }
           commit_to(&empty_bar[stage]);
-          if constexpr (NVF4) {
-            commit_to(&sf_empty_bar[sf_set]);
-            if (++sf_set == kSfSets) {
-              sf_set = 0;
-              sf_phase ^= 1;
-            }
-          }
+          if (NVF4 && ++sf_set == kSfSets) sf_set = 0;
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -549,64 +547,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         commit_to(&acc_full_bar[acc]);
       }
       if (!ok && issuer) {
-        abort_flag = 1;
-        atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusMmaTimeout));
-      }
-    }
-  } else if (NVF4 && warp == kPusherWarp0) {
-    // ------------------------------------------------------------------ scale-factor copier (NVFP4)
-    // One thread of the leader moves every stage's scale factors shared -> tensor memory, into
-    // the set the MMAs are not reading, and hands the set over with a commit.
-    if (leader && elect_one()) {
-      constexpr uint64_t kStageStep = Cfg::kStageBytes >> 4;
-      constexpr uint64_t kSfTileStep = kSfTileBytes >> 4;
-      const uint64_t sfa_desc0 = umma_desc_sf(smem_u32(stage_sfa(0)));
-      const uint64_t sfb_desc0 = umma_desc_sf(smem_u32(stage_sfb(0)));
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t set = 0, set_phase = 0;
-      bool ok = true;
-      WorkWalk walk(p, unit, num_units);
-      WorkItem item;
-      while (ok && walk.next(&item)) {
-        for (int kb = item.kb0; kb < item.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, &abort_flag) ||
-              !mbar_wait(&sf_empty_bar[set], set_phase ^ 1, &abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint64_t sfa_desc = sfa_desc0 + stage * kStageStep;
-          const uint64_t sfb_desc = sfb_desc0 + stage * kStageStep;
-          const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols + set * Cfg::kSfSetCols;
-          const uint32_t sfb_tmem = sfa_tmem + Cfg::kSfaCols;
-          auto copy = [&](uint32_t taddr, uint64_t desc) {
-            if constexpr (CTAS == 2) {
-              tmem_cp_sf_pair(taddr, desc);
-            } else {
-              tmem_cp_sf(taddr, desc);
-            }
-          };
-#pragma unroll
-          for (int j = 0; j < kMmasPerStage; ++j) copy(sfa_tmem + j * 4, sfa_desc + j * kSfTileStep);
-#pragma unroll
-          for (int j = 0; j < Cfg::kSfbCopies; ++j) copy(sfb_tmem + j * 4, sfb_desc + j * kSfTileStep);
-          if constexpr (CTAS == 2) {
-            umma_commit_pair_both(&sf_full_bar[set]);
-          } else {
-            umma_commit(&sf_full_bar[set]);
-          }
-          if (++set == kSfSets) {
-            set = 0;
-            set_phase ^= 1;
-          }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-      }
-      if (!ok) {
         abort_flag = 1;
         atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusMmaTimeout));
       }
