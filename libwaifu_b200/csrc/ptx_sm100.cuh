@@ -279,6 +279,11 @@ __device__ __forceinline__ void bulk_load_1d(void *smem_dst, const void *gmem_sr
       : "memory");
 }
 
+// Asks for the same run of bytes to be brought into L2; nothing waits for it.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *gmem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes) : "memory");
+}
+
 // ---- tcgen05: tensor memory --------------------------------------------------------------
 
 // Whole-warp instructions. `ncols` a power of two in [32, 512]. With CTAS == 2 the same warp of

@@ -251,6 +251,25 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_fp8_kernel(const SkinnyPar
     }
     fence_barrier_init();
   }
+  // The weight of the CTA's first stages into L2 while the kernel ahead in the stream may still run: a
+  // prefetch writes nothing, and the copies below read what they would have read anyway (one row against
+  // 3072 x 3072 from HBM: 6.43 -> 6.36 us).
+  if (warp == kConsumerWarps) {
+    int ahead = 0;
+    for (int u = blockIdx.x; u < p.units && ahead < p.stages; u += gridDim.x) {
+      const int row0 = u * unit_rows;
+      const int rows = min(unit_rows, p.n - row0);
+      for (int kc = 0; kc < p.k_chunks && ahead < p.stages; ++kc, ++ahead) {
+        const int k0 = kc * chunk_bytes;
+        const uint32_t bytes = static_cast<uint32_t>(min(chunk_bytes, p.kb - k0));
+        if (p.one_copy) {
+          if (lane == 0) bulk_prefetch_l2(p.w + static_cast<long long>(row0) * p.kb, bytes * rows);
+        } else {
+          for (int r = lane; r < rows; r += 32) bulk_prefetch_l2(p.w + static_cast<long long>(row0 + r) * p.kb + k0, bytes);
+        }
+      }
+    }
+  }
   __syncthreads();
   griddep_wait();
   griddep_launch_dependents();
