@@ -275,6 +275,59 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi, int is_bf16) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
+// Two floats in one 64-bit register, and the two-wide float instructions of sm_100: each half is rounded as
+// the scalar instruction rounds it, at half the issue slots: the epilogue, and not the main loop under it, is
+// what a tile of a short K waits for (4352 x 12288 x 3072 with bias and GELU 141 -> 134 us, 4096 x 3072 x 3072
+// with bias 36.4 -> 34.9, quantised rows; the same bits).
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float *lo, float *hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// gelu_tanh of both halves, the same operations in the same order.
+__device__ __forceinline__ uint64_t f2_gelu_tanh(uint64_t x) {
+  constexpr float kC0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
+  constexpr float kC1 = kC0 * 0.044715f;
+  const uint64_t z = f2_mul(x, f2_fma(f2_mul(x, x), f2_pack(kC1, kC1), f2_pack(kC0, kC0)));
+  float z0, z1, e0, e1, d0, d1, r0, r1;
+  f2_unpack(z, &z0, &z1);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(z0));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(z1));
+  f2_unpack(f2_add(f2_pack(e0, e1), f2_pack(1.0f, 1.0f)), &d0, &d1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
+  return f2_mul(x, f2_pack(r0, r1));
+}
+// A pair of 16-bit values widened.
+__device__ __forceinline__ uint64_t f2_widen(uint32_t w, int is_bf16) {
+  if (is_bf16) return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w));
+  return f2_pack(f.x, f.y);
+}
+__device__ __forceinline__ uint32_t f2_pack16(uint64_t v, int is_bf16) {
+  float lo, hi;
+  f2_unpack(v, &lo, &hi);
+  return pack16(lo, hi, is_bf16);
+}
+
 // Tile index -> (row tile, column tile).
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int *tm, int *tn) {
   const int band_tiles = tiles_n <= kBandMax ? tiles_n : kBandTiles;
@@ -752,7 +805,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // One 32-column chunk: scale, bias, activation, residual in fp32; one rounding; store.
       auto finish_chunk = [&](int c, uint32_t (&v)[32]) {
         const int nc = n0 + c * 32;
-        float x[32];
+        uint64_t x[16];  // pairs of columns
         // Staged form: once the store of the chunk before has read the warp's buffer, the
         // residual's 32 rows x 64 bytes are fetched into it with four coalesced 16-byte copies per
         // lane (8 rows x 64 bytes per instruction) that bypass the registers; the arithmetic below
@@ -774,35 +827,34 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           }
         }
         if (has_cs_vec) {
+          const uint64_t rs2 = f2_pack(rs, rs);
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
-            const float4 s4 = *reinterpret_cast<const float4 *>(cs_t + c * 32 + j);
-            x[j] = __uint_as_float(v[j]) * (rs * s4.x);
-            x[j + 1] = __uint_as_float(v[j + 1]) * (rs * s4.y);
-            x[j + 2] = __uint_as_float(v[j + 2]) * (rs * s4.z);
-            x[j + 3] = __uint_as_float(v[j + 3]) * (rs * s4.w);
+            const ulonglong2 s4 = *reinterpret_cast<const ulonglong2 *>(cs_t + c * 32 + j);
+            x[j / 2] = f2_mul(f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), f2_mul(rs2, s4.x));
+            x[j / 2 + 1] = f2_mul(f2_pack(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), f2_mul(rs2, s4.y));
           }
         } else {
+          const uint64_t rs_cs2 = f2_pack(rs_cs, rs_cs);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]) * rs_cs;
+          for (int j = 0; j < 16; ++j) x[j] = f2_mul(f2_pack(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), rs_cs2);
         }
         if (has_gs) {
+          const uint64_t gs2 = f2_pack(gscale, gscale);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] *= gscale;
+          for (int j = 0; j < 16; ++j) x[j] = f2_mul(x[j], gs2);
         }
         if (has_bias) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 b4 = *reinterpret_cast<const float4 *>(bias_t + c * 32 + j);
-            x[j] += b4.x;
-            x[j + 1] += b4.y;
-            x[j + 2] += b4.z;
-            x[j + 3] += b4.w;
+          for (int j = 0; j < 16; j += 2) {
+            const ulonglong2 b4 = *reinterpret_cast<const ulonglong2 *>(bias_t + c * 32 + 2 * j);
+            x[j] = f2_add(x[j], b4.x);
+            x[j + 1] = f2_add(x[j + 1], b4.y);
           }
         }
         if (p.act == kActGeluTanh) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = gelu_tanh(x[j]);
+          for (int j = 0; j < 16; ++j) x[j] = f2_gelu_tanh(x[j]);
         }
         if (staged) {
           if (has_res) {
@@ -813,22 +865,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               const uint4 q = *reinterpret_cast<const uint4 *>(obuf + own_row_off + ((g ^ own_swz) << 4));
               const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                if (is_bf16) {
-                  x[g * 8 + 2 * h] += __uint_as_float(w[h] << 16);
-                  x[g * 8 + 2 * h + 1] += __uint_as_float(w[h] & 0xffff0000u);
-                } else {
-                  const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[h]));
-                  x[g * 8 + 2 * h] += f.x;
-                  x[g * 8 + 2 * h + 1] += f.y;
-                }
-              }
+              for (int h = 0; h < 4; ++h) x[g * 4 + h] = f2_add(x[g * 4 + h], f2_widen(w[h], is_bf16));
             }
             // (a lane's row is read by that lane only, so it may be overwritten without another barrier)
           }
           uint32_t packed[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) packed[j] = pack16(x[2 * j], x[2 * j + 1], is_bf16);
+          for (int j = 0; j < 16; ++j) packed[j] = f2_pack16(x[j], is_bf16);
           if (p.row_amax != nullptr && row_ok) note_row_amax(packed, nc);
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
@@ -853,28 +896,22 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 const uint4 q = rp[g];
                 const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                  if (is_bf16) {
-                    x[g * 8 + 2 * h] += __uint_as_float(w[h] << 16);
-                    x[g * 8 + 2 * h + 1] += __uint_as_float(w[h] & 0xffff0000u);
-                  } else {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[h]));
-                    x[g * 8 + 2 * h] += f.x;
-                    x[g * 8 + 2 * h + 1] += f.y;
-                  }
-                }
+                for (int h = 0; h < 4; ++h) x[g * 4 + h] = f2_add(x[g * 4 + h], f2_widen(w[h], is_bf16));
               }
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (nc + j < p.n) x[j] += load16(p.residual, res_row + nc + j, is_bf16);
+            for (int j = 0; j < 16; ++j) {  // n is a multiple of 8
+              if (nc + 2 * j < p.n) {
+                x[j] = f2_add(x[j], f2_pack(load16(p.residual, res_row + nc + 2 * j, is_bf16),
+                                            load16(p.residual, res_row + nc + 2 * j + 1, is_bf16)));
+              }
             }
           }
         }
         uint32_t packed[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) packed[j] = pack16(x[2 * j], x[2 * j + 1], is_bf16);
+        for (int j = 0; j < 16; ++j) packed[j] = f2_pack16(x[j], is_bf16);
         if (!row_ok) return;
         if (p.row_amax != nullptr) note_row_amax(packed, nc);
         // (In the scatter form the peers' copies are made by the pusher warps from this one.)
