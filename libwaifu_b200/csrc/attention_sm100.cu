@@ -103,7 +103,6 @@ struct KernelParams {
   int mask_type;   // 0 none, 1 causal, 2 block causal, 3 block diagonal (flint/capi.h:118-133)
   int block_size;
   float scale_log2;
-  int take_over;  // two-tile kernel: CTAs go on with the units of CTAs that have not started
   int v_direct;  // two-tile kernel: v is read as it lies (an MN-major operand), not through its transposition
   uint32_t *status;
 };
@@ -665,10 +664,15 @@ constexpr int kProducerWarp2 = kSoftmaxWarps2;
 constexpr int kMmaWarp2 = kSoftmaxWarps2 + 1;
 // Twelve warps, three warpgroups, launched with 168 registers a thread; the one that loads and issues
 // (two of its warps have nothing to do) gives its own up to the two of the softmax, which hold a
-// row of 128 scores: 128 x 96 + 256 x 200, which is below 384 x 168.
+// row of 128 scores: 128 x 88 + 256 x 208 = 384 x 168 (a CTA that takes units over: 96 and 200).
 constexpr int kThreads2 = (kSoftmaxWarps2 + 4) * 32;
-constexpr int kIssueRegs = 96, kSoftmaxRegs = 200;
-static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2 * 168, "no more than the block was launched with");
+template <bool TAKE_OVER>
+constexpr int kIssueRegs = TAKE_OVER ? 96 : 88;
+template <bool TAKE_OVER>
+constexpr int kSoftmaxRegs = TAKE_OVER ? 200 : 208;
+static_assert(128 * kIssueRegs<true> + kSoftmaxWarps2 * 32 * kSoftmaxRegs<true> <= kThreads2 * 168 &&
+                  128 * kIssueRegs<false> + kSoftmaxWarps2 * 32 * kSoftmaxRegs<false> <= kThreads2 * 168,
+              "no more than the block was launched with");
 // A block's probabilities are handed over in so many parts of its keys. At head_dim 128 the product of
 // the first half runs under the exponentials of the second (2 x 24 x 4352: 396 -> 386 us); at 64,
 // where the products are half as long, one hand-over less is worth more (2 x 8 x 1000 x 2000: 34.6 us
@@ -676,7 +680,11 @@ static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2
 template <int D>
 constexpr int kPartsOf = D == 128 ? 2 : 1;
 constexpr int kMaxSlots = 6;
-constexpr int kTakeOverBlocks = 16;  // the longest walk whose CTA goes on with another unit
+// The longest walks, in blocks of keys, whose CTA goes on with another unit, under the causal masks and
+// without one: 4 x 32 x 1000 causal 63.4 -> 57.4 us, 2 x 24 x 2048 causal at head_dim 64 60 -> 55, 2 x 24 x 300
+// at 64 13.4 -> 12.5, 3 x 24 x 1000 49.6 -> 49.4; but 24 x 2048 73.6 -> 74.5, 2 x 24 x 4352 398 -> 425, causal 347
+// both ways: what a block takes in that form is a little longer, and a long walk has little to hide.
+constexpr int kTakeOverBlocksCausal = 16, kTakeOverBlocks = 8;
 
 struct Tail2 {
   uint4 claim;            // the answer to the last try_cancel
@@ -779,7 +787,8 @@ __device__ __forceinline__ int4 claimed_cta(const uint4 *answer) {
   return c;
 }
 
-template <int D>
+// TAKE_OVER: the CTA goes on with other units; else it leaves after its own.
+template <int D, bool TAKE_OVER>
 __global__ void __launch_bounds__(kThreads2, 1)
 attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
@@ -846,7 +855,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   // Load n of the ring, counted over all of the CTA's units (K of a block, V of it, K of the next), goes
   // to slot n % S.
   if (warp < kSoftmaxWarps2) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs<TAKE_OVER>));
     // ------------------------------------------------------------------ softmax and output
     const int tile = static_cast<int>(warp >> 2);
     const uint32_t quarter = warp & 3;
@@ -1000,6 +1009,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // four warps hand over only after these reads.
         tc_fence_before_sync();
       }
+      if constexpr (!TAKE_OVER) break;
       if (ok) {
         ok = __all_sync(0xffffffffu, read_next_unit(count, &at));
         __syncwarp();
@@ -1011,7 +1021,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       atomicCAS(p.status, 0u, kStatusAttentionTimeout);
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs<TAKE_OVER>));
     if (warp == kProducerWarp2) {
       // ------------------------------------------------------------------ producer
       if (elect_one()) {
@@ -1065,25 +1075,18 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               }
             }
           }
-          if (!ok) break;
+          if (!ok || !TAKE_OVER) break;
           // The next unit is claimed once the last block of this one is on its way: as late as its own
           // loads allow, so that the CTA that is ahead takes it.
-          if (p.take_over) {
-            mbar_arrive_expect_tx(&t.claim_bar, sizeof(t.claim));
-            claim_next_cta(&t.claim, &t.claim_bar);
-            if (!mbar_wait(&t.claim_bar, (count - 1) & 1, &abort_flag)) {
-              ok = false;
-              break;
-            }
-            at = claimed_cta(&t.claim);
-            fence_proxy_async_smem();  // the answer has been read before the next one overwrites it
-          } else {
-            at.w = 0;
-          }
-          if (!mbar_wait(&t.unit_empty_bar[count & 1], (((count - 1) >> 1) & 1) ^ 1, &abort_flag)) {
+          mbar_arrive_expect_tx(&t.claim_bar, sizeof(t.claim));
+          claim_next_cta(&t.claim, &t.claim_bar);
+          if (!mbar_wait(&t.claim_bar, (count - 1) & 1, &abort_flag) ||
+              !mbar_wait(&t.unit_empty_bar[count & 1], (((count - 1) >> 1) & 1) ^ 1, &abort_flag)) {
             ok = false;
             break;
           }
+          at = claimed_cta(&t.claim);
+          fence_proxy_async_smem();  // the answer has been read before the next one overwrites it
           t.next_unit[count & 1] = at;
           mbar_arrive(&t.unit_full_bar[count & 1]);
         }
@@ -1165,7 +1168,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           tc_fence_after_sync();
           scores(i, desc_of(nk));
           commit(&t.s_full_bar[i]);
-          if (last) commit(&t.q_empty_bar[i]);
+          if (TAKE_OVER && last) commit(&t.q_empty_bar[i]);
         };
         auto wait_queries = [&](int i) -> bool {
           const bool there = mbar_wait(&t.q_full_bar[i], q_phase[i], &abort_flag);
@@ -1206,7 +1209,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               bool last = j + 2 == cur[i];
               if (j + 1 == cur[i]) {
                 commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
-                if (more) continue;
+                if (more || !TAKE_OVER) continue;
                 // Through with the unit: on with the first scores of the next one, which run under the
                 // other tile's last product and this one's output.
                 if (!known) {
@@ -1323,11 +1326,11 @@ cudaError_t launch(const AttentionArgs &a, const CUtensorMap &tq, const CUtensor
   return cudaGetLastError();
 }
 
-template <int D>
+template <int D, bool TAKE_OVER>
 cudaError_t launch2(const AttentionArgs &a, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
                     const KernelParams &kp, const char **why) {
   using L = Layout2<D>;
-  auto kernel = attention2_kernel<D>;
+  auto kernel = attention2_kernel<D, TAKE_OVER>;
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
@@ -1447,10 +1450,6 @@ cudaError_t attention(const AttentionArgs &a, const char **why) {
   kp.status = a.status;
   const AttentionPlan plan = attention_plan(a);
   const bool two_tiles = plan.two_tiles;
-  // Walks of a few blocks are worth going on from one to the next; on long ones, which the power limit
-  // paces, it measured slower (4 x 32 x 1000 causal, eight blocks at most: 63.4 -> 57.4 us; 2 x 24 x 4352
-  // without a mask, 34 blocks: 450 -> 469).
-  kp.take_over = (a.kv_len + kBlockKv - 1) / kBlockKv <= kTakeOverBlocks ? 1 : 0;
   kp.v_direct = plan.v_direct ? 1 : 0;
 
   if (!kp.v_direct) {
@@ -1508,7 +1507,11 @@ cudaError_t attention(const AttentionArgs &a, const char **why) {
       return cudaErrorInvalidValue;
     }
   }
-  if (two_tiles) return d == 64 ? launch2<64>(a, tq, tk, tvt, kp, why) : launch2<128>(a, tq, tk, tvt, kp, why);
+  if (two_tiles) {
+    const bool take_over = (a.kv_len + kBlockKv - 1) / kBlockKv <= (kp.mask_type != 0 ? kTakeOverBlocksCausal : kTakeOverBlocks);
+    if (d == 64) return take_over ? launch2<64, true>(a, tq, tk, tvt, kp, why) : launch2<64, false>(a, tq, tk, tvt, kp, why);
+    return take_over ? launch2<128, true>(a, tq, tk, tvt, kp, why) : launch2<128, false>(a, tq, tk, tvt, kp, why);
+  }
   if (d == 64) return launch<64>(a, tq, tk, tvt, kp, why);
   return launch<128>(a, tq, tk, tvt, kp, why);
 }
