@@ -439,6 +439,13 @@ FLAPI int32_t fl_sm100_gemm_plan(int32_t kind, int32_t m, int32_t n, int32_t k, 
 FLAPI int32_t fl_sm100_one_round_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t allow_stream_k,
                                       int32_t *plan);
 
+/* The same kernel's cut of half (kind 0) or bfloat16 rows (1) into tiles of 256 rows, each computed by a
+ * cluster of two CTAs over the whole K: where it has one it is taken, before fl_sm100_one_round_plan's.
+ * plan[8] as there: [0] tile width (0: none, and the rest is 0), [1] 1, [2] CTAs, [3] K stages of a tile,
+ * [4] slots of the load ring, [5] of the ring of widened weight tiles (a CTA holds half of a tile's columns),
+ * [6] bytes of a load slot, [7] dynamic shared memory of a CTA. */
+FLAPI int32_t fl_sm100_one_round_pairs(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t *plan);
+
 /* Storage over device memory the caller already owns (for instance a torch tensor's): nothing
  * is copied and nothing is freed on destroy. The device counterpart of fl_tensor_data_borrow(). */
 FLAPI int32_t fl_tensor_data_borrow_device(void *device_ptr, fl_dtype_t dtype, int64_t numel, fl_tensor_data_t *out);

@@ -2612,6 +2612,18 @@ int32_t fl_sm100_one_round_plan(int32_t kind, int32_t m, int32_t n, int32_t k, i
   });
 }
 
+int32_t fl_sm100_one_round_pairs(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t *plan) {
+  return guard([&]() -> int32_t {
+    if (!plan) invalid("plan is null");
+    if (kind != kGemmF16 && kind != kGemmBF16) invalid("kind is 0 (half rows) or 1 (bfloat16 rows)");
+    if (m < 1 || n < 1 || k < 1 || sms < 2) invalid("m, n, k are positive and the device has at least two SMs");
+    int out[8];
+    gemm_pair_describe(static_cast<GemmKind>(kind), m, n, k, sms, out);
+    for (int i = 0; i < 8; ++i) plan[i] = out[i];
+    return clear_error();
+  });
+}
+
 int64_t fl_sm100_launch_count(void) {
   return g_gemm_launches.load() + g_block_launches.load() + helper_launch_count() + elementwise_launch_count() +
          general_matmul_launch_count();

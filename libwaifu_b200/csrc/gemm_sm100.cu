@@ -1271,7 +1271,9 @@ int sm_count() {
   return cached;
 }
 
-bool gemm_widens_bf16(int m, int n, int k) { return gemm_split_plan(kGemmBF16, 1, m, n, k, sm_count(), true).split > 0; }
+bool gemm_widens_bf16(int m, int n, int k) {
+  return gemm_pair_plan(kGemmBF16, m, n, k, sm_count()).split > 0 || gemm_split_plan(kGemmBF16, 1, m, n, k, sm_count(), true).split > 0;
+}
 
 // The schedule (see the head of this file). What the stream-K part can save is the idle share of
 // the last round, (units - remainder) / units of a tile's main loop; what it costs, measured, is
@@ -1387,7 +1389,9 @@ cudaError_t launch_gemm(const GemmArgs &a, const char **why) {
   const bool bf16_widening = a.b_is_e4m3 && a.kind == kGemmBF16;
   if ((!a.force_single_cta || bf16_widening) && gemm_split_supported(a)) {
     const bool stream_k = a.sk_partials && a.sk_counters && !a.no_stream_k;
-    const SplitPlan split = gemm_split_plan(a.kind, a.b_is_e4m3, a.m, a.n, a.k, sm_count(), stream_k);
+    SplitPlan split = {0, 0, false};
+    if (a.b_is_e4m3 && a.kind != kGemmE4M3) split = gemm_pair_plan(a.kind, a.m, a.n, a.k, sm_count());
+    if (split.split == 0) split = gemm_split_plan(a.kind, a.b_is_e4m3, a.m, a.n, a.k, sm_count(), stream_k);
     if (split.split > 0) return launch_gemm_split(a, split, why);
   }
   if (a.b_is_e4m3 && (a.kind != kGemmF16 || kp.num_out > 1)) {

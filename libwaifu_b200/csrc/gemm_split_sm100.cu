@@ -14,6 +14,11 @@
 //   warp  9    MMA: four tcgen05.mma per stage (128 x block_n, 32 bytes of K per row each)
 // Every operand row of a stage is 128 bytes in the 128-byte swizzle, except the raw e4m3 tile of
 // the widening form (64 bytes of K, as it lies).
+//
+// PAIR, for 16-bit rows of more than one row block: a cluster of two CTAs computes a tile of 256 rows with
+// tcgen05.mma.cta_group::2, each with 128 of the rows and half of the tile's columns, which it loads,
+// widens and keeps for both. So a weight tile is fetched and widened once for 256 rows, where the form
+// above does it for 128. K stays in one piece.
 #include "gemm_split_sm100.cuh"
 
 #include <cuda.h>
@@ -39,6 +44,9 @@ constexpr int kMaxLoadStages = 8;
 constexpr int kMaxWideSlots = 4;
 constexpr int kATileBytes = kTileM * kStageRowBytes;
 constexpr int kSmemPerCta = 227 * 1024 - 1024;  // (static shared memory beside it)
+
+// A pair's estimate has to be this far below the other form's, or the persistent kernel's.
+constexpr float kPairMargin = 0.94f;
 
 struct SplitParams {
   int m, n, num_kb;
@@ -98,12 +106,14 @@ __device__ __forceinline__ const uint16_t *residual_at(const SplitParams &p, int
 __device__ __forceinline__ void prefetch_l2(const void *at) { asm volatile("prefetch.global.L2 [%0];" ::"l"(at)); }
 
 // KIND: kKindF8, or kKindF16 / kKindBF16 with WIDEN: the weight is e4m3 and the rows are 16-bit.
-template <int KIND, bool WIDEN>
+template <int KIND, bool WIDEN, bool PAIR = false>
 __global__ void __launch_bounds__(kSplitThreads, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const SplitParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  static_assert(WIDEN || !PAIR, "pairs are for the widening form");
   __shared__ __align__(8) uint64_t full_bar[kMaxLoadStages], empty_bar[kMaxLoadStages];
+  __shared__ __align__(8) uint64_t raw_full_bar[PAIR ? kMaxLoadStages : 1];  // this CTA's share of the weight tile
   __shared__ __align__(8) uint64_t wide_full_bar[kMaxWideSlots], wide_empty_bar[kMaxWideSlots];
   __shared__ __align__(8) uint64_t acc_full_bar;
   __shared__ uint32_t tmem_base_slot;
@@ -111,10 +121,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31;
-  const int rank = p.split > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
-  const int tile = blockIdx.x / p.split;
+  // (a pair's CTAs finish all columns of their own rows, as an undivided tile's do)
+  const int peer = PAIR ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int rank = !PAIR && p.split > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+  const bool leader = peer == 0;
+  const int tile = blockIdx.x / (PAIR ? 2 : p.split);
   const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;  // neighbours share a weight tile
-  const int m0 = tm * kTileM, n0 = tn * p.block_n;
+  const int m0 = PAIR ? (2 * tm + peer) * kTileM : tm * kTileM;
+  const int n0 = tn * p.block_n;
+  const int b_rows = PAIR ? p.block_n / 2 : p.block_n;  // of the weight tile, in this CTA
+  const int b_row0 = n0 + peer * b_rows;
   const int kb0 = p.num_kb * rank / p.split, kb1 = p.num_kb * (rank + 1) / p.split;
   const int b_row_bytes = WIDEN ? kStageRowBytes / 2 : kStageRowBytes;
 
@@ -122,9 +138,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (static_cast<int>(lane) < p.load_stages) {
       mbar_init(&full_bar[lane], 1);
       mbar_init(&empty_bar[lane], 1);
+      if constexpr (PAIR) mbar_init(&raw_full_bar[lane], 1);
     }
     if (lane < kMaxWideSlots) {
-      mbar_init(&wide_full_bar[lane], WIDEN ? kWorkWarps / p.wide_slots : 1);
+      mbar_init(&wide_full_bar[lane], WIDEN ? kWorkWarps / p.wide_slots * (PAIR ? 2 : 1) : 1);
       mbar_init(&wide_empty_bar[lane], 1);
     }
     if (lane == 0) {
@@ -138,14 +155,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tma_prefetch_desc(&tmap_b);
     // The first stages of the weight into L2 while the kernel ahead in the stream may still run: a
     // prefetch writes nothing and the loads below read what they would have read anyway.
-    for (int kb = kb0; kb < kb1 && kb < kb0 + p.load_stages; ++kb) tma_prefetch_l2_2d(&tmap_b, kb * b_row_bytes, n0);
+    for (int kb = kb0; kb < kb1 && kb < kb0 + p.load_stages; ++kb) tma_prefetch_l2_2d(&tmap_b, kb * b_row_bytes, b_row0);
   }
   if (warp == kIssueWarp) {
-    tmem_alloc<1>(&tmem_base_slot, p.tmem_cols);
-    tmem_relinquish<1>();
+    tmem_alloc<PAIR ? 2 : 1>(&tmem_base_slot, p.tmem_cols);
+    tmem_relinquish<PAIR ? 2 : 1>();
   }
   tc_fence_before_sync();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   griddep_wait();
@@ -172,9 +190,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           break;
         }
         uint8_t *base = smem + s * p.load_bytes;
-        mbar_arrive_expect_tx(&full_bar[s], bytes);
-        tma_load_2d(base + kATileBytes, &tmap_b, &full_bar[s], kb * b_row_bytes, n0);
-        tma_load_2d(base, &tmap_a, &full_bar[s], kb * kStageRowBytes, m0);
+        if constexpr (PAIR) {
+          // The weight's bytes count on this CTA's own barrier, for its widening warps, the rows of both
+          // CTAs on the leader's.
+          mbar_arrive_expect_tx(&raw_full_bar[s], static_cast<uint32_t>(b_rows * b_row_bytes));
+          tma_load_2d(base + kATileBytes, &tmap_b, &raw_full_bar[s], kb * b_row_bytes, b_row0);
+          if (leader) mbar_arrive_expect_tx(&full_bar[s], 2 * kATileBytes);
+          tma_load_2d_pair(base, &tmap_a, map_to_cta(smem_u32(&full_bar[s]), 0), kb * kStageRowBytes, m0);
+        } else {
+          mbar_arrive_expect_tx(&full_bar[s], bytes);
+          tma_load_2d(base + kATileBytes, &tmap_b, &full_bar[s], kb * b_row_bytes, n0);
+          tma_load_2d(base, &tmap_a, &full_bar[s], kb * kStageRowBytes, m0);
+        }
         if (++s == p.load_stages) {
           s = 0;
           phase ^= 1;
@@ -187,29 +214,41 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else if (warp == kIssueWarp) {
     // (the whole warp walks the loop and one lane issues, as in the persistent kernel)
+    // A pair's leader issues for both; its commits arrive at the same barrier in both.
     const bool issuer = elect_one();
     constexpr uint32_t kFmt = KIND == kKindBF16 ? 1u : 0u;
-    const uint32_t idesc = umma_idesc(kTileM, static_cast<uint32_t>(p.block_n), kFmt, kFmt);
+    const uint32_t idesc = umma_idesc(PAIR ? 2 * kTileM : kTileM, static_cast<uint32_t>(p.block_n), kFmt, kFmt);
     const uint32_t smem0 = smem_u32(smem);
+    auto commit = [&](uint64_t *bar) {
+      if constexpr (PAIR) {
+        umma_commit_pair_both(bar);
+      } else {
+        umma_commit(bar);
+      }
+    };
     bool ok = true;
     int s = 0, w = 0;
     uint32_t phase = 0, wide_phase = 0;
-    for (int kb = kb0; kb < kb1; ++kb) {
+    for (int kb = leader ? kb0 : kb1; kb < kb1; ++kb) {
       if (!mbar_wait(&full_bar[s], phase, &abort_flag) || (WIDEN && !mbar_wait(&wide_full_bar[w], wide_phase, &abort_flag))) {
         ok = false;
         break;
       }
       tc_fence_after_sync();
       const uint64_t ad = umma_desc_sw128(smem0 + s * p.load_bytes);
-      const uint64_t bd = umma_desc_sw128(WIDEN ? smem0 + p.wide_off + w * p.block_n * kStageRowBytes
+      const uint64_t bd = umma_desc_sw128(WIDEN ? smem0 + p.wide_off + w * b_rows * kStageRowBytes
                                                 : smem0 + s * p.load_bytes + kATileBytes);
 #pragma unroll
       for (int i = 0; i < kStepsPerStage; ++i) {
-        if (issuer) umma_ss<KIND>(tmem_base, ad + i * 2, bd + i * 2, idesc, (kb > kb0 || i > 0) ? 1u : 0u);
+        if constexpr (PAIR) {
+          if (issuer) umma_ss_pair<KIND>(tmem_base, ad + i * 2, bd + i * 2, idesc, (kb > kb0 || i > 0) ? 1u : 0u);
+        } else {
+          if (issuer) umma_ss<KIND>(tmem_base, ad + i * 2, bd + i * 2, idesc, (kb > kb0 || i > 0) ? 1u : 0u);
+        }
       }
       if (issuer) {
-        umma_commit(&empty_bar[s]);
-        if (WIDEN) umma_commit(&wide_empty_bar[w]);
+        commit(&empty_bar[s]);
+        if (WIDEN) commit(&wide_empty_bar[w]);
       }
       if (WIDEN && ++w == p.wide_slots) {
         w = 0;
@@ -220,7 +259,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         phase ^= 1;
       }
     }
-    if (ok && issuer) umma_commit(&acc_full_bar);
+    if (ok && issuer && leader) commit(&acc_full_bar);
     if (!ok && issuer) {
       abort_flag = 1;
       atomicCAS(p.status, 0u, static_cast<uint32_t>(kStatusMmaTimeout));
@@ -235,15 +274,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     bool ok = true;
     for (int it = w; it < kb1 - kb0; it += p.wide_slots) {
       const int s = it % p.load_stages;
-      if (!mbar_wait(&full_bar[s], (it / p.load_stages) & 1, &abort_flag) ||
+      if (!mbar_wait(PAIR ? &raw_full_bar[s] : &full_bar[s], (it / p.load_stages) & 1, &abort_flag) ||
           !mbar_wait(&wide_empty_bar[w], ((it / p.wide_slots) & 1) ^ 1, &abort_flag)) {
         ok = false;
         break;
       }
       const uint8_t *raw = smem + s * p.load_bytes + kATileBytes;
-      uint8_t *wide = smem + p.wide_off + w * p.block_n * kStageRowBytes;
+      uint8_t *wide = smem + p.wide_off + w * b_rows * kStageRowBytes;
 #pragma unroll 4
-      for (int piece = first; piece < p.block_n * 4; piece += group_warps * 32) {
+      for (int piece = first; piece < b_rows * 4; piece += group_warps * 32) {
         const uint32_t r = static_cast<uint32_t>(piece) >> 2, q = static_cast<uint32_t>(piece) & 3;
         const uint4 v = *reinterpret_cast<const uint4 *>(raw + piece * 16);
         uint4 lo, hi;
@@ -258,7 +297,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
       fence_proxy_async_smem();  // the UMMA reads these bytes through the async proxy
       __syncwarp();
-      if (lane == 0) mbar_arrive(&wide_full_bar[w]);
+      if (lane == 0) {
+        if (PAIR && !leader) {
+          mbar_arrive_remote(map_to_cta(smem_u32(&wide_full_bar[w]), 0));
+        } else {
+          mbar_arrive(&wide_full_bar[w]);
+        }
+      }
     }
     if (!ok && lane == 0) {
       abort_flag = 1;
@@ -403,9 +448,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies that may still be in flight
     __syncthreads();
   }
+  // The leader's instructions read the other CTA's shared memory, and both signal each other.
+  if constexpr (PAIR) cluster_sync_all();
   if (warp == kIssueWarp) {
     tc_fence_after_sync();
-    tmem_dealloc<1>(tmem_base, p.tmem_cols);
+    tmem_dealloc<PAIR ? 2 : 1>(tmem_base, p.tmem_cols);
   }
 }
 
@@ -449,12 +496,13 @@ struct SplitGeometry {
 
 SplitGeometry split_geometry(bool widen, int m, int n, int k, const SplitPlan &plan) {
   SplitGeometry g = {};
+  const int tile_m = plan.pair ? 2 * kTileM : kTileM, b_rows = plan.pair ? plan.block_n / 2 : plan.block_n;
   g.num_kb = (k * (widen ? 2 : 1) + kStageRowBytes - 1) / kStageRowBytes;
-  g.tiles_m = (m + kTileM - 1) / kTileM;
-  g.ctas = g.tiles_m * ((n + plan.block_n - 1) / plan.block_n) * plan.split;
-  g.load_bytes = kATileBytes + plan.block_n * (widen ? kStageRowBytes / 2 : kStageRowBytes);
-  g.wide_slots = plan.block_n <= 128 ? kMaxWideSlots : 2;
-  const int wide_bytes = widen ? g.wide_slots * plan.block_n * kStageRowBytes : 0;
+  g.tiles_m = (m + tile_m - 1) / tile_m;
+  g.ctas = g.tiles_m * ((n + plan.block_n - 1) / plan.block_n) * (plan.pair ? 2 : plan.split);
+  g.load_bytes = kATileBytes + b_rows * (widen ? kStageRowBytes / 2 : kStageRowBytes);
+  g.wide_slots = b_rows <= (plan.pair ? 96 : 128) ? kMaxWideSlots : 2;
+  const int wide_bytes = widen ? g.wide_slots * b_rows * kStageRowBytes : 0;
   const int longest = (g.num_kb + plan.split - 1) / plan.split;
   g.load_stages = std::min((kSmemPerCta - 1024 - wide_bytes) / g.load_bytes, kMaxLoadStages);
   if (widen) {
@@ -468,18 +516,18 @@ SplitGeometry split_geometry(bool widen, int m, int n, int k, const SplitPlan &p
   return g;
 }
 
-template <int KIND, bool WIDEN>
+template <int KIND, bool WIDEN, bool PAIR = false>
 cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {
   const uint64_t row_bytes = static_cast<uint64_t>(a.k) * (KIND == kKindF8 ? 1 : 2);
   CUtensorMap ta, tb;
-  const uint32_t bn = static_cast<uint32_t>(plan.block_n);
+  const uint32_t bn = static_cast<uint32_t>(PAIR ? plan.block_n / 2 : plan.block_n);  // weight rows to a CTA
   if (!make_map(&ta, a.a, a.m, row_bytes, kStageRowBytes, kTileM, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !(WIDEN ? make_map(&tb, a.b, a.n, row_bytes / 2, kStageRowBytes / 2, bn, CU_TENSOR_MAP_SWIZZLE_NONE)
               : make_map(&tb, a.b, a.n, row_bytes, kStageRowBytes, bn, CU_TENSOR_MAP_SWIZZLE_128B))) {
     *why = "cuTensorMapEncodeTiled refused an operand";
     return cudaErrorInvalidValue;
   }
-  auto kernel = gemm_split_kernel<KIND, WIDEN>;
+  auto kernel = gemm_split_kernel<KIND, WIDEN, PAIR>;
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
@@ -515,7 +563,7 @@ cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **
   p.vector_io = (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
                 (!a.residual || ((reinterpret_cast<uintptr_t>(a.residual) & 15) == 0 && a.residual_ld % 8 == 0));
   p.tmem_cols = 32;
-  while (p.tmem_cols < bn) p.tmem_cols *= 2;
+  while (p.tmem_cols < static_cast<uint32_t>(plan.block_n)) p.tmem_cols *= 2;
   p.status = a.status;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(g.ctas), 1, 1);
@@ -526,11 +574,11 @@ cudaError_t launch_split(const GemmArgs &a, const SplitPlan &plan, const char **
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(plan.split);
+  attr[1].val.clusterDim.x = static_cast<unsigned>(PAIR ? 2 : plan.split);
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = plan.split > 1 ? 2 : 1;
+  cfg.numAttrs = PAIR || plan.split > 1 ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
   if (e != cudaSuccess) *why = "kernel launch failed";
   return e;
@@ -551,8 +599,9 @@ bool gemm_split_supported(const GemmArgs &a) {
 //   77 x 2560 x 2048, half: 17.7 us on the persistent kernel, 11.2 here; 300 x 1280 x 640 15.4 and
 //   7.8; 512 x 5120 x 3072 in bfloat16 39 (with a widening pass) and 30.7; e4m3 rows with
 //   the quantiser, 300 x 1280 x 1280 15.3 and 10.0, 1024 x 3072 x 3072 21.8 and 20.1.
-SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k) {
-  SplitPlan best = {0, 0};
+static SplitPlan timed_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k, float *estimate) {
+  SplitPlan best = {0, 0, false};
+  *estimate = 0.0f;
   if (kind != kGemmE4M3 && !b_is_e4m3) return best;
   const bool widen = kind != kGemmE4M3;
   const int num_kb = (k * (widen ? 2 : 1) + kStageRowBytes - 1) / kStageRowBytes;
@@ -617,28 +666,69 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
       const float time = (num_kb + split - 1) / split * stage + bn * scale * (widen ? 0.044f : 0.03f) + exchange + (widen ? 2.6f : 6.3f);
       if (time < best_time) {
         best_time = time;
-        best = {bn, split};
+        best = {bn, split, false};
       }
+    }
+  }
+  *estimate = best_time;
+  return best;
+}
+
+SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int sms, bool stream_k) {
+  float estimate;
+  return timed_plan(kind, b_is_e4m3, m, n, k, sms, stream_k, &estimate);
+}
+
+// Estimated as above, fitted to 34 shapes of 129 to 2048 rows and every width: a stage takes its way through the
+// widening warps and across the pair and back, 0.315 us with four widened slots, 0.45 with the two there is room
+// for above 192 columns. 512 x 5120 x 3072 in bfloat16: 30.6 us in tiles of 128 rows, 25.1 in tiles of 256 x 160;
+// 238 x 14088 x 2304 31.1 and 23.4, 1705 x 1400 x 3696 in half 34.5 and 27.6; below some thirty tiles the shorter
+// stages and the divided K of the other form win (300 x 2560 x 2048 15.9 and 16.9).
+SplitPlan gemm_pair_plan(GemmKind kind, int m, int n, int k, int sms) {
+  SplitPlan best = {0, 0, false};
+  if ((kind != kGemmF16 && kind != kGemmBF16) || m <= kTileM) return best;
+  float best_time;
+  timed_plan(kind, 1, m, n, k, sms, true, &best_time);
+  best_time *= kPairMargin;
+  const int num_kb = (k * 2 + kStageRowBytes - 1) / kStageRowBytes;
+  const int tiles_m = (m + 2 * kTileM - 1) / (2 * kTileM);
+  for (int bn = 64; bn <= 256; bn += 32) {
+    if (static_cast<long long>(tiles_m) * ((n + bn - 1) / bn) > sms / 2) continue;
+    const float time = num_kb * (bn <= 192 ? 0.315f : 0.45f) + bn * 0.029f + (bn <= 192 ? 5.2f : 5.8f);
+    if (time < best_time) {
+      best_time = time;
+      best = {bn, 1, true};
     }
   }
   return best;
 }
 
-void gemm_split_describe(GemmKind kind, int m, int n, int k, int sms, bool stream_k, int *plan) {
+namespace {
+
+void describe(bool widen, int m, int n, int k, const SplitPlan &cut, int *plan) {
   for (int i = 0; i < 8; ++i) plan[i] = 0;
-  const SplitPlan cut = gemm_split_plan(kind, kind != kGemmE4M3, m, n, k, sms, stream_k);
   if (cut.split == 0) return;
-  const SplitGeometry g = split_geometry(kind != kGemmE4M3, m, n, k, cut);
+  const SplitGeometry g = split_geometry(widen, m, n, k, cut);
   plan[0] = cut.block_n, plan[1] = cut.split, plan[2] = g.ctas, plan[3] = g.num_kb;
-  plan[4] = g.load_stages, plan[5] = kind != kGemmE4M3 ? g.wide_slots : 0, plan[6] = g.load_bytes, plan[7] = g.smem_bytes;
+  plan[4] = g.load_stages, plan[5] = widen ? g.wide_slots : 0, plan[6] = g.load_bytes, plan[7] = g.smem_bytes;
+}
+
+}  // namespace
+
+void gemm_split_describe(GemmKind kind, int m, int n, int k, int sms, bool stream_k, int *plan) {
+  describe(kind != kGemmE4M3, m, n, k, gemm_split_plan(kind, kind != kGemmE4M3, m, n, k, sms, stream_k), plan);
+}
+
+void gemm_pair_describe(GemmKind kind, int m, int n, int k, int sms, int *plan) {
+  describe(true, m, n, k, gemm_pair_plan(kind, m, n, k, sms), plan);
 }
 
 cudaError_t launch_gemm_split(const GemmArgs &a, const SplitPlan &plan, const char **why) {
   *why = "";
   switch (a.kind) {
     case kGemmE4M3: return launch_split<kKindF8, false>(a, plan, why);
-    case kGemmBF16: return launch_split<kKindBF16, true>(a, plan, why);
-    default: return launch_split<kKindF16, true>(a, plan, why);
+    case kGemmBF16: return plan.pair ? launch_split<kKindBF16, true, true>(a, plan, why) : launch_split<kKindBF16, true>(a, plan, why);
+    default: return plan.pair ? launch_split<kKindF16, true, true>(a, plan, why) : launch_split<kKindF16, true>(a, plan, why);
   }
 }
 

@@ -1,0 +1,46 @@
+"""GPU parity of the one-round kernel's tiles of 256 rows (fl_fp8_matmul[_add] on more than one row block
+against an e4m3 weight) with the oracle: every tile width, row counts that leave a pair's second CTA few
+rows or none, columns and K that end inside a tile and a stage. Tolerances as in test_gpu_one_round.py."""
+import numpy as np
+import pytest
+
+from helpers import check_parity, random_codes, randn
+from test_gpu_one_round import matmul
+from test_one_round_pairs_cpu import pairs
+
+pytestmark = pytest.mark.gpu
+
+# every width, and what it is taken at
+CASES = [(663, 2832, 1152, 128), (129, 8632, 2704, 128), (512, 5120, 3072, 160), (1705, 1400, 3696, 160), (238, 14088, 2304, 192),
+         (385, 7048, 3088, 192), (256, 16384, 3072, 224)]
+
+
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("m,n,k,width", CASES)
+@pytest.mark.parametrize("is_bf16", [False, True])
+@pytest.mark.parametrize("addend", ["none", "bias", "residual"])
+def test_matmul_in_pairs(flint, oracle, m, n, k, width, is_bf16, addend):
+    if pairs(1, m, n, k, sms())["block_n"] != width or (not is_bf16 and pairs(0, m, n, k, sms())["block_n"] == 0):
+        pytest.skip("not taken on this card")
+    rng = np.random.default_rng(m + n + k)
+    a = oracle.narrow(randn(rng, (m, k)), is_bf16)
+    codes = random_codes(rng, n, k)
+    add = None if addend == "none" else oracle.narrow(randn(rng, (n,) if addend == "bias" else (m, n)), is_bf16)
+    got = matmul(flint, a, codes, 0.0137, is_bf16, add)
+    check_parity(oracle, got, oracle.fp8_matmul(a, codes, [np.float32(0.0137)], add, is_bf16), is_bf16, what=f"{m}x{n}x{k}")
+
+
+@pytest.mark.parametrize("is_bf16", [False, True])
+def test_nan_codes_stay_nan_in_pairs(flint, oracle, is_bf16):
+    rng = np.random.default_rng(8)
+    m, n, k = 663, 2832, 1152
+    assert pairs(int(is_bf16), m, n, k, 148)["block_n"] > 0
+    a, codes = oracle.narrow(randn(rng, (m, k)), is_bf16), random_codes(rng, n, k)
+    codes[3, 17], codes[2700, 1151] = 0x7F, 0xFF
+    y = oracle.widen(matmul(flint, a, codes, 0.0137, is_bf16), is_bf16)
+    assert np.isnan(y[:, [3, 2700]]).all()
+    assert np.isfinite(np.delete(y, [3, 2700], axis=1)).all()

@@ -1,0 +1,49 @@
+"""The one-round kernel's tiles of 256 rows (a pair of CTAs each), their index arithmetic without a GPU."""
+import ctypes
+import random
+
+import pytest
+
+from libwaifu_b200 import flint as F
+
+NAMES = ("block_n", "split", "ctas", "num_kb", "load_slots", "wide_slots", "slot_bytes", "smem")
+
+
+def pairs(kind, m, n, k, sms=148):
+    out = (ctypes.c_int32 * 8)()
+    F.check(F.lib().fl_sm100_one_round_pairs(kind, m, n, k, sms, out))
+    return dict(zip(NAMES, out))
+
+
+@pytest.mark.parametrize("sms", [148, 132, 16, 2])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_pair_invariants(kind, sms):
+    """All pairs are resident at once; a CTA's half of the columns is whole 16-row groups whose slots stay
+    on 1024-byte boundaries; rings and exchange buffer fit; a ring of loads holds whole turns of the
+    widened ring, so that a warp meets every phase of its barriers."""
+    rng = random.Random(23)
+    taken = 0
+    for _ in range(3000):
+        m, n, k = int(2 ** rng.uniform(0, 13)), 8 * int(2 ** rng.uniform(0, 11.2)), 16 * int(2 ** rng.uniform(0, 9.7))
+        p = pairs(kind, m, n, k, sms)
+        if p["block_n"] == 0:
+            assert not any(p.values())
+            continue
+        taken += 1
+        what = f"{m}x{n}x{k} {p}"
+        half = p["block_n"] // 2
+        assert m > 128 and p["split"] == 1 and 32 <= p["block_n"] <= 256 and p["block_n"] % 32 == 0, what
+        assert p["num_kb"] == -(-k * 2 // 128)
+        assert p["ctas"] == -(-m // 256) * -(-n // p["block_n"]) * 2 and p["ctas"] <= sms, what
+        assert p["slot_bytes"] == 128 * 128 + half * 64 and p["slot_bytes"] % 1024 == 0 and half * 128 % 1024 == 0, what
+        assert p["wide_slots"] in (2, 4) and 1 <= p["load_slots"] <= 8 and p["load_slots"] % p["wide_slots"] == 0, what
+        assert p["smem"] - 1024 >= p["load_slots"] * p["slot_bytes"] + p["wide_slots"] * half * 128, what
+        assert p["smem"] - 1024 >= p["block_n"] // 4 * (128 * 16 + 16) and p["smem"] <= 227 * 1024 - 1024, what
+    assert taken > 0 or sms < 132
+
+
+def test_refusals():
+    out = (ctypes.c_int32 * 8)()
+    for bad in [(2, 200, 8, 16, 148), (-1, 200, 8, 16, 148), (0, 0, 8, 16, 148), (0, 200, 8, 16, 1)]:
+        assert F.lib().fl_sm100_one_round_pairs(*bad, out) == F.FL_ERROR_INVALID_ARG
+    assert F.lib().fl_sm100_one_round_pairs(0, 200, 8, 16, 148, None) == F.FL_ERROR_INVALID_ARG
