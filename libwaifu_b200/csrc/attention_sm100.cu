@@ -652,9 +652,9 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 // (scores -> softmax -> P -> product -> the next scores, which overwrite P); the other tile's
 // chain runs in its gaps.
 //
-// The grid has a CTA per unit (two tiles of one head's queries), but a running CTA may take over units
-// whose own CTA has not started yet (clusterlaunchcontrol.try_cancel) instead of leaving its SM to
-// it. Keys, values and queries of the next unit then arrive, and its first scores are computed, under
+// Runs of short walks take a second form of the kernel (attention2_units_kernel, below). The grid has a CTA
+// per unit (two tiles of one head's queries) there too, but a running CTA takes over units whose own
+// CTA has not started yet (clusterlaunchcontrol.try_cancel) instead of leaving its SM to it. Keys, values and queries of the next unit then arrive, and its first scores are computed, under
 // the last products and the output of the one before, and barriers and tensor memory are set up once
 // per SM. The hardware hands the units out in the grid's order, as it starts CTAs.
 constexpr int kTiles = 2;
@@ -666,12 +666,10 @@ constexpr int kMmaWarp2 = kSoftmaxWarps2 + 1;
 // (two of its warps have nothing to do) gives its own up to the two of the softmax, which hold a
 // row of 128 scores: 128 x 88 + 256 x 208 = 384 x 168 (a CTA that takes units over: 96 and 200).
 constexpr int kThreads2 = (kSoftmaxWarps2 + 4) * 32;
-template <bool TAKE_OVER>
-constexpr int kIssueRegs = TAKE_OVER ? 96 : 88;
-template <bool TAKE_OVER>
-constexpr int kSoftmaxRegs = TAKE_OVER ? 200 : 208;
-static_assert(128 * kIssueRegs<true> + kSoftmaxWarps2 * 32 * kSoftmaxRegs<true> <= kThreads2 * 168 &&
-                  128 * kIssueRegs<false> + kSoftmaxWarps2 * 32 * kSoftmaxRegs<false> <= kThreads2 * 168,
+constexpr int kIssueRegs = 88, kSoftmaxRegs = 208;
+constexpr int kUnitsIssueRegs = 96, kUnitsSoftmaxRegs = 200;
+static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2 * 168 &&
+                  128 * kUnitsIssueRegs + kSoftmaxWarps2 * 32 * kUnitsSoftmaxRegs <= kThreads2 * 168,
               "no more than the block was launched with");
 // A block's probabilities are handed over in so many parts of its keys. At head_dim 128 the product of
 // the first half runs under the exponentials of the second (2 x 24 x 4352: 396 -> 386 us); at 64,
@@ -683,7 +681,9 @@ constexpr int kMaxSlots = 6;
 // The longest walks, in blocks of keys, whose CTA goes on with another unit, under the causal masks and
 // without one: 4 x 32 x 1000 causal 63.4 -> 57.4 us, 2 x 24 x 2048 causal at head_dim 64 60 -> 55, 2 x 24 x 300
 // at 64 13.4 -> 12.5, 3 x 24 x 1000 49.6 -> 49.4; but 24 x 2048 73.6 -> 74.5, 2 x 24 x 4352 398 -> 425, causal 347
-// both ways: what a block takes in that form is a little longer, and a long walk has little to hide.
+// both ways: what a block takes in that form is a little longer, and a long walk has little to hide. (One
+// kernel with the loop over units compiled out took 459 for the second shape among others of its kind,
+// the kernel without it 449.)
 constexpr int kTakeOverBlocksCausal = 16, kTakeOverBlocks = 8;
 
 struct Tail2 {
@@ -722,6 +722,415 @@ struct Layout2 {
   static_assert(kOCol + kTiles * D <= kTmemCols, "tensor memory holds 512 columns");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
+
+template <int D>
+__global__ void __launch_bounds__(kThreads2, 1)
+attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                  const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
+  using L = Layout2<D>;
+  constexpr int S = L::kSlots;
+  constexpr int kPParts = kPartsOf<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  Tail2 &t = *reinterpret_cast<Tail2 *>(smem + L::kTailOff);
+  volatile uint32_t &abort_flag = *reinterpret_cast<volatile uint32_t *>(&t.abort_flag);
+
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  if ((smem_u32(smem) & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicCAS(p.status, 0u, kStatusAttentionLayout);
+    return;
+  }
+  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its
+  // keys and values in L2. Under the causal masks the later queries have more keys to walk: the last
+  // unit of every head goes first, then the one before it, so that the grid ends on the short ones
+  // whatever the head.
+  int unit = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
+  if (p.mask_type != 0) {
+    const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
+    const int order = unit + units * (head + heads * batch);
+    unit = units - 1 - order / all;
+    head = order % all % heads;
+    batch = order % all / heads;
+  }
+  const int q0 = unit * (kTiles * kBlockQ);
+  const int kv_head = head / p.group;
+  const int offset = p.kv_len - p.q_len;
+  // Both tiles start at the first block of keys that some query of the CTA sees.
+  const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
+  const int kv_begin = first_key_of(p, q0 + offset);
+  const int kv_end = last_key_of(p, last_row + offset) + 1;
+  const int block0 = kv_begin / kBlockKv;
+  const int num_blocks = (kv_end + kBlockKv - 1) / kBlockKv - block0;
+  // Under the causal masks the first tile's queries see nothing of the last blocks the second walks;
+  // a tile past the last query has none.
+  auto blocks_of = [&](int i) -> int {
+    if (q0 + i * kBlockQ >= p.q_len) return 0;
+    const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
+    return min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv - block0);
+  };
+
+  if (threadIdx.x == 0) {
+    t.abort_flag = 0;
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&t.slot_full_bar[i], 1);
+      mbar_init(&t.slot_empty_bar[i], 1);
+    }
+    for (int i = 0; i < kTiles; ++i) {
+      mbar_init(&t.q_full_bar[i], 1);
+      mbar_init(&t.s_full_bar[i], 1);
+      for (int h = 0; h < kPParts; ++h) mbar_init(&t.p_full_bar[i][h], kTileWarps);
+      mbar_init(&t.pv_done_bar[i], 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == kProducerWarp2 && lane == 0) {
+    tma_prefetch_desc(&tmap_q);
+    tma_prefetch_desc(&tmap_k);
+    tma_prefetch_desc(&tmap_vt);
+  }
+  if (warp == kMmaWarp2) {
+    tmem_alloc<1>(&t.tmem_base_slot, L::kTmemCols);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = t.tmem_base_slot;
+
+  auto q_tile = [&](int i) { return smem + L::kQOff + i * L::kQBytes; };
+  auto slot = [&](int i) { return smem + L::kSlotOff + i * L::kSlotBytes; };
+
+  // Load n of the ring (K of block n / 2 when n is even, V of it when odd) goes to slot n % S.
+  if (warp < kSoftmaxWarps2) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    // ------------------------------------------------------------------ softmax and output
+    const int tile = static_cast<int>(warp >> 2);
+    const uint32_t quarter = warp & 3;
+    const int tq0 = q0 + tile * kBlockQ;  // the tile's first query
+    const int row = static_cast<int>(quarter) * 32 + static_cast<int>(lane);
+    const int q_pos = tq0 + row + offset;
+    const int key_first = first_key_of(p, q_pos), key_last = last_key_of(p, q_pos);
+    const int tile_last_row = min(tq0 + kBlockQ, p.q_len) - 1;
+    // What every query of the tile sees (an empty range for a tile past the last query: every block
+    // is then an edge block, and nothing of it is stored).
+    const int common_first = first_key_of(p, tile_last_row + offset), common_last = last_key_of(p, tq0 + offset);
+    const uint32_t t_lane = tmem_base + ((quarter * 32u) << 16);
+    const uint32_t t_scores = t_lane + tile * L::kSCols;  // the row's 128 scores, then its 128 probabilities in 64 columns
+    const uint32_t t_out = t_lane + L::kOCol + tile * D;
+    constexpr int kChunks = kBlockKv / 32;
+    static_assert(kChunks == 4, "four chunks of scores pack into the first two");
+    constexpr float kRescaleStep = 8.0f;
+    float m_used = -INFINITY;
+    float l_run = 0.0f;
+    bool ok = true;
+    uint32_t sc[kChunks][32];
+
+    const int my_blocks = blocks_of(tile);
+    for (int j = 0; j < my_blocks && ok; ++j) {
+      // The row's scores of the block into registers in one round trip. (Scores of block j are
+      // issued behind the product of block j - 1: once they are here the tile's output is complete
+      // up to that block.)
+      ok = __all_sync(0xffffffffu, mbar_wait(&t.s_full_bar[tile], j & 1, &abort_flag));
+      if (!ok) break;
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
+      const int block_key0 = (block0 + j) * kBlockKv;
+      const bool edge = block_key0 < common_first || block_key0 + kBlockKv - 1 > common_last;
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (edge) {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const int key = block_key0 + c * 32 + i;
+            if (key > key_last || key < key_first) sc[c][i] = __float_as_uint(-INFINITY);
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
+        }
+      }
+      const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+      if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
+        const float m_new = fmaxf(m_used, m_blk);
+        const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
+        l_run *= alpha;
+        if (j > 0) {
+#pragma unroll 1
+          for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
+            uint32_t v[16];
+            tmem_ld_32x16(t_out + c * 16, v);
+            tmem_ld_wait(v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+            tmem_st_32x16(t_out + c * 16, v);
+          }
+        }
+        m_used = m_new;
+      }
+      const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
+      // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
+      // (a slot whose scores have been used by then).
+      const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
+      uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
+      auto emit = [&](auto bf16_tag, int part) {
+        constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
+#pragma unroll
+        for (int h = 0; h < kChunks / kPParts; ++h) {
+          const int c = part * (kChunks / kPParts) + h;
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
+            float e0, e1;
+            if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
+              float x0, x1;
+              f2_unpack(x, &x0, &x1);
+              e0 = fast_exp2(x0);
+              e1 = fast_exp2(x1);
+            } else {
+              exp2_pair_poly(x, &e0, &e1);
+            }
+            sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
+            sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
+          }
+        }
+      };
+      // Each half of the block's keys is handed over as soon as it is there: its product runs under
+      // the exponentials of the other half.
+#pragma unroll
+      for (int part = 0; part < kPParts; ++part) {
+        if (p.is_bf16) {
+          emit(std::true_type{}, part);
+        } else {
+          emit(std::false_type{}, part);
+        }
+        tmem_st_32x32(t_scores + part * 32, sc[part]);
+        if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
+        tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
+        tc_fence_before_sync();  // before the MMAs that the hand-over starts
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
+      }
+      float s0, s1, s2, s3;
+      f2_unpack(sums[0], &s0, &s1);
+      f2_unpack(sums[1], &s2, &s3);
+      l_run += (s0 + s1) + (s2 + s3);
+    }
+    // The last product.
+    if (ok && my_blocks > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&t.pv_done_bar[tile], 0, &abort_flag));
+      tc_fence_after_sync();
+    }
+    if (ok) {
+      const bool live = tq0 + row < p.q_len;
+      const float inv = 1.0f / l_run;
+      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + batch * p.out_stride[0] + head * p.out_stride[1] +
+                      static_cast<int64_t>(tq0 + row) * p.out_stride[2];
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32(t_out + c * 32, v);
+        tmem_ld_wait(v);
+        if (live) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint4 w;
+            w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
+            w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
+            w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
+            w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
+            *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
+          }
+        }
+      }
+    }
+    if (!ok && lane == 0) {
+      abort_flag = 1;
+      atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == kProducerWarp2) {
+      // ------------------------------------------------------------------ producer
+      if (elect_one()) {
+        bool ok = true;
+        auto load = [&](void *dst, const CUtensorMap *map, uint64_t *bar, int32_t c0, int32_t c1, int32_t c2) {
+          tma_load_4d(dst, map, bar, c0, c1, c2, batch);
+        };
+        for (int i = 0; i < kTiles; ++i) {
+          mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
+#pragma unroll
+          for (int a = 0; a < L::kQAtoms; ++a) {
+            load(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, q0 + i * kBlockQ, head);
+          }
+        }
+        for (int n = 0; n < 2 * num_blocks && ok; ++n) {
+          const int st = n % S, j = n >> 1;
+          if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
+          const int key0 = (block0 + j) * kBlockKv;
+          if ((n & 1) == 0) {
+#pragma unroll
+            for (int a = 0; a < L::kQAtoms; ++a) {
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+            }
+          } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
+#pragma unroll
+            for (int a = 0; a < L::kQAtoms; ++a) {
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+            }
+          } else {
+#pragma unroll
+            for (int a = 0; a < L::kVAtoms; ++a) {
+              tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st], (key0 + a * kAtomElems) * 2, 0,
+                          batch * p.kv_heads + kv_head);
+            }
+          }
+        }
+        if (!ok) {
+          abort_flag = 1;
+          atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+        }
+      }
+    } else if (warp == kMmaWarp2) {
+      // ------------------------------------------------------------------ MMA issuer
+      // The whole warp walks the loop and an elected lane issues: what an instruction takes
+      // (descriptors, addresses) then lives in uniform registers. An issuing warp per tile measured
+      // slower (386 us for 2 x 24 x 4352, 439 to 509 so): a tile's products are then stretched by the
+      // other's, and the tiles no longer take turns. A pair of CTAs sharing K and V (cta_group::2)
+      // measured 399, and 82 against 62 on 4 x 32 x 1000 causal.
+      const bool issuer = elect_one();
+      {
+        const uint32_t fmt = p.is_bf16 ? 1u : 0u;
+        const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
+        const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
+        constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
+        constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
+        constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
+        constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
+        const uint64_t qdesc0 = umma_desc_sw128(smem_u32(q_tile(0)));
+        const uint64_t sdesc0 = umma_desc_sw128(smem_u32(slot(0)));
+        bool ok = true;
+        auto commit = [&](uint64_t *bar) {
+          if (issuer) umma_commit(bar);
+        };
+        auto scores = [&](int i, uint64_t kd) {  // S_i = Q_i K^T
+          const uint32_t s_tmem = tmem_base + i * L::kSCols;
+          const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
+#pragma unroll
+          for (int m = 0; m < kScoreMmas; ++m) {
+            const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+            const uint64_t qa = qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep);
+            const uint64_t ka = kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep);
+            if (issuer) umma_ss<kKindF16>(s_tmem, qa, ka, idesc_s, m != 0 ? 1u : 0u);
+          }
+        };
+        // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes
+        // on, the operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64
+        // head_dim positions lie a 128-key atom apart.
+        const uint32_t idesc_o_mn = idesc_o | (1u << 16);
+        const uint64_t mn_fields = umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0);
+        auto product = [&](int i, int part, uint64_t vd, uint32_t first_block) {  // O_i += P_i V over one part of the block's keys
+          const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
+          const uint32_t p_tmem = tmem_base + i * L::kSCols;
+          constexpr int kPartMmas = kOutMmas / kPParts;
+          if (p.v_direct) {
+#pragma unroll
+            for (int k = 0; k < kPartMmas; ++k) {
+              const int m = part * kPartMmas + k;
+              const uint64_t va = (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4));
+              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, va, idesc_o_mn, m != 0 ? 1u : (first_block ^ 1u));
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < kPartMmas; ++k) {
+              const int m = part * kPartMmas + k;
+              const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
+                          m != 0 ? 1u : (first_block ^ 1u));
+            }
+          }
+        };
+        auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
+        auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
+        const int blocks[kTiles] = {blocks_of(0), blocks_of(1)};
+        for (int i = 0; i < kTiles && ok; ++i) ok = mbar_wait(&t.q_full_bar[i], 0, &abort_flag);
+        if (ok && num_blocks > 0) ok = wait_full(0);
+        if (ok && num_blocks > 0) {
+          tc_fence_after_sync();
+#pragma unroll
+          for (int i = 0; i < kTiles; ++i) {
+            if (blocks[i] == 0) continue;
+            scores(i, desc_of(0));
+            commit(&t.s_full_bar[i]);
+          }
+          commit(&t.slot_empty_bar[0]);
+        }
+        for (int j = 0; j < num_blocks && ok; ++j) {
+          const bool more = j + 1 < num_blocks;
+          const int nv = 2 * j + 1, nk = 2 * j + 2;
+          if (!wait_full(nv)) ok = false;
+#pragma unroll
+          for (int i = 0; i < kTiles; ++i) {
+            if (!ok || j >= blocks[i]) continue;
+            // The product reads P from the columns the next scores overwrite: the instructions of one
+            // thread run in the order they were issued.
+#pragma unroll
+            for (int part = 0; part < kPParts; ++part) {
+              if (ok) ok = mbar_wait(&t.p_full_bar[i][part], j & 1, &abort_flag);
+              if (!ok) break;
+              tc_fence_after_sync();
+              product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
+            }
+            if (!ok) continue;
+            if (j + 1 == blocks[i]) {
+              commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
+            } else {
+              if (!wait_full(nk)) {  // (seen by the first tile's turn, for the second's too)
+                ok = false;
+                continue;
+              }
+              tc_fence_after_sync();
+              scores(i, desc_of(nk));
+              commit(&t.s_full_bar[i]);
+            }
+          }
+          if (!ok) break;
+          commit(&t.slot_empty_bar[nv % S]);  // both tiles have read the two slots
+          if (more) commit(&t.slot_empty_bar[nk % S]);
+        }
+        if (!ok && issuer) {
+          abort_flag = 1;
+          atomicCAS(p.status, 0u, kStatusAttentionTimeout);
+        }
+      }
+    }
+  }
+
+  // ---------------------------------------------------------------------- teardown
+  tc_fence_before_sync();
+  __syncthreads();
+  if (abort_flag != 0) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == kMmaWarp2) {
+    tc_fence_after_sync();
+    tmem_dealloc<1>(tmem_base, L::kTmemCols);
+  }
+}
+
+// ---- the same, going on from unit to unit ------------------------------------------------------
 
 // Two tiles of 128 queries of one head and the blocks of keys they walk, from the first on (of the
 // masks only the block diagonal one hides a run's first keys, and it is not served here).
@@ -787,10 +1196,9 @@ __device__ __forceinline__ int4 claimed_cta(const uint4 *answer) {
   return c;
 }
 
-// TAKE_OVER: the CTA goes on with other units; else it leaves after its own.
-template <int D, bool TAKE_OVER>
+template <int D>
 __global__ void __launch_bounds__(kThreads2, 1)
-attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
   using L = Layout2<D>;
   constexpr int S = L::kSlots;
@@ -855,7 +1263,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   // Load n of the ring, counted over all of the CTA's units (K of a block, V of it, K of the next), goes
   // to slot n % S.
   if (warp < kSoftmaxWarps2) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs<TAKE_OVER>));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kUnitsSoftmaxRegs));
     // ------------------------------------------------------------------ softmax and output
     const int tile = static_cast<int>(warp >> 2);
     const uint32_t quarter = warp & 3;
@@ -1009,7 +1417,6 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // four warps hand over only after these reads.
         tc_fence_before_sync();
       }
-      if constexpr (!TAKE_OVER) break;
       if (ok) {
         ok = __all_sync(0xffffffffu, read_next_unit(count, &at));
         __syncwarp();
@@ -1021,7 +1428,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       atomicCAS(p.status, 0u, kStatusAttentionTimeout);
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs<TAKE_OVER>));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kUnitsIssueRegs));
     if (warp == kProducerWarp2) {
       // ------------------------------------------------------------------ producer
       if (elect_one()) {
@@ -1075,7 +1482,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               }
             }
           }
-          if (!ok || !TAKE_OVER) break;
+          if (!ok) break;
           // The next unit is claimed once the last block of this one is on its way: as late as its own
           // loads allow, so that the CTA that is ahead takes it.
           mbar_arrive_expect_tx(&t.claim_bar, sizeof(t.claim));
@@ -1168,7 +1575,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           tc_fence_after_sync();
           scores(i, desc_of(nk));
           commit(&t.s_full_bar[i]);
-          if (TAKE_OVER && last) commit(&t.q_empty_bar[i]);
+          if (last) commit(&t.q_empty_bar[i]);
         };
         auto wait_queries = [&](int i) -> bool {
           const bool there = mbar_wait(&t.q_full_bar[i], q_phase[i], &abort_flag);
@@ -1209,7 +1616,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               bool last = j + 2 == cur[i];
               if (j + 1 == cur[i]) {
                 commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
-                if (more || !TAKE_OVER) continue;
+                if (more) continue;
                 // Through with the unit: on with the first scores of the next one, which run under the
                 // other tile's last product and this one's output.
                 if (!known) {
@@ -1326,11 +1733,11 @@ cudaError_t launch(const AttentionArgs &a, const CUtensorMap &tq, const CUtensor
   return cudaGetLastError();
 }
 
-template <int D, bool TAKE_OVER>
+template <int D, bool UNITS>
 cudaError_t launch2(const AttentionArgs &a, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
                     const KernelParams &kp, const char **why) {
   using L = Layout2<D>;
-  auto kernel = attention2_kernel<D, TAKE_OVER>;
+  auto kernel = UNITS ? attention2_units_kernel<D> : attention2_kernel<D>;
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
@@ -1343,6 +1750,10 @@ cudaError_t launch2(const AttentionArgs &a, const CUtensorMap &tq, const CUtenso
   const int per_cta = kTiles * kBlockQ;
   const dim3 grid(static_cast<unsigned>((a.q_len + per_cta - 1) / per_cta), static_cast<unsigned>(a.heads),
                   static_cast<unsigned>(a.batch));
+  if (!UNITS) {
+    kernel<<<grid, kThreads2, L::kSmemBytes, a.stream>>>(tq, tk, tvt, kp);
+    return cudaGetLastError();
+  }
   // (barriers, tensor memory and the descriptors' way in may run under the end of the kernel before)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
