@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) quantize_fp8_act_kernel(const uint16_t *_
                                                              uint8_t *__restrict__ codes,
                                                              float *__restrict__ scales) {
   griddep_wait();
-  griddep_launch_dependents();
+  griddep_launch_dependents();  // everything ahead is complete: a product may ask for its weight meanwhile
   __shared__ float red[4];
   const int64_t row = blockIdx.x;
   const uint16_t *xr = x + row * k;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) quantize_fp8_act_reg_kernel(const uint16_
                                                                  uint8_t *__restrict__ codes,
                                                                  float *__restrict__ scales) {
   griddep_wait();
-  griddep_launch_dependents();
+  griddep_launch_dependents();  // (as above)
   __shared__ float red[8];
   const int64_t row = blockIdx.x;
   const uint4 *xv = reinterpret_cast<const uint4 *>(x + row * k);
