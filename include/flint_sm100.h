@@ -441,9 +441,10 @@ FLAPI int32_t fl_sm100_one_round_plan(int32_t kind, int32_t m, int32_t n, int32_
 
 /* The same kernel's cut of half (kind 0) or bfloat16 rows (1) into tiles of 256 rows, each computed by a
  * cluster of two CTAs over the whole K: where it has one it is taken, before fl_sm100_one_round_plan's.
- * plan[8] as there: [0] tile width (0: none, and the rest is 0), [1] 1, [2] CTAs, [3] K stages of a tile,
- * [4] slots of the load ring, [5] of the ring of widened weight tiles (a CTA holds half of a tile's columns),
- * [6] bytes of a load slot, [7] dynamic shared memory of a CTA. */
+ * plan[8] as there: [0] tile width (0: none, and the rest is 0; so everywhere in a process started with
+ * FLINT_SM100_SINGLE_CTA=1), [1] 1, [2] CTAs, [3] K stages of a tile, [4] slots of the load ring, [5] of the
+ * ring of widened weight tiles (a CTA holds half of a tile's columns), [6] bytes of a load slot, [7] dynamic
+ * shared memory of a CTA. */
 FLAPI int32_t fl_sm100_one_round_pairs(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t *plan);
 
 /* Storage over device memory the caller already owns (for instance a torch tensor's): nothing

@@ -660,14 +660,7 @@ void run_gemm(GemmKind kind, int m, int n, int k, const void *a, const void *b, 
   g.out_col0 = ep.out_col0;
   g.status = status_word();
   g.stream = 0;
-  // FLINT_SM100_SINGLE_CTA=1 keeps every GEMM on the persistent kernel, without CTA pairs (for A/B
-  // measurements); bfloat16 rows against an e4m3 weight, where few tiles go to the one-round kernel
-  // without a widened copy of the weight, still go there.
-  static const bool single_cta = []() {
-    const char *v = std::getenv("FLINT_SM100_SINGLE_CTA");
-    return v && v[0] == '1';
-  }();
-  g.force_single_cta = single_cta ? 1 : 0;
+  g.force_single_cta = gemm_single_cta_only() ? 1 : 0;
   // FLINT_SM100_NO_STREAM_K=1 keeps every tile whole (for A/B measurements and the parity tests
   // that compare the two schedules).
   const char *no_sk = std::getenv("FLINT_SM100_NO_STREAM_K");

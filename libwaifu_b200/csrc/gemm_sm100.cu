@@ -49,6 +49,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cstdlib>
 #include <mutex>
 
 #include "gemm_split_sm100.cuh"
@@ -1269,6 +1270,14 @@ int sm_count() {
     }
   }
   return cached;
+}
+
+bool gemm_single_cta_only() {
+  static const bool only = [] {
+    const char *v = std::getenv("FLINT_SM100_SINGLE_CTA");
+    return v && v[0] == '1';
+  }();
+  return only;
 }
 
 bool gemm_widens_bf16(int m, int n, int k) {

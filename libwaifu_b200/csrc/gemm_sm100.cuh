@@ -78,7 +78,7 @@ struct GemmArgs {
   int64_t out_ld;              // 0: pitch n
   int out_col0;
   uint32_t *status;            // device word, zeroed by the caller; non-zero after a failed wait
-  int force_single_cta;        // 1: never pair CTAs (for tests that compare the two forms)
+  int force_single_cta;        // 1: never pair CTAs (gemm_single_cta_only())
   // Workspace of the stream-K part of the schedule (the K stages of the last, partly filled rounds
   // dealt out evenly over all SMs); without one every tile is computed whole by one unit.
   // sk_partials: room for fp32 accumulator parts, gemm_stream_k_partial_floats() of them at most;
@@ -99,6 +99,11 @@ cudaError_t launch_gemm(const GemmArgs &args, const char **why);
 // Whether a product of bfloat16 rows and an e4m3 weight is taken as it is (few tiles), or wants the
 // weight widened to bfloat16 beforehand.
 bool gemm_widens_bf16(int m, int n, int k);
+
+// FLINT_SM100_SINGLE_CTA=1, read once: every GEMM on the persistent kernel, without CTA pairs (for A/B
+// measurements); bfloat16 rows against an e4m3 weight, where few tiles go to the one-round kernel without
+// a widened copy of the weight, still go there, in tiles of one CTA's rows.
+bool gemm_single_cta_only();
 
 // Number of SMs the persistent grid is sized for on the current device.
 int sm_count();

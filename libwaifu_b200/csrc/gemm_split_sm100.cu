@@ -686,7 +686,7 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
 // stages and the divided K of the other form win (300 x 2560 x 2048 15.9 and 16.9).
 SplitPlan gemm_pair_plan(GemmKind kind, int m, int n, int k, int sms) {
   SplitPlan best = {0, 0, false};
-  if ((kind != kGemmF16 && kind != kGemmBF16) || m <= kTileM) return best;
+  if ((kind != kGemmF16 && kind != kGemmBF16) || m <= kTileM || gemm_single_cta_only()) return best;
   float best_time;
   timed_plan(kind, 1, m, n, k, sms, true, &best_time);
   best_time *= kPairMargin;

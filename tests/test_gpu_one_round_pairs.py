@@ -1,6 +1,10 @@
 """GPU parity of the one-round kernel's tiles of 256 rows (fl_fp8_matmul[_add] on more than one row block
 against an e4m3 weight) with the oracle: every tile width, row counts that leave a pair's second CTA few
 rows or none, columns and K that end inside a tile and a stage. Tolerances as in test_gpu_one_round.py."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -44,3 +48,31 @@ def test_nan_codes_stay_nan_in_pairs(flint, oracle, is_bf16):
     y = oracle.widen(matmul(flint, a, codes, 0.0137, is_bf16), is_bf16)
     assert np.isnan(y[:, [3, 2700]]).all()
     assert np.isfinite(np.delete(y, [3, 2700], axis=1)).all()
+
+
+SINGLE = """
+import sys
+sys.path[:0] = sys.argv[1:3]
+import numpy as np
+from libwaifu_b200 import flint
+from oracle import oracle
+from helpers import check_parity, random_codes, randn
+from test_gpu_one_round import matmul
+from test_one_round_pairs_cpu import pairs
+rng = np.random.default_rng(4)
+for m, n, k in [(663, 2832, 1152), (1440, 2176, 1504)]:
+    for is_bf16 in (True, False):
+        assert pairs(int(is_bf16), m, n, k)["block_n"] == 0
+        a, codes = oracle.narrow(randn(rng, (m, k)), is_bf16), random_codes(rng, n, k)
+        got = matmul(flint, a, codes, 0.0137, is_bf16)
+        check_parity(oracle, got, oracle.fp8_matmul(a, codes, [np.float32(0.0137)], None, is_bf16), is_bf16, what=f"{m}x{n}x{k}")
+"""
+
+
+def test_products_that_have_pairs_run_without_them(flint):
+    """Under FLINT_SM100_SINGLE_CTA=1, on tiles of 128 rows and, the second shape, on the persistent kernel, for
+    which bfloat16 rows want the weight widened beforehand."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    assert all(pairs(kind, 1440, 2176, 1504)["block_n"] for kind in (0, 1))
+    subprocess.run([sys.executable, "-c", SINGLE, here, os.path.dirname(here)], env=dict(os.environ, FLINT_SM100_SINGLE_CTA="1"), check=True,
+                   timeout=300)

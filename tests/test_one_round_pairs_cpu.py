@@ -1,6 +1,9 @@
 """The one-round kernel's tiles of 256 rows (a pair of CTAs each), their index arithmetic without a GPU."""
 import ctypes
+import os
 import random
+import subprocess
+import sys
 
 import pytest
 
@@ -47,3 +50,13 @@ def test_refusals():
     for bad in [(2, 200, 8, 16, 148), (-1, 200, 8, 16, 148), (0, 0, 8, 16, 148), (0, 200, 8, 16, 1)]:
         assert F.lib().fl_sm100_one_round_pairs(*bad, out) == F.FL_ERROR_INVALID_ARG
     assert F.lib().fl_sm100_one_round_pairs(0, 200, 8, 16, 148, None) == F.FL_ERROR_INVALID_ARG
+
+
+def test_no_pairs_where_single_ctas_were_asked_for():
+    """FLINT_SM100_SINGLE_CTA=1, read when a process first asks: no tile of 256 rows, which pairs CTAs."""
+    script = ("import sys; sys.path[:0] = [%r, %r]; from test_one_round_pairs_cpu import pairs; "
+              "print([pairs(kind, 512, 5120, 3072)['block_n'] for kind in (0, 1)])"
+              % (os.path.dirname(os.path.abspath(__file__)), os.path.dirname(os.path.dirname(os.path.abspath(__file__)))))
+    said = [subprocess.run([sys.executable, "-c", script], env=dict(os.environ, FLINT_SM100_SINGLE_CTA=flag), check=True, capture_output=True,
+                           text=True).stdout.strip() for flag in ("1", "0")]
+    assert said == ["[0, 0]", "[160, 160]"]
