@@ -414,6 +414,12 @@ FLAPI int32_t fl_sm100_few_rows_plan(int32_t m, int32_t n, int32_t k, int32_t we
  * for a bad argument. */
 FLAPI int32_t fl_sm100_few_rows_route(int32_t entry, int32_t m, int32_t n, int32_t k);
 
+/* Whether fl_attention of this shape, mask and block size, on a device of `sms` SMs and with the environment's
+ * switches unset, runs on the form of its kernel in which a CTA goes on with pairs of query tiles whose
+ * own CTA has not started: 1 or 0; -1 for a bad argument. Host arithmetic only, no GPU needed. */
+FLAPI int32_t fl_sm100_attention_takes_over(int32_t batch, int32_t heads, int32_t q_len, int32_t kv_len, int32_t head_dim,
+                                            int32_t mask, int32_t block_size, int32_t sms);
+
 /* Which form of the persistent tile kernel a product of `kind` (0 half, 1 bfloat16, 2 e4m3, 3 nvfp4)
  * and shape runs on and how its tiles are dealt out over a device of `sms` SMs, where it runs there: a
  * product of few rows (fl_sm100_few_rows_route) or few tiles (fl_sm100_one_round_plan) may not.

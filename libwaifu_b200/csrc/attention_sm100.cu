@@ -29,9 +29,11 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
+#include "gemm_sm100.cuh"
 #include "ptx_sm100.cuh"
 
 namespace flsm100 {
@@ -654,9 +656,10 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 //
 // Runs of short walks take a second form of the kernel (attention2_units_kernel, below). The grid has a CTA
 // per unit (two tiles of one head's queries) there too, but a running CTA takes over units whose own
-// CTA has not started yet (clusterlaunchcontrol.try_cancel) instead of leaving its SM to it. Keys, values and queries of the next unit then arrive, and its first scores are computed, under
-// the last products and the output of the one before, and barriers and tensor memory are set up once
-// per SM. The hardware hands the units out in the grid's order, as it starts CTAs.
+// CTA has not started yet (clusterlaunchcontrol.try_cancel) instead of leaving its SM to it. Keys,
+// values and queries of the next unit then arrive, and its first scores are computed, under the last
+// products and the output of the one before, and barriers and tensor memory are set up once per SM. The
+// hardware hands the units out in the grid's order, as it starts CTAs.
 constexpr int kTiles = 2;
 constexpr int kTileWarps = 4;
 constexpr int kSoftmaxWarps2 = kTiles * kTileWarps;
@@ -678,13 +681,25 @@ static_assert(128 * kIssueRegs + kSoftmaxWarps2 * 32 * kSoftmaxRegs <= kThreads2
 template <int D>
 constexpr int kPartsOf = D == 128 ? 2 : 1;
 constexpr int kMaxSlots = 6;
-// The longest walks, in blocks of keys, whose CTA goes on with another unit, under the causal masks and
-// without one: 4 x 32 x 1000 causal 63.4 -> 57.4 us, 2 x 24 x 2048 causal at head_dim 64 60 -> 55, 2 x 24 x 300
-// at 64 13.4 -> 12.5, 3 x 24 x 1000 49.6 -> 49.4; but 24 x 2048 73.6 -> 74.5, 2 x 24 x 4352 398 -> 425, causal 347
-// both ways: what a block takes in that form is a little longer, and a long walk has little to hide. (One
-// kernel with the loop over units compiled out took 459 for the second shape among others of its kind,
-// the kernel without it 449.)
+// Where a CTA goes on with another unit, by the blocks of keys of the longest walk and the number of units (microseconds
+// back to back, the kernel of one unit and this one; SMs: 148). A block takes a little longer in that form, so it pays
+// where units follow one another on an SM, or where walks are so short that a unit's set-up is felt.
+//  * Up to 16 blocks under the causal masks and 8 without one. Above, 24 x 2048 73.6 -> 74.5, 2 x 24 x 4352 398 -> 425.
+//    (One kernel with the loop over units compiled out took 459 for the second shape among others of its kind, the kernel
+//    without it 449.)
+//  * At head_dim 64 all of these: 450 units of 2 to 16 blocks causal 34.9 -> 24.5 to 67.4 -> 58.0, 144 units 12.3 -> 9.7
+//    to 32.7 -> 32.2.
+//  * At 128 all walks up to 8 blocks (causal) or 4: 100 units causal 12.3 -> 11.2 to 22.6 -> 22.2, 450 43.5 -> 30.8 to
+//    59.7 -> 51.6.
+//  * Longer ones where few SMs have a unit: three in seven up to 12 blocks (48 units of 6 18.4 -> 16.7, 60 of 12 causal 28.7 ->
+//    27.8, but 63 of 14 31.5 -> 32.5, 80 of 8 22.5 -> 23.5), a third above (48 of 16 36.9 -> 35.7).
+//  * And where there is more than a unit an SM and the walks together are at least 0.8 of the longest on every SM: unmasked
+//    168 units of 8 43.2 -> 40.2, causal 224 of 16 44.8 -> 43.1, 300 59.7 -> 54.9. In between, the longest unit's own chain
+//    is what is waited for: unmasked 120 of 8 22.5 -> 24.2, causal 192 of 16 37.3 -> 41.8, 120 of 12 29.9 -> 31.4, block-causal
+//    120 of 16 (block 1900) 37.4 -> 40.5.
 constexpr int kTakeOverBlocksCausal = 16, kTakeOverBlocks = 8;
+constexpr int kAlwaysBlocksCausal = 8, kAlwaysBlocks = 4;
+constexpr int kFewUnitsBlocks = 12;
 
 struct Tail2 {
   uint4 claim;            // the answer to the last try_cancel
@@ -1199,7 +1214,7 @@ __device__ __forceinline__ int4 claimed_cta(const uint4 *answer) {
 template <int D>
 __global__ void __launch_bounds__(kThreads2, 1)
 attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                  const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
+                        const __grid_constant__ CUtensorMap tmap_vt, const KernelParams p) {
   using L = Layout2<D>;
   constexpr int S = L::kSlots;
   constexpr int kPParts = kPartsOf<D>;
@@ -1811,6 +1826,28 @@ size_t attention_scratch_bytes(int batch, int kv_heads, int kv_len, int head_dim
   return static_cast<size_t>(batch) * kv_heads * head_dim * round_up(kv_len, kPadKv) * 2;
 }
 
+bool attention_takes_over(const AttentionArgs &a, int sms) {
+  const bool causal = a.mask_type != 0 && !(a.mask_type >= 2 && a.block_size >= a.kv_len);  // (one block over every key is no mask)
+  const int longest = (a.kv_len + kBlockKv - 1) / kBlockKv;
+  if (longest > (causal ? kTakeOverBlocksCausal : kTakeOverBlocks)) return false;
+  if (a.head_dim == 64 || longest <= (causal ? kAlwaysBlocksCausal : kAlwaysBlocks)) return true;
+  const int64_t runs = static_cast<int64_t>(a.batch) * a.heads;
+  const int per_run = (a.q_len + kTiles * kBlockQ - 1) / (kTiles * kBlockQ);
+  const int64_t units = runs * per_run;
+  if (units * (longest <= kFewUnitsBlocks ? 7 : 9) <= sms * 3) return true;
+  if (units <= sms) return false;
+  int64_t walked = static_cast<int64_t>(per_run) * longest;  // by the units of one head
+  if (causal) {  // (the kernel's last_key_of of a unit's last query; kv_len is at most 2048 here, and no less than q_len)
+    walked = 0;
+    for (int u = 0; u < per_run; ++u) {
+      int last = std::min((u + 1) * kTiles * kBlockQ, a.q_len) - 1 + a.kv_len - a.q_len;
+      if (a.mask_type == 2) last = last / a.block_size * a.block_size + a.block_size - 1;
+      walked += (std::min(a.kv_len - 1, last) + kBlockKv) / kBlockKv;
+    }
+  }
+  return walked * runs * 5 >= static_cast<int64_t>(sms) * longest * 4;
+}
+
 AttentionPlan attention_plan(const AttentionArgs &a) {
   // Two tiles of queries per CTA where a head has more than one tile of them; the block diagonal
   // mask, whose tiles see different keys, and short query runs keep one tile per CTA.
@@ -1831,6 +1868,7 @@ AttentionPlan attention_plan(const AttentionArgs &a) {
   bool v_plain = true;
   for (int i = 0; i < 3; ++i) v_plain = v_plain && !(v_extent[i] > 1 && a.v_stride[i] == 0);
   plan.v_direct = plan.two_tiles && v_plain && !transposed_v_only;
+  plan.take_over = plan.two_tiles && attention_takes_over(a, sm_count());
   plan.launches = plan.v_direct ? 1 : 2;
   return plan;
 }
@@ -1919,7 +1957,7 @@ cudaError_t attention(const AttentionArgs &a, const char **why) {
     }
   }
   if (two_tiles) {
-    const bool take_over = (a.kv_len + kBlockKv - 1) / kBlockKv <= (kp.mask_type != 0 ? kTakeOverBlocksCausal : kTakeOverBlocks);
+    const bool take_over = plan.take_over;
     if (d == 64) return take_over ? launch2<64, true>(a, tq, tk, tvt, kp, why) : launch2<64, false>(a, tq, tk, tvt, kp, why);
     return take_over ? launch2<128, true>(a, tq, tk, tvt, kp, why) : launch2<128, false>(a, tq, tk, tvt, kp, why);
   }

@@ -37,9 +37,12 @@ size_t attention_scratch_bytes(int batch, int kv_heads, int kv_len, int head_dim
 struct AttentionPlan {
   bool two_tiles;
   bool v_direct;
+  bool take_over;  // (of the two-tile kernels) a CTA goes on with units whose own CTA has not started
   int launches;
 };
 AttentionPlan attention_plan(const AttentionArgs &a);
+// The plan's take_over on a device of `sms` SMs, by shape and mask alone.
+bool attention_takes_over(const AttentionArgs &a, int sms);
 // One launch where two tiles of queries share a CTA (more than 128 queries, any mask but the block
 // diagonal one, a v without repeated dimensions): v is read as it lies. Otherwise two: the
 // transposition of v into the scratch, and the one-tile kernel.

@@ -2581,6 +2581,23 @@ int32_t fl_sm100_few_rows_route(int32_t entry, int32_t m, int32_t n, int32_t k) 
   }
 }
 
+int32_t fl_sm100_attention_takes_over(int32_t batch, int32_t heads, int32_t q_len, int32_t kv_len, int32_t head_dim,
+                                      int32_t mask, int32_t block_size, int32_t sms) {
+  AttentionArgs a = {};
+  a.batch = batch;
+  a.heads = a.kv_heads = heads;
+  a.q_len = q_len;
+  a.kv_len = kv_len;
+  a.head_dim = head_dim;
+  a.mask_type = mask;
+  a.block_size = block_size;
+  const char *why = "";
+  if (batch < 1 || q_len < 1 || sms < 1) return -1;
+  for (int i = 0; i < 3; ++i) a.q_stride[i] = a.k_stride[i] = a.v_stride[i] = a.out_stride[i] = 8;
+  if (!attention_supported(a, &why)) return -1;
+  return attention_plan(a).two_tiles && attention_takes_over(a, sms) ? 1 : 0;
+}
+
 int32_t fl_sm100_gemm_plan(int32_t kind, int32_t m, int32_t n, int32_t k, int32_t sms, int32_t allow_stream_k, int32_t *plan) {
   return guard([&]() -> int32_t {
     if (!plan) invalid("plan is null");

@@ -104,6 +104,7 @@ def lib() -> ctypes.CDLL:
     L.fl_add.argtypes = [V, V, V, V]; L.fl_add.restype = c_int32
     L.fl_sm100_gemm_plan.argtypes = [c_int32] * 6 + [POINTER(c_int32)]; L.fl_sm100_gemm_plan.restype = c_int32
     L.fl_sm100_one_round_plan.argtypes = [c_int32] * 6 + [POINTER(c_int32)]; L.fl_sm100_one_round_plan.restype = c_int32
+    L.fl_sm100_attention_takes_over.argtypes = [c_int32] * 8; L.fl_sm100_attention_takes_over.restype = c_int32
     L.fl_sm100_one_round_pairs.argtypes = [c_int32] * 5 + [POINTER(c_int32)]; L.fl_sm100_one_round_pairs.restype = c_int32
     L.fl_sm100_selftest_wait_timeout.argtypes = [c_int32]; L.fl_sm100_selftest_wait_timeout.restype = c_int32
     L.fl_sm100_selftest_set_static_status.argtypes = [ctypes.c_uint32]; L.fl_sm100_selftest_set_static_status.restype = c_int32
