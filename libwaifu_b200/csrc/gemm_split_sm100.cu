@@ -45,8 +45,12 @@ constexpr int kMaxWideSlots = 4;
 constexpr int kATileBytes = kTileM * kStageRowBytes;
 constexpr int kSmemPerCta = 227 * 1024 - 1024;  // (static shared memory beside it)
 
-// A pair's estimate has to be this far below the other form's, or the persistent kernel's.
-constexpr float kPairMargin = 0.94f;
+// A pair's estimate has to be this far below the other form's, or the persistent kernel's. Half rows of a short
+// K in tiles above 128 columns are estimated too low by more: of 46 such shapes 14 lie between the two lines, and 13 of
+// them measured slower in pairs (1593 x 1696 x 816 14.0 us in tiles of 128 rows and 15.0 in pairs, 1553 x 1856 x 672 13.7
+// and 14.4, 569 x 4528 x 1088 15.9 and 16.6); below both lines 18.1 and 16.8 (2001 x 1632 x 1120).
+constexpr float kPairMargin = 0.94f, kPairMarginShortHalf = 0.9f;
+constexpr int kPairShortStages = 18;
 
 struct SplitParams {
   int m, n, num_kb;
@@ -687,15 +691,15 @@ SplitPlan gemm_split_plan(GemmKind kind, int b_is_e4m3, int m, int n, int k, int
 SplitPlan gemm_pair_plan(GemmKind kind, int m, int n, int k, int sms) {
   SplitPlan best = {0, 0, false};
   if ((kind != kGemmF16 && kind != kGemmBF16) || m <= kTileM || gemm_single_cta_only()) return best;
-  float best_time;
-  timed_plan(kind, 1, m, n, k, sms, true, &best_time);
-  best_time *= kPairMargin;
+  float other, best_time = 0.0f;
+  timed_plan(kind, 1, m, n, k, sms, true, &other);
   const int num_kb = (k * 2 + kStageRowBytes - 1) / kStageRowBytes;
   const int tiles_m = (m + 2 * kTileM - 1) / (2 * kTileM);
   for (int bn = 64; bn <= 256; bn += 32) {
     if (static_cast<long long>(tiles_m) * ((n + bn - 1) / bn) > sms / 2) continue;
     const float time = num_kb * (bn <= 192 ? 0.315f : 0.45f) + bn * 0.029f + (bn <= 192 ? 5.2f : 5.8f);
-    if (time < best_time) {
+    const bool short_half = kind == kGemmF16 && num_kb <= kPairShortStages && bn > 128;
+    if (time < other * (short_half ? kPairMarginShortHalf : kPairMargin) && (best.split == 0 || time < best_time)) {
       best_time = time;
       best = {bn, 1, true};
     }

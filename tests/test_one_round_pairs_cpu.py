@@ -60,3 +60,12 @@ def test_no_pairs_where_single_ctas_were_asked_for():
     said = [subprocess.run([sys.executable, "-c", script], env=dict(os.environ, FLINT_SM100_SINGLE_CTA=flag), check=True, capture_output=True,
                            text=True).stdout.strip() for flag in ("1", "0")]
     assert said == ["[0, 0]", "[160, 160]"]
+
+
+def test_half_rows_of_a_short_k_that_measured_slower_in_pairs():
+    """Either side of the second line, and bfloat16 rows of the same shapes, whose other ways take longer."""
+    for m, n, k in [(1593, 1696, 816), (1553, 1856, 672), (569, 4528, 1088), (1031, 2488, 1008), (423, 4936, 880), (1978, 1296, 1088)]:
+        assert pairs(0, m, n, k)["block_n"] == 0, (m, n, k)
+        assert pairs(1, m, n, k)["block_n"] > 128, (m, n, k)
+    for m, n, k in [(486, 4424, 1072), (234, 8840, 1136), (904, 2080, 1296), (2001, 1632, 1120), (689, 4472, 1008), (1940, 1648, 1344)]:
+        assert pairs(0, m, n, k)["block_n"] > 0, (m, n, k)
