@@ -217,7 +217,8 @@ __device__ __forceinline__ void widen_e4m3x4(uint32_t w, uint32_t &p01, uint32_t
 // instructions (never with QUANT).
 // W16: the weight itself is 16-bit (the unquantised linear layer of fl_matmul): no widening, eight
 // K positions per 16-byte piece instead of sixteen.
-template <bool QUANT, bool BF16, bool W16>
+// AHEAD: the first stages of the weight are asked for ahead of the kernel before.
+template <bool QUANT, bool BF16, bool W16, bool AHEAD>
 __global__ void __launch_bounds__(kThreads, 2) skinny_fp8_kernel(const SkinnyParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int x_bytes = (p.m * p.pitch_x + 127) / 128 * 128;
@@ -252,9 +253,8 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_fp8_kernel(const SkinnyPar
     fence_barrier_init();
   }
   // The weight of the CTA's first stages into L2 while the kernel ahead in the stream may still run: a
-  // prefetch writes nothing, and the copies below read what they would have read anyway (one row against
-  // 3072 x 3072 from HBM: 6.43 -> 6.36 us).
-  if (warp == kConsumerWarps) {
+  // prefetch writes nothing, and the copies below read what they would have read anyway (see kAheadBytes).
+  if (AHEAD && warp == kConsumerWarps) {
     int ahead = 0;
     for (int u = blockIdx.x; u < p.units && ahead < p.stages; u += gridDim.x) {
       const int row0 = u * unit_rows;
@@ -752,8 +752,8 @@ int pick_wn_log2(int k) {
   return slices >= 5 ? 0 : slices >= 3 ? 1 : slices == 2 ? 2 : 3;
 }
 
-template <bool QUANT, bool BF16, bool W16>
-cudaError_t launch(SkinnyParams &p, cudaStream_t stream) {
+template <bool QUANT, bool BF16, bool W16, bool AHEAD>
+cudaError_t launch_as(SkinnyParams &p, cudaStream_t stream) {
   constexpr int wbytes = W16 ? 2 : 1;
   constexpr int xbytes = QUANT ? 1 : 2;
   p.kb = p.k * wbytes;
@@ -779,7 +779,7 @@ cudaError_t launch(SkinnyParams &p, cudaStream_t stream) {
 #ifdef FLSM100_PROBE
   if (const char *v = std::getenv("FLSM100_PROBE")) p.probe = std::atoi(v);
 #endif
-  auto kernel = skinny_fp8_kernel<QUANT, BF16, W16>;
+  auto kernel = skinny_fp8_kernel<QUANT, BF16, W16, AHEAD>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
@@ -799,6 +799,19 @@ cudaError_t launch(SkinnyParams &p, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+// Weights from here on are asked for ahead. With more of them in rotation than L2 holds, as in a model's layers:
+// 1 x 3072 x 3072 7.65 -> 7.09 us (quantised rows 7.82 -> 7.42), 1 x 1536 x 4096 6.64 -> 6.40, 4 x 3072 x 8192 19.6 -> 18.9. The
+// instructions cost every launch some 0.2 us with quantised rows, which a weight already in L2 shows (1 x 3072 x 3072
+// 6.82 -> 7.06, with 16-bit rows 6.43 -> 6.38) and a small one wherever it lies: 1 x 2304 x 1536 3.87 -> 4.07, quantised 4.89 ->
+// 5.12, 3 x 2304 x 1536 quantised 5.1 -> 5.6. So they are compiled out below.
+constexpr long long kAheadBytes = 4 << 20;
+
+template <bool QUANT, bool BF16, bool W16>
+cudaError_t launch(SkinnyParams &p, cudaStream_t stream) {
+  const bool ahead = static_cast<long long>(p.n) * p.k * (W16 ? 2 : 1) >= kAheadBytes;
+  return ahead ? launch_as<QUANT, BF16, W16, true>(p, stream) : launch_as<QUANT, BF16, W16, false>(p, stream);
 }
 
 bool supported(int m, int n, int k, int wbytes, int xbytes, const void *x, const void *w, const void *out, bool has_residual) {

@@ -102,6 +102,24 @@ def test_few_rows(flint, oracle, m, n, k, is_bf16):
         check_parity(oracle, got, want, is_bf16, what=f"few rows {m}x{n}x{k} act={act} bias={bias} res={residual}")
 
 
+@pytest.mark.parametrize("m,n,kb", [(1, 2048, 2048), (3, 2040, 2048), (2, 1368, 3072), (2, 584, 7184)])
+@pytest.mark.parametrize("is_bf16", [True, False])
+def test_few_rows_either_side_of_the_weights_asked_for_ahead(flint, oracle, m, n, kb, is_bf16):
+    """4 MiB of weight (and 16 KB less, and a little more with a K in two pieces): quantised rows, 16-bit rows
+    against the same bytes, and a 16-bit weight of as many."""
+    F = flint
+    rng = np.random.default_rng(m + n + kb)
+    dt = F.DType.BFLOAT16 if is_bf16 else F.DType.FLOAT16
+    x, codes, scales, b, r = make_case(oracle, rng, m, n, kb, is_bf16, True, True)
+    check_parity(oracle, run(F, x, codes, scales, b, r, 1, is_bf16), oracle.fp8_linear(x, codes, scales, b, r, 1, is_bf16), is_bf16, what="linear")
+    got = F.fp8_matmul(dev(F, x, dt), dev(F, codes, F.DType.FP8E4M3), dev(F, np.array([0.0137], np.float32), F.DType.FLOAT)).numpy()
+    check_parity(oracle, got, oracle.fp8_matmul(x, codes, [np.float32(0.0137)], None, is_bf16), is_bf16, what="matmul")
+    a, w = x[:, :kb // 2].copy(), oracle.narrow(randn(rng, (n, kb // 2), 0.05), is_bf16)
+    want = oracle.epilogue(oracle.gemm_f32_nt(oracle.widen(a, is_bf16), oracle.widen(w, is_bf16)), out_is_bf16=is_bf16)
+    check_parity(oracle, F.linear_16(dev(F, a, dt), dev(F, w, dt)).numpy(), want, is_bf16, what="16-bit weight")
+    F.synchronize()
+
+
 @pytest.mark.parametrize("m,n,k", [(5, 3080, 2064), (32, 3072, 2048), (17, 4104, 4096), (4, 3072, 2304), (2, 8200, 2048),
                                    (16, 19080, 3072), (9, 3072, 12288)])
 @pytest.mark.parametrize("is_bf16", [True, False])
