@@ -418,21 +418,20 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   const uint32_t load_bytes = static_cast<uint32_t>(p.cpc * kStageK + kAtoms * x_atom);  // (bytes outside arrive as zeros)
-  auto load_w = [&](int st) {
-#pragma unroll
-    for (int a = 0; a < kAtoms; ++a) {
-      tma_load_2d(smem + (st % p.stages) * stage_bytes + a * kAtomBytes, &tmap_w, &full_bar[st % p.stages], st * kStageK + a * 128, n0);
-    }
-  };
   // Behind the rows' own quantiser, which lets this kernel start once everything ahead of it in the
   // stream is complete, only the rows have to be waited for: the ring's weight is on its way under the
-  // quantiser (2 x 18432 x 3072 in bfloat16, both launches, weight from HBM: 14.37 -> 13.93 us).
+  // quantiser (both launches, weight from HBM: 2 x 18432 x 3072 in bfloat16 14.2 -> 13.6 us, 4 x 3072 x 12288 18.6 ->
+  // 17.6). The producer has these stages' rows in a loop of their own: with a test of the stage in one
+  // loop, and the weight's loads ahead of the rows', the second shape took 19.0.
   const int early = p.weight_early ? min(num_stages, p.stages) : 0;
   if (warp == kQProducer && early > 0) {
     if (elect_one()) {
       for (int st = 0; st < early; ++st) {
         mbar_arrive_expect_tx(&full_bar[st], load_bytes);
-        load_w(st);
+#pragma unroll
+        for (int a = 0; a < kAtoms; ++a) {
+          tma_load_2d(smem + st * stage_bytes + a * kAtomBytes, &tmap_w, &full_bar[st], st * kStageK + a * 128, n0);
+        }
       }
     }
     __syncwarp();
@@ -443,19 +442,24 @@ fewrow_q8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (warp == kQProducer) {
     if (elect_one()) {
       bool ok = true;
-      for (int st = 0; st < num_stages && ok; ++st) {
-        const int s = st % p.stages;
-        if (st >= early) {
-          if (!mbar_wait(&empty_bar[s], ((st / p.stages) & 1) ^ 1, &abort_flag)) {
-            ok = false;
-            break;
-          }
-          mbar_arrive_expect_tx(&full_bar[s], load_bytes);
-          load_w(st);
-        }
+      for (int st = 0; st < early; ++st) {
 #pragma unroll
         for (int a = 0; a < kAtoms; ++a) {
-          tma_load_2d(smem + s * stage_bytes + kRawWBytes + a * x_atom, &tmap_x, &full_bar[s], st * kStageK + a * 128, 0);
+          tma_load_2d(smem + st * stage_bytes + kRawWBytes + a * x_atom, &tmap_x, &full_bar[st], st * kStageK + a * 128, 0);
+        }
+      }
+      for (int st = early; st < num_stages && ok; ++st) {
+        const int s = st % p.stages;
+        if (!mbar_wait(&empty_bar[s], ((st / p.stages) & 1) ^ 1, &abort_flag)) {
+          ok = false;
+          break;
+        }
+        uint8_t *base = smem + s * stage_bytes;
+        mbar_arrive_expect_tx(&full_bar[s], load_bytes);
+#pragma unroll
+        for (int a = 0; a < kAtoms; ++a) {
+          tma_load_2d(base + a * kAtomBytes, &tmap_w, &full_bar[s], st * kStageK + a * 128, n0);
+          tma_load_2d(base + kRawWBytes + a * x_atom, &tmap_x, &full_bar[s], st * kStageK + a * 128, 0);
         }
       }
       if (!ok) {
