@@ -64,7 +64,6 @@ constexpr int kRowBytes = 128;          // bytes of K per operand row per stage
 constexpr int kMmaKBytes = 32;          // bytes of K one tcgen05.mma consumes per row
 constexpr int kMmasPerStage = kRowBytes / kMmaKBytes;
 constexpr int kSfTileBytes = 512;       // 128 rows x 4 scale factors
-constexpr int kSfSets = 3;              // of scale factors in tensor memory
 constexpr int kNumWarps = 12;
 constexpr int kNumThreads = kNumWarps * 32;
 constexpr int kMaxEpilogueWarps = 8;
@@ -245,17 +244,17 @@ struct Config : Roles<B8> {
   static constexpr int kColParamOffset = kOutStageOffset + kOutStageBytes;
   static constexpr int kSmemBytes = kColParamOffset + kColParamBytes + 1024;  // + slack to align to 1024
   static_assert(kStageBytes % 512 == 0, "the output staging behind the stages has to stay 512-byte aligned");
-  // Tensor memory columns: two accumulators, then three sets of one stage's scale factors, which the
-  // MMA thread copies there ahead of the stage's MMAs: both run in the order of their issue, so nothing
-  // is handed over (a copying thread of its own, with a commit and a wait in both directions for every
-  // set, took 82.4 us for the whole of 4352 x 9216 x 3072, this 78.6).
+  // Tensor memory columns: two accumulators, then one stage's scale factors, which the MMA thread copies
+  // there ahead of the stage's MMAs: both run in the order of their issue, so nothing is handed over (a
+  // copying thread of its own, with a commit and a wait in both directions for every one of three sets,
+  // took 82.4 us for the whole of 4352 x 9216 x 3072, this 78.6), and one set is as good as three (83.4 us with
+  // three and 83.5 with one among others of its kind, 512 x 1280 x 1024 10.54 and 10.34).
   static constexpr int kAccCols = 2 * BLOCK_N;
   static constexpr int kSfaCols = NVF4 ? kMmasPerStage * 4 : 0;
   static constexpr int kSfbColsPerMma = NVF4 ? BLOCK_N / 32 : 0;
   static constexpr int kSfbCols = kMmasPerStage * kSfbColsPerMma;
   static_assert(kSfbCols == 4 * kSfbCopies, "a copy fills four columns");
-  static constexpr int kSfSetCols = kSfaCols + kSfbCols;
-  static constexpr int kUsedCols = kAccCols + kSfSets * kSfSetCols;
+  static constexpr int kUsedCols = kAccCols + kSfaCols + kSfbCols;
   static constexpr int kTmemCols = kUsedCols <= 32 ? 32 : kUsedCols <= 64 ? 64 : kUsedCols <= 128 ? 128
                                    : kUsedCols <= 256 ? 256 : 512;
   static_assert(kUsedCols <= 512, "tensor memory holds 512 columns");
@@ -526,8 +525,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       (void)sfa_desc0;
       (void)sfb_desc0;
       (void)kSfTileStep;
-      uint32_t sf_set = 0;  // NVFP4: the next stage's set of scale factors, over all tiles
-      (void)sf_set;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -553,7 +550,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint64_t adesc = adesc0 + stage * kStageStep;
           const uint64_t bdesc = bdesc0 + stage * kStageStep;
           if constexpr (NVF4) {
-            const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols + sf_set * Cfg::kSfSetCols;
+            const uint32_t sfa_tmem = tmem_base + Cfg::kAccCols;
             const uint32_t sfb_tmem = sfa_tmem + Cfg::kSfaCols;
             // Copies and multiplications issued by one thread run in the order they were issued.
             const uint64_t sfa_desc = sfa_desc0 + stage * kStageStep;
@@ -591,7 +588,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
           }
           commit_to(&empty_bar[stage]);
-          if (NVF4 && ++sf_set == kSfSets) sf_set = 0;
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
