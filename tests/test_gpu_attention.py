@@ -226,3 +226,42 @@ def test_more_units_than_the_gpu_holds_with_one_block_each(flint, oracle):
     q, k, v = make(oracle, rng, 2, 96, 96, 200, 77, 64, False)
     got = run(flint, q, k, v, False, False)
     check(oracle, got, oracle.attention(q, k, v, False, False), False, "one block")
+
+
+def goes_on(flint, n, h, L, S, d, mask, block=0):
+    import torch
+    return flint.lib().fl_sm100_attention_takes_over(n, h, L, S, d, mask, block, torch.cuda.get_device_properties(0).multi_processor_count) == 1
+
+
+@pytest.mark.parametrize("n,h,hk,L,S,d,block", [
+    (1, 150, 2, 600, 700, 128, 200),  # blocks of keys that end inside a tile: the tiles of a unit end apart by none, one or two
+    (2, 80, 80, 520, 600, 64, 300),   # wider than two tiles of keys
+    (1, 200, 40, 300, 300, 128, 64),
+    (1, 75, 15, 1100, 1100, 64, 520),
+    (1, 160, 16, 515, 1300, 128, 700),  # a longer walk, on a full GPU
+])
+@pytest.mark.parametrize("is_bf16", [True, False])
+def test_more_units_than_the_gpu_holds_block_causal(flint, oracle, n, h, hk, L, S, d, block, is_bf16):
+    assert goes_on(flint, n, h, L, S, d, flint.MaskType.BLOCK_CAUSAL, block)
+    rng = np.random.default_rng(L + S + h + block)
+    q, k, v = make(oracle, rng, n, h, hk, L, S, d, is_bf16)
+    got = run(flint, q, k, v, 2, is_bf16, block)
+    check(oracle, got, oracle.attention(q, k, v, 2, is_bf16, block), is_bf16, f"{(n, h, hk, L, S, d)} block {block}")
+
+
+@pytest.mark.parametrize("n,h,hk,L,S,d", [(2, 90, 90, 300, 300, 64), (3, 60, 12, 257, 400, 128)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_more_units_than_the_gpu_holds_with_a_v_that_repeats(flint, oracle, n, h, hk, L, S, d, causal):
+    """v shared by the batch rows through a stride of 0: read through its transposition, and still unit after unit."""
+    F = flint
+    assert goes_on(F, n, h, L, S, d, int(causal))
+    rng = np.random.default_rng(L + S + h)
+    q, k, v = make(oracle, rng, n, h, hk, L, S, d, True)
+    bf = F.DType.BFLOAT16
+    tq, tk = (F.Tensor.from_numpy(t, bf, F.Device.CUDA) for t in (q, k))
+    shared = F.Tensor.from_numpy(v[:1].copy(), bf, F.Device.CUDA).view_as((n, hk, S, d), (0, S * d, d, 1))
+    before = F.launch_count()
+    got = F.attention(tq, tk, shared, int(causal), 0).numpy()
+    assert F.launch_count() == before + 2
+    F.synchronize()
+    check(oracle, got, oracle.attention(q, k, np.repeat(v[:1], n, axis=0), causal, True), True, f"{(n, h, hk, L, S, d)} causal={causal}")

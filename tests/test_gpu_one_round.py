@@ -2,8 +2,9 @@
 the CPU oracle: one row and one column block and their remainders, K in one piece and divided over
 clusters of two, four and eight, K of an odd number of stages, a result no 16-byte store can write,
 every term of the epilogue, and the weight's NaN codes. Each shape's cut (tile width, CTAs of a cluster)
-stands beside it and is asserted, so that a change of the rule cannot empty the test. Half rows that the
-few-row kernels take are left out; bfloat16 ones are in where a rule sends them here."""
+stands beside it and is asserted, and that it has none into tiles of 256 rows, so that a change of a
+rule cannot empty the test. Half rows that the few-row kernels take are left out; bfloat16 ones are in where a
+rule sends them here."""
 import ctypes
 
 import numpy as np
@@ -28,17 +29,22 @@ def matmul(F, a, codes, scale, is_bf16, addend=None):
 
 
 def cut(F, kind, m, n, k):
-    """(tile width, CTAs of a cluster) of a product of half (0), bfloat16 (1) or quantised (2) rows on this card."""
+    """(tile width, CTAs of a cluster) of a product of half (0), bfloat16 (1) or quantised (2) rows on this card, in
+    tiles of 128 rows, which have to be the ones it runs on."""
     import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     out = (ctypes.c_int32 * 8)()
-    F.check(F.lib().fl_sm100_one_round_plan(kind, m, n, k, torch.cuda.get_device_properties(0).multi_processor_count, 1, out))
+    if kind < 2:
+        F.check(F.lib().fl_sm100_one_round_pairs(kind, m, n, k, sms, out))
+        assert out[0] == 0, "goes to tiles of 256 rows"
+    F.check(F.lib().fl_sm100_one_round_plan(kind, m, n, k, sms, 1, out))
     return out[0], out[1]
 
 
 CUTS = {(77, 2560, 2048): (128, 4), (65, 1288, 640): (32, 2), (127, 136, 272): (32, 2), (128, 1280, 656): (32, 2), (129, 1304, 1040): (64, 2),
-        (300, 1280, 640): (64, 2), (512, 5120, 784): (144, 1), (1000, 1280, 1280): (160, 2), (70, 264, 4096): (128, 8), (130, 72, 12288): (128, 8)}
+        (300, 1280, 640): (64, 2), (131, 9528, 288): (144, 1), (1000, 1280, 1280): (160, 2), (70, 264, 4096): (128, 8), (130, 72, 12288): (128, 8)}
 SHAPES = [(77, 2560, 2048), (65, 1288, 640), (127, 136, 272), (128, 1280, 656), (129, 1304, 1040), (300, 1280, 640),
-          (512, 5120, 784), (1000, 1280, 1280), (70, 264, 4096), (130, 72, 12288)]
+          (131, 9528, 288), (1000, 1280, 1280), (70, 264, 4096), (130, 72, 12288)]
 
 
 @pytest.mark.parametrize("m,n,k", SHAPES)
@@ -56,7 +62,7 @@ def test_matmul(flint, oracle, m, n, k, is_bf16, addend):
 
 @pytest.mark.parametrize("m,n,k,width,split", [(129, 11880, 272, 176, 1), (257, 8712, 272, 192, 1), (65, 11880, 1616, 192, 2),
                                                (129, 2376, 2064, 192, 4), (257, 10296, 272, 224, 1), (129, 7128, 1616, 224, 2),
-                                               (257, 11880, 272, 256, 1), (129, 9064, 1616, 256, 2)])
+                                               (257, 11880, 272, 256, 1), (269, 6056, 1488, 256, 2)])
 @pytest.mark.parametrize("is_bf16", [False, True])
 def test_matmul_in_wide_tiles(flint, oracle, m, n, k, width, split, is_bf16):
     assert cut(flint, int(is_bf16), m, n, k) == (width, split)

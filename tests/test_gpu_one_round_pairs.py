@@ -1,6 +1,7 @@
 """GPU parity of the one-round kernel's tiles of 256 rows (fl_fp8_matmul[_add] on more than one row block
-against an e4m3 weight) with the oracle: every tile width, row counts that leave a pair's second CTA few
-rows or none, columns and K that end inside a tile and a stage. Tolerances as in test_gpu_one_round.py."""
+against an e4m3 weight) with the oracle: every tile width that the rule takes, row counts that leave a pair's
+second CTA few rows or none, columns and K that end inside a tile and a stage. Each shape's width stands beside
+it and is asserted. Tolerances as in test_gpu_one_round.py."""
 import os
 import subprocess
 import sys
@@ -14,9 +15,12 @@ from test_one_round_pairs_cpu import pairs
 
 pytestmark = pytest.mark.gpu
 
-# every width, and what it is taken at
-CASES = [(663, 2832, 1152, 128), (129, 8632, 2704, 128), (512, 5120, 3072, 160), (1705, 1400, 3696, 160), (238, 14088, 2304, 192),
-         (385, 7048, 3088, 192), (256, 16384, 3072, 224)]
+# m, n, k, and the tile width for half and for bfloat16 rows (0: no tiles of 256 rows, and the case is left out). The
+# last five leave the second CTA of the last row block without a row.
+CASES = [(396, 3496, 1312, 96, 96), (663, 2832, 1152, 128, 128), (129, 8632, 2704, 128, 128), (512, 5120, 3072, 160, 160),
+         (1705, 1400, 3696, 160, 160), (238, 14088, 2304, 192, 192), (385, 7048, 3088, 192, 192), (256, 16384, 3072, 0, 224),
+         (399, 9096, 272, 0, 256), (1299, 1528, 1120, 128, 128), (1284, 1888, 944, 160, 160), (1293, 2296, 464, 192, 192),
+         (1320, 2304, 288, 0, 192), (778, 4528, 1168, 0, 256)]
 
 
 def sms():
@@ -24,12 +28,10 @@ def sms():
     return torch.cuda.get_device_properties(0).multi_processor_count
 
 
-@pytest.mark.parametrize("m,n,k,width", CASES)
-@pytest.mark.parametrize("is_bf16", [False, True])
+@pytest.mark.parametrize("m,n,k,width,is_bf16", [(*c[:3], c[3 + is_bf16], bool(is_bf16)) for c in CASES for is_bf16 in (0, 1) if c[3 + is_bf16]])
 @pytest.mark.parametrize("addend", ["none", "bias", "residual"])
 def test_matmul_in_pairs(flint, oracle, m, n, k, width, is_bf16, addend):
-    if pairs(1, m, n, k, sms())["block_n"] != width or (not is_bf16 and pairs(0, m, n, k, sms())["block_n"] == 0):
-        pytest.skip("not taken on this card")
+    assert pairs(int(is_bf16), m, n, k, sms())["block_n"] == width
     rng = np.random.default_rng(m + n + k)
     a = oracle.narrow(randn(rng, (m, k)), is_bf16)
     codes = random_codes(rng, n, k)

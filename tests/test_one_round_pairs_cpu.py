@@ -35,7 +35,7 @@ def test_pair_invariants(kind, sms):
         taken += 1
         what = f"{m}x{n}x{k} {p}"
         half = p["block_n"] // 2
-        assert m > 128 and p["split"] == 1 and 32 <= p["block_n"] <= 256 and p["block_n"] % 32 == 0, what
+        assert m > 128 and p["split"] == 1 and 64 <= p["block_n"] <= 256 and p["block_n"] % 32 == 0, what
         assert p["num_kb"] == -(-k * 2 // 128)
         assert p["ctas"] == -(-m // 256) * -(-n // p["block_n"]) * 2 and p["ctas"] <= sms, what
         assert p["slot_bytes"] == 128 * 128 + half * 64 and p["slot_bytes"] % 1024 == 0 and half * 128 % 1024 == 0, what
