@@ -143,26 +143,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Two floats in one 64-bit register, for the two-wide float instructions of sm_100.
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float *lo, float *hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // 2^x for a pair of exponents x <= 2^kRescaleStep's, without the special-function unit: that unit
 // delivers 16 results a cycle and SM, so the 128 x 128 exponentials of a block would hold it for
 // 1024 cycles; one pair in four of a row goes through here instead, on the multiply-add pipes

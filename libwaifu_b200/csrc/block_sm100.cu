@@ -27,26 +27,7 @@ __device__ __forceinline__ uint16_t narrow(float v, int is_bf16) {
 constexpr int kUnits = 2;
 constexpr int kMaxWarps = 16;
 
-// Two float32 values in one 64-bit register and instructions that work on both lanes at once, each
-// lane rounded as the scalar instruction rounds it: this kernel is bound by instruction issue.
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float *lo, float *hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
+// (The kernel below is bound by instruction issue: two-wide float instructions halve the arithmetic's.)
 __device__ __forceinline__ uint64_t bf16x2_widen(uint32_t w) {
   return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }

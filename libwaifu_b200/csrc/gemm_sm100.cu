@@ -275,33 +275,9 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi, int is_bf16) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
-// Two floats in one 64-bit register, and the two-wide float instructions of sm_100: each half is rounded as
-// the scalar instruction rounds it, at half the issue slots: the epilogue, and not the main loop under it, is
-// what a tile of a short K waits for (4352 x 12288 x 3072 with bias and GELU 141 -> 134 us, 4096 x 3072 x 3072
-// with bias 36.4 -> 34.9, quantised rows; the same bits).
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float *lo, float *hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
+// The epilogue works on pairs of columns: it, and not the main loop under it, is what a tile of a short K waits
+// for (4352 x 12288 x 3072 with bias and GELU 141 -> 134 us, 4096 x 3072 x 3072 with bias 36.4 -> 34.9, quantised
+// rows; the same bits).
 // gelu_tanh of both halves, the same operations in the same order.
 __device__ __forceinline__ uint64_t f2_gelu_tanh(uint64_t x) {
   constexpr float kC0 = -2.0f * 0.7978845608028654f * 1.4426950408889634f;

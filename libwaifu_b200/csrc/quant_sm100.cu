@@ -375,32 +375,8 @@ __global__ void __launch_bounds__(THREADS) ln_modulate_quantize_reg_kernel(const
   }
 }
 
-// Two float32 values in one 64-bit register and the instructions that work on both lanes at once
-// (each lane rounded to nearest even exactly as the scalar instruction rounds it): the row kernels
-// are bound by instruction issue, not by memory, and these halve the arithmetic's instructions.
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float *lo, float *hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
+// The row kernels for bfloat16 are bound by instruction issue, not by memory: two-wide instructions
+// halve the arithmetic's.
 // The two bfloat16 of a 32-bit word, widened: the low one in the low lane.
 __device__ __forceinline__ uint64_t bf16x2_widen(uint32_t w) {
   return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
