@@ -718,6 +718,229 @@ struct Layout2 {
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
 
+// Two tiles of 128 queries of one head and the blocks of keys they walk, from the first on (of the
+// masks only the block diagonal one hides a run's first keys, and it is not served here).
+struct Unit2 {
+  int head, batch, q0;
+  int num_blocks;
+  int blocks[kTiles];  // how many of them each tile walks: 0 for a tile past the last query
+
+  // Without a mask the units of one head run side by side and share its keys and values in L2. Under
+  // the causal masks the later queries have more keys to walk: the last unit of every head goes first,
+  // then the one before it, so that the grid ends on the short ones whatever the head.
+  __device__ __forceinline__ Unit2(const KernelParams &p, int x, int y, int z) : head(y), batch(z) {
+    int unit = x;
+    if (p.mask_type != 0) {
+      const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
+      const int order = x + units * (y + heads * z);
+      unit = units - 1 - order / all;
+      head = order % all % heads;
+      batch = order % all / heads;
+    }
+    q0 = unit * (kTiles * kBlockQ);
+    const int offset = p.kv_len - p.q_len;
+    const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
+    num_blocks = (last_key_of(p, last_row + offset) + kBlockKv) / kBlockKv;
+    // Under the causal masks the first tile's queries see nothing of the last blocks the second walks.
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) {
+      const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
+      blocks[i] = q0 + i * kBlockQ >= p.q_len ? 0 : min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv);
+    }
+  }
+};
+
+// What the two kernels below share: a block's softmax, a row's output and the instructions of the products. They
+// differ in how they walk: one unit, or one after another.
+
+// Block j of the keys for one query (a lane's row of the tile): its scores from tensor memory, the running
+// maximum and sum, and the probabilities back into tensor memory, part by part. The row sees keys up to
+// `key_last`, every row of the tile those up to `common_last`.
+template <int D>
+__device__ __forceinline__ void softmax_block(const KernelParams &p, uint32_t t_scores, uint32_t t_out, int j, int common_last,
+                                              int key_last, uint64_t *p_full_bar, uint32_t lane, float *m_used_io,
+                                              float *l_run_io) {
+  constexpr int kPParts = kPartsOf<D>;
+  constexpr int kChunks = kBlockKv / 32;
+  static_assert(kChunks == 4, "four chunks of scores pack into the first two");
+  constexpr float kRescaleStep = 8.0f;
+  float m_used = *m_used_io, l_run = *l_run_io;
+  uint32_t sc[kChunks][32];  // the row's scores of the block, in one round trip
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
+  const int block_key0 = j * kBlockKv;
+  const bool edge = block_key0 + kBlockKv - 1 > common_last;
+  float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (edge) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        if (block_key0 + c * 32 + i > key_last) sc[c][i] = __float_as_uint(-INFINITY);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
+    }
+  }
+  const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+  if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
+    const float m_new = fmaxf(m_used, m_blk);
+    const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
+    l_run *= alpha;
+    if (j > 0) {
+#pragma unroll 1
+      for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
+        uint32_t v[16];
+        tmem_ld_32x16(t_out + c * 16, v);
+        tmem_ld_wait(v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+        tmem_st_32x16(t_out + c * 16, v);
+      }
+    }
+    m_used = m_new;
+  }
+  const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
+  // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
+  // (a slot whose scores have been used by then).
+  const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
+  uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
+  auto emit = [&](auto bf16_tag, int part) {
+    constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
+#pragma unroll
+    for (int h = 0; h < kChunks / kPParts; ++h) {
+      const int c = part * (kChunks / kPParts) + h;
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
+        float e0, e1;
+        if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
+          float x0, x1;
+          f2_unpack(x, &x0, &x1);
+          e0 = fast_exp2(x0);
+          e1 = fast_exp2(x1);
+        } else {
+          exp2_pair_poly(x, &e0, &e1);
+        }
+        sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
+        sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
+      }
+    }
+  };
+  // Each half of the block's keys is handed over as soon as it is there: its product runs under
+  // the exponentials of the other half.
+#pragma unroll
+  for (int part = 0; part < kPParts; ++part) {
+    if (p.is_bf16) {
+      emit(std::true_type{}, part);
+    } else {
+      emit(std::false_type{}, part);
+    }
+    tmem_st_32x32(t_scores + part * 32, sc[part]);
+    if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
+    tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
+    tc_fence_before_sync();  // before the MMAs that the hand-over starts
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&p_full_bar[part]);
+  }
+  float s0, s1, s2, s3;
+  f2_unpack(sums[0], &s0, &s1);
+  f2_unpack(sums[1], &s2, &s3);
+  l_run += (s0 + s1) + (s2 + s3);
+  *m_used_io = m_used;
+  *l_run_io = l_run;
+}
+
+// A finished row of a tile's output, divided by the sum of its probabilities.
+template <int D>
+__device__ __forceinline__ void store_output(const KernelParams &p, uint32_t t_out, float l_run, bool live, uint16_t *dst) {
+  const float inv = 1.0f / l_run;
+#pragma unroll 1
+  for (int c = 0; c < D / 32; ++c) {
+    uint32_t v[32];
+    tmem_ld_32x32(t_out + c * 32, v);
+    tmem_ld_wait(v);
+    if (live) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        uint4 w;
+        w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
+        w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
+        w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
+        w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
+        *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
+      }
+    }
+  }
+}
+
+// The instructions of a tile's two products. The whole warp calls, the elected lane issues.
+template <int D>
+struct TileMmas {
+  using L = Layout2<D>;
+  static constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
+  static constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
+  static constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
+  static constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
+  uint32_t tmem_base, idesc_s, idesc_o, idesc_o_mn;
+  uint64_t qdesc0, mn_fields;
+  bool issuer, v_direct;
+
+  // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes on, the
+  // operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64 head_dim positions
+  // lie a 128-key atom apart.
+  __device__ __forceinline__ TileMmas(const KernelParams &p, uint32_t tmem, uint32_t q_smem, bool elected)
+      : tmem_base(tmem), qdesc0(umma_desc_sw128(q_smem)),
+        mn_fields(umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0)), issuer(elected), v_direct(p.v_direct != 0) {
+    const uint32_t fmt = p.is_bf16 ? 1u : 0u;
+    idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
+    idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
+    idesc_o_mn = idesc_o | (1u << 16);
+  }
+
+  __device__ __forceinline__ void scores(int i, uint64_t kd) const {  // S_i = Q_i K^T
+    const uint32_t s_tmem = tmem_base + i * L::kSCols;
+    const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
+#pragma unroll
+    for (int m = 0; m < kScoreMmas; ++m) {
+      const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+      const uint64_t qa = qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep);
+      const uint64_t ka = kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep);
+      if (issuer) umma_ss<kKindF16>(s_tmem, qa, ka, idesc_s, m != 0 ? 1u : 0u);
+    }
+  }
+
+  // O_i += P_i V over one part of the block's keys
+  __device__ __forceinline__ void product(int i, int part, uint64_t vd, uint32_t first_block) const {
+    const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
+    const uint32_t p_tmem = tmem_base + i * L::kSCols;
+    constexpr int kPartMmas = kOutMmas / kPartsOf<D>;
+    if (v_direct) {
+#pragma unroll
+      for (int k = 0; k < kPartMmas; ++k) {
+        const int m = part * kPartMmas + k;
+        const uint64_t va = (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4));
+        if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, va, idesc_o_mn, m != 0 ? 1u : (first_block ^ 1u));
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPartMmas; ++k) {
+        const int m = part * kPartMmas + k;
+        const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
+        if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
+                    m != 0 ? 1u : (first_block ^ 1u));
+      }
+    }
+  }
+};
+
 template <int D>
 __global__ void __launch_bounds__(kThreads2, 1)
 attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -735,34 +958,8 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (threadIdx.x == 0) atomicCAS(p.status, 0u, kStatusAttentionLayout);
     return;
   }
-  // A unit is a CTA's two tiles. Without a mask the units of one head run side by side and share its
-  // keys and values in L2. Under the causal masks the later queries have more keys to walk: the last
-  // unit of every head goes first, then the one before it, so that the grid ends on the short ones
-  // whatever the head.
-  int unit = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
-  if (p.mask_type != 0) {
-    const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
-    const int order = unit + units * (head + heads * batch);
-    unit = units - 1 - order / all;
-    head = order % all % heads;
-    batch = order % all / heads;
-  }
-  const int q0 = unit * (kTiles * kBlockQ);
-  const int kv_head = head / p.group;
+  const Unit2 u(p, blockIdx.x, blockIdx.y, blockIdx.z);
   const int offset = p.kv_len - p.q_len;
-  // Both tiles start at the first block of keys that some query of the CTA sees.
-  const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
-  const int kv_begin = first_key_of(p, q0 + offset);
-  const int kv_end = last_key_of(p, last_row + offset) + 1;
-  const int block0 = kv_begin / kBlockKv;
-  const int num_blocks = (kv_end + kBlockKv - 1) / kBlockKv - block0;
-  // Under the causal masks the first tile's queries see nothing of the last blocks the second walks;
-  // a tile past the last query has none.
-  auto blocks_of = [&](int i) -> int {
-    if (q0 + i * kBlockQ >= p.q_len) return 0;
-    const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
-    return min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv - block0);
-  };
 
   if (threadIdx.x == 0) {
     t.abort_flag = 0;
@@ -801,122 +998,25 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // ------------------------------------------------------------------ softmax and output
     const int tile = static_cast<int>(warp >> 2);
     const uint32_t quarter = warp & 3;
-    const int tq0 = q0 + tile * kBlockQ;  // the tile's first query
+    const int tq0 = u.q0 + tile * kBlockQ;  // the tile's first query
     const int row = static_cast<int>(quarter) * 32 + static_cast<int>(lane);
-    const int q_pos = tq0 + row + offset;
-    const int key_first = first_key_of(p, q_pos), key_last = last_key_of(p, q_pos);
-    const int tile_last_row = min(tq0 + kBlockQ, p.q_len) - 1;
-    // What every query of the tile sees (an empty range for a tile past the last query: every block
-    // is then an edge block, and nothing of it is stored).
-    const int common_first = first_key_of(p, tile_last_row + offset), common_last = last_key_of(p, tq0 + offset);
+    const int key_last = last_key_of(p, tq0 + row + offset);
+    const int common_last = last_key_of(p, tq0 + offset);  // what every query of the tile sees
     const uint32_t t_lane = tmem_base + ((quarter * 32u) << 16);
     const uint32_t t_scores = t_lane + tile * L::kSCols;  // the row's 128 scores, then its 128 probabilities in 64 columns
     const uint32_t t_out = t_lane + L::kOCol + tile * D;
-    constexpr int kChunks = kBlockKv / 32;
-    static_assert(kChunks == 4, "four chunks of scores pack into the first two");
-    constexpr float kRescaleStep = 8.0f;
     float m_used = -INFINITY;
     float l_run = 0.0f;
     bool ok = true;
-    uint32_t sc[kChunks][32];
 
-    const int my_blocks = blocks_of(tile);
+    const int my_blocks = tile == 0 ? u.blocks[0] : u.blocks[1];
     for (int j = 0; j < my_blocks && ok; ++j) {
-      // The row's scores of the block into registers in one round trip. (Scores of block j are
-      // issued behind the product of block j - 1: once they are here the tile's output is complete
-      // up to that block.)
+      // (Scores of block j are issued behind the product of block j - 1: once they are here the tile's
+      // output is complete up to that block.)
       ok = __all_sync(0xffffffffu, mbar_wait(&t.s_full_bar[tile], j & 1, &abort_flag));
       if (!ok) break;
       tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
-      const int block_key0 = (block0 + j) * kBlockKv;
-      const bool edge = block_key0 < common_first || block_key0 + kBlockKv - 1 > common_last;
-      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (edge) {
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = block_key0 + c * 32 + i;
-            if (key > key_last || key < key_first) sc[c][i] = __float_as_uint(-INFINITY);
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
-        }
-      }
-      const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
-      if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
-        const float m_new = fmaxf(m_used, m_blk);
-        const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
-        l_run *= alpha;
-        if (j > 0) {
-#pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
-            uint32_t v[16];
-            tmem_ld_32x16(t_out + c * 16, v);
-            tmem_ld_wait(v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x16(t_out + c * 16, v);
-          }
-        }
-        m_used = m_new;
-      }
-      const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
-      // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
-      // (a slot whose scores have been used by then).
-      const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
-      uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
-      auto emit = [&](auto bf16_tag, int part) {
-        constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
-#pragma unroll
-        for (int h = 0; h < kChunks / kPParts; ++h) {
-          const int c = part * (kChunks / kPParts) + h;
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
-            float e0, e1;
-            if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
-              float x0, x1;
-              f2_unpack(x, &x0, &x1);
-              e0 = fast_exp2(x0);
-              e1 = fast_exp2(x1);
-            } else {
-              exp2_pair_poly(x, &e0, &e1);
-            }
-            sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
-            sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
-          }
-        }
-      };
-      // Each half of the block's keys is handed over as soon as it is there: its product runs under
-      // the exponentials of the other half.
-#pragma unroll
-      for (int part = 0; part < kPParts; ++part) {
-        if (p.is_bf16) {
-          emit(std::true_type{}, part);
-        } else {
-          emit(std::false_type{}, part);
-        }
-        tmem_st_32x32(t_scores + part * 32, sc[part]);
-        if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
-        tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
-        tc_fence_before_sync();  // before the MMAs that the hand-over starts
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
-      }
-      float s0, s1, s2, s3;
-      f2_unpack(sums[0], &s0, &s1);
-      f2_unpack(sums[1], &s2, &s3);
-      l_run += (s0 + s1) + (s2 + s3);
+      softmax_block<D>(p, t_scores, t_out, j, common_last, key_last, t.p_full_bar[tile], lane, &m_used, &l_run);
     }
     // The last product.
     if (ok && my_blocks > 0) {
@@ -925,26 +1025,9 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     if (ok) {
       const bool live = tq0 + row < p.q_len;
-      const float inv = 1.0f / l_run;
-      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + batch * p.out_stride[0] + head * p.out_stride[1] +
+      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + u.batch * p.out_stride[0] + u.head * p.out_stride[1] +
                       static_cast<int64_t>(tq0 + row) * p.out_stride[2];
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32(t_out + c * 32, v);
-        tmem_ld_wait(v);
-        if (live) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 w;
-            w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
-            w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
-            w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
-            w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
-            *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
-          }
-        }
-      }
+      store_output<D>(p, t_out, l_run, live, dst);
     }
     if (!ok && lane == 0) {
       abort_flag = 1;
@@ -957,38 +1040,38 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (elect_one()) {
         bool ok = true;
         auto load = [&](void *dst, const CUtensorMap *map, uint64_t *bar, int32_t c0, int32_t c1, int32_t c2) {
-          tma_load_4d(dst, map, bar, c0, c1, c2, batch);
+          tma_load_4d(dst, map, bar, c0, c1, c2, u.batch);
         };
         for (int i = 0; i < kTiles; ++i) {
           mbar_arrive_expect_tx(&t.q_full_bar[i], L::kQBytes);
 #pragma unroll
           for (int a = 0; a < L::kQAtoms; ++a) {
-            load(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, q0 + i * kBlockQ, head);
+            load(q_tile(i) + a * kBlockQ * kAtomBytes, &tmap_q, &t.q_full_bar[i], a * kAtomBytes, u.q0 + i * kBlockQ, u.head);
           }
         }
-        for (int n = 0; n < 2 * num_blocks && ok; ++n) {
+        for (int n = 0; n < 2 * u.num_blocks && ok; ++n) {
           const int st = n % S, j = n >> 1;
           if (!mbar_wait(&t.slot_empty_bar[st], ((n / S) & 1) ^ 1, &abort_flag)) {
             ok = false;
             break;
           }
           mbar_arrive_expect_tx(&t.slot_full_bar[st], L::kSlotBytes);
-          const int key0 = (block0 + j) * kBlockKv;
+          const int key0 = j * kBlockKv;
           if ((n & 1) == 0) {
 #pragma unroll
             for (int a = 0; a < L::kQAtoms; ++a) {
-              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_k, &t.slot_full_bar[st], a * kAtomBytes, key0, u.head / p.group);
             }
           } else if (p.v_direct) {  // v like k: 128 keys x 64 elements of head_dim per atom
 #pragma unroll
             for (int a = 0; a < L::kQAtoms; ++a) {
-              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, kv_head);
+              load(slot(st) + a * kBlockKv * kAtomBytes, &tmap_vt, &t.slot_full_bar[st], a * kAtomBytes, key0, u.head / p.group);
             }
           } else {
 #pragma unroll
             for (int a = 0; a < L::kVAtoms; ++a) {
               tma_load_3d(slot(st) + a * L::kVAtomBytes, &tmap_vt, &t.slot_full_bar[st], (key0 + a * kAtomElems) * 2, 0,
-                          batch * p.kv_heads + kv_head);
+                          u.batch * p.kv_heads + u.head / p.group);
             }
           }
         }
@@ -1006,78 +1089,33 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       // measured 399, and 82 against 62 on 4 x 32 x 1000 causal.
       const bool issuer = elect_one();
       {
-        const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-        const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
-        const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
-        constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
-        constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
-        constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
-        constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
-        const uint64_t qdesc0 = umma_desc_sw128(smem_u32(q_tile(0)));
+        const TileMmas<D> mma(p, tmem_base, smem_u32(q_tile(0)), issuer);
         const uint64_t sdesc0 = umma_desc_sw128(smem_u32(slot(0)));
         bool ok = true;
         auto commit = [&](uint64_t *bar) {
           if (issuer) umma_commit(bar);
         };
-        auto scores = [&](int i, uint64_t kd) {  // S_i = Q_i K^T
-          const uint32_t s_tmem = tmem_base + i * L::kSCols;
-          const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
-#pragma unroll
-          for (int m = 0; m < kScoreMmas; ++m) {
-            const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-            const uint64_t qa = qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep);
-            const uint64_t ka = kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep);
-            if (issuer) umma_ss<kKindF16>(s_tmem, qa, ka, idesc_s, m != 0 ? 1u : 0u);
-          }
-        };
-        // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes
-        // on, the operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64
-        // head_dim positions lie a 128-key atom apart.
-        const uint32_t idesc_o_mn = idesc_o | (1u << 16);
-        const uint64_t mn_fields = umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0);
-        auto product = [&](int i, int part, uint64_t vd, uint32_t first_block) {  // O_i += P_i V over one part of the block's keys
-          const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
-          const uint32_t p_tmem = tmem_base + i * L::kSCols;
-          constexpr int kPartMmas = kOutMmas / kPParts;
-          if (p.v_direct) {
-#pragma unroll
-            for (int k = 0; k < kPartMmas; ++k) {
-              const int m = part * kPartMmas + k;
-              const uint64_t va = (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4));
-              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, va, idesc_o_mn, m != 0 ? 1u : (first_block ^ 1u));
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < kPartMmas; ++k) {
-              const int m = part * kPartMmas + k;
-              const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
-                          m != 0 ? 1u : (first_block ^ 1u));
-            }
-          }
-        };
         auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
         auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
-        const int blocks[kTiles] = {blocks_of(0), blocks_of(1)};
         for (int i = 0; i < kTiles && ok; ++i) ok = mbar_wait(&t.q_full_bar[i], 0, &abort_flag);
-        if (ok && num_blocks > 0) ok = wait_full(0);
-        if (ok && num_blocks > 0) {
+        if (ok && u.num_blocks > 0) ok = wait_full(0);
+        if (ok && u.num_blocks > 0) {
           tc_fence_after_sync();
 #pragma unroll
           for (int i = 0; i < kTiles; ++i) {
-            if (blocks[i] == 0) continue;
-            scores(i, desc_of(0));
+            if (u.blocks[i] == 0) continue;
+            mma.scores(i, desc_of(0));
             commit(&t.s_full_bar[i]);
           }
           commit(&t.slot_empty_bar[0]);
         }
-        for (int j = 0; j < num_blocks && ok; ++j) {
-          const bool more = j + 1 < num_blocks;
+        for (int j = 0; j < u.num_blocks && ok; ++j) {
+          const bool more = j + 1 < u.num_blocks;
           const int nv = 2 * j + 1, nk = 2 * j + 2;
           if (!wait_full(nv)) ok = false;
 #pragma unroll
           for (int i = 0; i < kTiles; ++i) {
-            if (!ok || j >= blocks[i]) continue;
+            if (!ok || j >= u.blocks[i]) continue;
             // The product reads P from the columns the next scores overwrite: the instructions of one
             // thread run in the order they were issued.
 #pragma unroll
@@ -1085,10 +1123,10 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               if (ok) ok = mbar_wait(&t.p_full_bar[i][part], j & 1, &abort_flag);
               if (!ok) break;
               tc_fence_after_sync();
-              product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
+              mma.product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
             }
             if (!ok) continue;
-            if (j + 1 == blocks[i]) {
+            if (j + 1 == u.blocks[i]) {
               commit(&t.pv_done_bar[i]);  // (a block's scores, which the softmax waits for, follow its product)
             } else {
               if (!wait_full(nk)) {  // (seen by the first tile's turn, for the second's too)
@@ -1096,7 +1134,7 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                 continue;
               }
               tc_fence_after_sync();
-              scores(i, desc_of(nk));
+              mma.scores(i, desc_of(nk));
               commit(&t.s_full_bar[i]);
             }
           }
@@ -1126,38 +1164,6 @@ attention2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 }
 
 // ---- the same, going on from unit to unit ------------------------------------------------------
-
-// Two tiles of 128 queries of one head and the blocks of keys they walk, from the first on (of the
-// masks only the block diagonal one hides a run's first keys, and it is not served here).
-struct Unit2 {
-  int head, batch, q0;
-  int num_blocks;
-  int blocks[kTiles];  // how many of them each tile walks: 0 for a tile past the last query
-
-  // Without a mask the units of one head run side by side and share its keys and values in L2. Under
-  // the causal masks the later queries have more keys to walk: the last unit of every head goes first,
-  // then the one before it, so that the grid ends on the short ones whatever the head.
-  __device__ __forceinline__ Unit2(const KernelParams &p, int x, int y, int z) : head(y), batch(z) {
-    int unit = x;
-    if (p.mask_type != 0) {
-      const int units = gridDim.x, heads = gridDim.y, all = heads * gridDim.z;
-      const int order = x + units * (y + heads * z);
-      unit = units - 1 - order / all;
-      head = order % all % heads;
-      batch = order % all / heads;
-    }
-    q0 = unit * (kTiles * kBlockQ);
-    const int offset = p.kv_len - p.q_len;
-    const int last_row = min(q0 + kTiles * kBlockQ, p.q_len) - 1;
-    num_blocks = (last_key_of(p, last_row + offset) + kBlockKv) / kBlockKv;
-    // Under the causal masks the first tile's queries see nothing of the last blocks the second walks.
-#pragma unroll
-    for (int i = 0; i < kTiles; ++i) {
-      const int last = min(q0 + (i + 1) * kBlockQ, p.q_len) - 1;
-      blocks[i] = q0 + i * kBlockQ >= p.q_len ? 0 : min(num_blocks, (last_key_of(p, last + offset) + kBlockKv) / kBlockKv);
-    }
-  }
-};
 
 // Asks for a CTA of this grid that has not started: sixteen bytes of answer, counted on `bar`.
 __device__ __forceinline__ void claim_next_cta(uint4 *answer, uint64_t *bar) {
@@ -1266,11 +1272,7 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const uint32_t t_lane = tmem_base + ((quarter * 32u) << 16);
     const uint32_t t_scores = t_lane + tile * L::kSCols;  // the row's 128 scores, then its 128 probabilities in 64 columns
     const uint32_t t_out = t_lane + L::kOCol + tile * D;
-    constexpr int kChunks = kBlockKv / 32;
-    static_assert(kChunks == 4, "four chunks of scores pack into the first two");
-    constexpr float kRescaleStep = 8.0f;
     bool ok = true;
-    uint32_t sc[kChunks][32];
     uint32_t s_phase = 0, pv_phase = 0;  // of the tile's scores and of its finished outputs
     int4 at = make_int4(blockIdx.x, blockIdx.y, blockIdx.z, 1);
 
@@ -1284,101 +1286,13 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       float l_run = 0.0f;
       const int my_blocks = tile == 0 ? u.blocks[0] : u.blocks[1];
       for (int j = 0; j < my_blocks && ok; ++j) {
-        // The row's scores of the block into registers in one round trip. (Scores of block j are
-        // issued behind the product of block j - 1: once they are here the tile's output is complete
-        // up to that block.)
+        // (Scores of block j are issued behind the product of block j - 1: once they are here the tile's
+        // output is complete up to that block.)
         ok = __all_sync(0xffffffffu, mbar_wait(&t.s_full_bar[tile], s_phase, &abort_flag));
         if (!ok) break;
         s_phase ^= 1;
         tc_fence_after_sync();
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(t_scores + c * 32, sc[c]);
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) tmem_ld_wait(sc[c]);
-        const int block_key0 = j * kBlockKv;
-        const bool edge = block_key0 + kBlockKv - 1 > common_last;
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        if (edge) {
-#pragma unroll
-          for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (block_key0 + c * 32 + i > key_last) sc[c][i] = __float_as_uint(-INFINITY);
-            }
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
-          }
-        }
-        const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
-        if (__any_sync(0xffffffffu, m_blk > m_used + kRescaleStep)) {
-          const float m_new = fmaxf(m_used, m_blk);
-          const float alpha = exp2f(m_used - ((m_new == -INFINITY) ? 0.0f : m_new));
-          l_run *= alpha;
-          if (j > 0) {
-#pragma unroll 1
-            for (int c = 0; c < D / 16; ++c) {  // sixteen columns at a time: the block's scores stay in registers
-              uint32_t v[16];
-              tmem_ld_32x16(t_out + c * 16, v);
-              tmem_ld_wait(v);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-              tmem_st_32x16(t_out + c * 16, v);
-            }
-          }
-          m_used = m_new;
-        }
-        const float m_sub = (m_used == -INFINITY) ? 0.0f : m_used;
-        // The probabilities, packed in place: pair i of the row's keys becomes column i of its P
-        // (a slot whose scores have been used by then).
-        const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(-m_sub, -m_sub);
-        uint64_t sums[2] = {0, 0};  // (pairs of float32 zeros)
-        auto emit = [&](auto bf16_tag, int part) {
-          constexpr int kBf16 = decltype(bf16_tag)::value ? 1 : 0;
-#pragma unroll
-          for (int h = 0; h < kChunks / kPParts; ++h) {
-            const int c = part * (kChunks / kPParts) + h;
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              const uint64_t x = f2_fma(f2_pack(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
-              float e0, e1;
-              if ((i & 6) != 6) {  // one pair in four goes through the cubic, the others through the special-function unit
-                float x0, x1;
-                f2_unpack(x, &x0, &x1);
-                e0 = fast_exp2(x0);
-                e1 = fast_exp2(x1);
-              } else {
-                exp2_pair_poly(x, &e0, &e1);
-              }
-              sums[(i >> 1) & 1] = f2_add(sums[(i >> 1) & 1], f2_pack(e0, e1));
-              sc[c >> 1][(c & 1) * 16 + (i >> 1)] = pack16(e0, e1, kBf16);
-            }
-          }
-        };
-        // Each half of the block's keys is handed over as soon as it is there: its product runs under
-        // the exponentials of the other half.
-#pragma unroll
-        for (int part = 0; part < kPParts; ++part) {
-          if (p.is_bf16) {
-            emit(std::true_type{}, part);
-          } else {
-            emit(std::false_type{}, part);
-          }
-          tmem_st_32x32(t_scores + part * 32, sc[part]);
-          if (kPParts == 1) tmem_st_32x32(t_scores + 32, sc[1]);
-          tmem_st_wait();          // the probabilities and a rescaled output are in tensor memory
-          tc_fence_before_sync();  // before the MMAs that the hand-over starts
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&t.p_full_bar[tile][part]);
-        }
-        float s0, s1, s2, s3;
-        f2_unpack(sums[0], &s0, &s1);
-        f2_unpack(sums[1], &s2, &s3);
-        l_run += (s0 + s1) + (s2 + s3);
+        softmax_block<D>(p, t_scores, t_out, j, common_last, key_last, t.p_full_bar[tile], lane, &m_used, &l_run);
       }
       // The last product.
       if (ok && my_blocks > 0) {
@@ -1388,26 +1302,9 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       }
       if (ok && my_blocks > 0) {
         const bool live = tq0 + row < p.q_len;
-        const float inv = 1.0f / l_run;
         uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + u.batch * p.out_stride[0] + u.head * p.out_stride[1] +
                         static_cast<int64_t>(tq0 + row) * p.out_stride[2];
-#pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(t_out + c * 32, v);
-          tmem_ld_wait(v);
-          if (live) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              uint4 w;
-              w.x = pack16(__uint_as_float(v[g * 8 + 0]) * inv, __uint_as_float(v[g * 8 + 1]) * inv, p.is_bf16);
-              w.y = pack16(__uint_as_float(v[g * 8 + 2]) * inv, __uint_as_float(v[g * 8 + 3]) * inv, p.is_bf16);
-              w.z = pack16(__uint_as_float(v[g * 8 + 4]) * inv, __uint_as_float(v[g * 8 + 5]) * inv, p.is_bf16);
-              w.w = pack16(__uint_as_float(v[g * 8 + 6]) * inv, __uint_as_float(v[g * 8 + 7]) * inv, p.is_bf16);
-              *reinterpret_cast<uint4 *>(dst + c * 32 + g * 8) = w;
-            }
-          }
-        }
+        store_output<D>(p, t_out, l_run, live, dst);
         // The next unit's first product overwrites this output: it waits for probabilities that the tile's
         // four warps hand over only after these reads.
         tc_fence_before_sync();
@@ -1506,55 +1403,11 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       // measured 399, and 82 against 62 on 4 x 32 x 1000 causal.
       const bool issuer = elect_one();
       {
-        const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-        const uint32_t idesc_s = umma_idesc(kBlockQ, kBlockKv, fmt, fmt);
-        const uint32_t idesc_o = umma_idesc(kBlockQ, D, fmt, fmt);
-        constexpr uint64_t kMmaStep = kMmaKBytes >> 4;
-        constexpr int kMmasPerAtom = kAtomBytes / kMmaKBytes;
-        constexpr int kScoreMmas = L::kQAtoms * kMmasPerAtom;
-        constexpr int kOutMmas = L::kVAtoms * kMmasPerAtom;  // one per 16 keys: 8 columns of P each
-        const uint64_t qdesc0 = umma_desc_sw128(smem_u32(q_tile(0)));
+        const TileMmas<D> mma(p, tmem_base, smem_u32(q_tile(0)), issuer);
         const uint64_t sdesc0 = umma_desc_sw128(smem_u32(slot(0)));
         bool ok = true;
         auto commit = [&](uint64_t *bar) {
           if (issuer) umma_commit(bar);
-        };
-        auto scores = [&](int i, uint64_t kd) {  // S_i = Q_i K^T
-          const uint32_t s_tmem = tmem_base + i * L::kSCols;
-          const uint64_t qd = qdesc0 + static_cast<uint64_t>(i * (L::kQBytes >> 4));
-#pragma unroll
-          for (int m = 0; m < kScoreMmas; ++m) {
-            const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-            const uint64_t qa = qd + (((a * kBlockQ * kAtomBytes) >> 4) + s * kMmaStep);
-            const uint64_t ka = kd + (((a * kBlockKv * kAtomBytes) >> 4) + s * kMmaStep);
-            if (issuer) umma_ss<kKindF16>(s_tmem, qa, ka, idesc_s, m != 0 ? 1u : 0u);
-          }
-        };
-        // With v as it lies, a slot's rows are keys: an instruction's 16 keys are 16 rows of 128 bytes
-        // on, the operand is MN-major (bit 16 of the instruction descriptor) and its runs of 64
-        // head_dim positions lie a 128-key atom apart.
-        const uint32_t idesc_o_mn = idesc_o | (1u << 16);
-        const uint64_t mn_fields = umma_desc_sw128_mn(0, kBlockKv * kAtomBytes) ^ umma_desc_sw128(0);
-        auto product = [&](int i, int part, uint64_t vd, uint32_t first_block) {  // O_i += P_i V over one part of the block's keys
-          const uint32_t o_tmem = tmem_base + L::kOCol + i * D;
-          const uint32_t p_tmem = tmem_base + i * L::kSCols;
-          constexpr int kPartMmas = kOutMmas / kPParts;
-          if (p.v_direct) {
-#pragma unroll
-            for (int k = 0; k < kPartMmas; ++k) {
-              const int m = part * kPartMmas + k;
-              const uint64_t va = (vd ^ mn_fields) + static_cast<uint64_t>(m * ((16 * kAtomBytes) >> 4));
-              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, va, idesc_o_mn, m != 0 ? 1u : (first_block ^ 1u));
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < kPartMmas; ++k) {
-              const int m = part * kPartMmas + k;
-              const int a = m / kMmasPerAtom, s = m % kMmasPerAtom;
-              if (issuer) umma_ts_f16(o_tmem, p_tmem + m * 8, vd + (((a * L::kVAtomBytes) >> 4) + s * kMmaStep), idesc_o,
-                          m != 0 ? 1u : (first_block ^ 1u));
-            }
-          }
         };
         auto wait_full = [&](int n) -> bool { return mbar_wait(&t.slot_full_bar[n % S], (n / S) & 1, &abort_flag); };
         auto desc_of = [&](int n) -> uint64_t { return sdesc0 + static_cast<uint64_t>((n % S) * (L::kSlotBytes >> 4)); };
@@ -1568,7 +1421,7 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         // Tile i's scores with the keys in load nk; `last`: of its unit, so that its queries may be replaced.
         auto issue_scores = [&](int i, int nk, bool last) {
           tc_fence_after_sync();
-          scores(i, desc_of(nk));
+          mma.scores(i, desc_of(nk));
           commit(&t.s_full_bar[i]);
           if (last) commit(&t.q_empty_bar[i]);
         };
@@ -1604,7 +1457,7 @@ attention2_units_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 if (ok) ok = mbar_wait(&t.p_full_bar[i][part], p_phase[i], &abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
-                product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
+                mma.product(i, part, desc_of(nv), j == 0 ? 1u : 0u);
               }
               if (!ok) continue;
               p_phase[i] ^= 1;
